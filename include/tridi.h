@@ -304,6 +304,11 @@ tridi_status tridi_refine_f32(const float *a, const float *b, const float *c, co
 tridi_status tridi_selfcheck_df_to_double(const float *hi, const float *lo, double *out, long n,
                                           tridi_stream_t stream);
 
+/* Self-check: q[i] = a[i] / b[i] the way the FP64 solvers divide (on the
+   integer units, within 1 ulp of the IEEE quotient; device arrays of n
+   elements). */
+tridi_status tridi_selfcheck_div_f64(const double *a, const double *b, double *q, long n, tridi_stream_t stream);
+
 /* Self-check of the bounded device waits (no counterpart in the reference):
    one CTA of num_threads threads (1..1024) waits on an mbarrier for at most
    limit_cycles SM cycles (1 .. ~2e9, the kernels' own limit).  With

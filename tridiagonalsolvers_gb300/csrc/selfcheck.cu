@@ -24,7 +24,21 @@ __global__ void wait_selfcheck_kernel(long long limit_cycles, int arrive, unsign
   timed_out[threadIdx.x] = ok ? 0 : 1;
 }
 
+// The FP64 solvers' division (div64.cuh) on its own.
+__global__ void div64_selfcheck_kernel(const double* a, const double* b, double* q, long n) {
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    q[i] = div64(a[i], invert64(b[i]));
+}
+
 }  // namespace tridi
+
+extern "C" tridi_status tridi_selfcheck_div_f64(const double* a, const double* b, double* q, long n,
+                                                tridi_stream_t stream) {
+  if (!a || !b || !q || n < 1) return TRIDI_ERROR_INVALID_VALUE;
+  const long blocks = (n + 255) / 256;
+  tridi::div64_selfcheck_kernel<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, tridi::as_stream(stream)>>>(a, b, q, n);
+  return tridi::cuda_status(cudaGetLastError());
+}
 
 extern "C" tridi_status tridi_selfcheck_wait(long long limit_cycles, int arrive, int* timed_out, int num_threads,
                                              tridi_stream_t stream) {

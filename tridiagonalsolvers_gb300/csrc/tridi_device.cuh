@@ -7,6 +7,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include "div64.cuh"
 #include "tridi.h"
 
 namespace tridi {
@@ -15,8 +16,8 @@ namespace tridi {
 // hardware's approximate reciprocal of the divisor (PTX rcp.approx.ftz.f32,
 // at most 1 ulp from 1/b; the product at most 2 ulp from the IEEE quotient),
 // no slow-path branch and no range fix-up (divisors here are O(1), far from
-// the denormal range that .ftz flushes).  FP64: the IEEE quotient.  Each
-// division of the reference's formulas becomes one tdiv, so results stay
+// the denormal range that .ftz flushes).  FP64: the quotient to nearest,
+// formed on the integer units (div64.cuh).  Each division of the reference's formulas becomes one tdiv, so results stay
 // within a few ulp of the reference's arithmetic.
 __device__ __forceinline__ float rcp_approx(float v) {
   float r;
@@ -24,7 +25,7 @@ __device__ __forceinline__ float rcp_approx(float v) {
   return r;
 }
 __device__ __forceinline__ float tdiv(float a, float b) { return a * rcp_approx(b); }
-__device__ __forceinline__ double tdiv(double a, double b) { return a / b; }
+__device__ __forceinline__ double tdiv(double a, double b) { return div64(a, invert64(b)); }
 
 // One equation a*x[i-1] + b*x[i] + c*x[i+1] = d.
 template <class T>
