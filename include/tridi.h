@@ -125,7 +125,8 @@ tridi_status tridi_crpcr_f64(const double *a, const double *b, const double *c, 
 
 /* Bank-conflict-free cyclic reduction.  Replaces crNBC() (crNBC.cu:123 /
    crNBCKernel :20) and crNBC32() (crNBC32banks.cu:123 / crNBC32Kernel :20).
-   n a power of two, 2 <= n <= 4096 (FP64: 2048).  Two kernels with the same
+   n a power of two, 2 <= n <= 4096 (FP64: 2048, the kernel of tridi_cr_f64,
+   whatever the tunable).  FP32: two kernels with the same
    arithmetic and bit-identical results: the register CR of tridi_cr_* (rows
    in registers, the staging ring read with conflict-free 16-byte loads; used
    by default) and a shared-memory CR whose every level is conflict-free by

@@ -10,7 +10,7 @@
 // Newton-Raphson step) and multiplied by the numerator's significand, so a
 // division issues no FP64 instruction at all; several quotients by one
 // divisor share its reciprocal.  In place of the IEEE division in the same
-// kernels: 16384 x 1024 CR 2939 -> 1452 us, 4096 x 1000 any-size 683 -> 312 us.
+// kernels: 16384 x 1024 CR 2939 -> 1456 us, 4096 x 1000 any-size 683 -> 257 us.
 //
 // Accuracy: the reciprocal is within 2^-60 of 1/b relative, the product is
 // rounded to nearest once: the quotient is within (1/2 + 2^-7) ulp of a / b,
@@ -29,7 +29,13 @@ __device__ __forceinline__ float div64_seed(float f) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
   return r;
 }
-__device__ __forceinline__ uint64_t div64_bits(double v) { return (uint64_t)__double_as_longlong(v); }
+// (a PTX move, so that the compiler does not see the value behind the bits:
+// it would turn tests of the exponent field into FP64 compares)
+__device__ __forceinline__ uint64_t div64_bits(double v) {
+  uint64_t u;
+  asm("mov.b64 %0, %1;" : "=l"(u) : "d"(v));
+  return u;
+}
 __device__ __forceinline__ double div64_value(uint64_t v) { return __longlong_as_double((long long)v); }
 __device__ __forceinline__ uint32_t div64_fbits(float v) { return __float_as_uint(v); }
 __device__ __forceinline__ float div64_fvalue(uint32_t v) { return __uint_as_float(v); }
@@ -72,9 +78,21 @@ __host__ __device__ __forceinline__ uint64_t reciprocal_q64(uint64_t bits) {
 
 __host__ __device__ __forceinline__ Inv64 invert64(double b) { return Inv64{reciprocal_q64(div64_bits(b)), b}; }
 
-// The IEEE quotient, for the operands that quotient_fast() refuses (out of
-// line: rare, and its code would otherwise sit in every kernel many times).
-__host__ __device__ __attribute__((noinline)) inline double quotient_ieee(double a, double b) { return a / b; }
+// The IEEE quotient, for the operands that quotient_fast() refuses.  Out of
+// line, with the bits passed as integers: rare, and any part of it that the
+// compiler moved ahead of the test would cost FP64 issue at every division.
+#ifdef __CUDACC__
+static __device__ __noinline__ uint64_t quotient_ieee_bits(uint64_t a, uint64_t b) {
+  return (uint64_t)__double_as_longlong(__ddiv_rn(__longlong_as_double((long long)a), __longlong_as_double((long long)b)));
+}
+#endif
+__host__ __device__ __forceinline__ double quotient_ieee(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return div64_value(quotient_ieee_bits(div64_bits(a), div64_bits(b)));
+#else
+  return a / b;
+#endif
+}
 
 // a / v.b into q; false where an operand or the quotient is zero-divisor,
 // subnormal, infinite or NaN (q is then meaningless).  A zero a is fine.

@@ -9,34 +9,25 @@ namespace tridi {
 
 namespace {
 
-// Per-(precision, n) shape: K rows per thread, TPS = n/K threads per system.
-// Groups of at most one warp use shuffles; wider groups use shared memory.
+// Per-n shape (FP32; FP64 has a kernel of its own, cr64.cu): K rows per
+// thread, TPS = n/K threads per system.  Groups of at most one warp use
+// shuffles; wider groups use shared memory.
 struct Shape {
   int K;
   int tps;
   bool warp;
 };
 
-template <class T>
 bool choose_shape(int n, Shape* s) {
-  if (!is_pow2(n) || n < 2) return false;
-  int K;
-  if (sizeof(T) == 4) {
-    if (n > 4096) return false;
-    K = n <= 16 ? n / 2 : (n == 4096 ? 16 : 8);
-  } else {
-    if (n > 2048) return false;
-    K = n <= 8 ? n / 2 : (n == 2048 ? 8 : 4);
-  }
+  if (!is_pow2(n) || n < 2 || n > 4096) return false;
+  int K = n <= 16 ? n / 2 : (n == 4096 ? 16 : 8);
   // rows per thread: the process-wide tunable, else the autotuned choice for
-  // this n (FP32 only), else the rule above
+  // this n, else the rule above
   int tk = tunable(TRIDI_TUNE_CR_ROWS);
-  if (tk <= 0 && sizeof(T) == 4) tk = tuned(TRIDI_AUTOTUNE_CR_ROWS, ilog2(n));
+  if (tk <= 0) tk = tuned(TRIDI_AUTOTUNE_CR_ROWS, ilog2(n));
   if (tk > 0 && is_pow2(tk) && tk <= n / 2 && n / tk <= 256) {
     // only shapes with an instantiated kernel (see solve_hybrid)
-    const bool warp = n / tk <= 32;
-    const bool have = sizeof(T) == 4 ? (warp ? tk <= 16 : (tk == 8 || tk == 16)) : (warp ? tk <= 4 : (tk == 4 || tk == 8));
-    if (have) K = tk;
+    if (n / tk <= 32 ? tk <= 16 : (tk == 8 || tk == 16)) K = tk;
   }
   s->K = K;
   s->tps = n / K;
@@ -97,12 +88,11 @@ cudaError_t launch_one(const HybridParams& p0, const DeviceInfo& dev, cudaStream
   HybridParams p = p0;
   const bool tma_ok = aligned16(p.a) && aligned16(p.b) && aligned16(p.c) && aligned16(p.d) && aligned16(p.x) &&
                       ((size_t)p.n * sizeof(T)) % 16 == 0 && !g_host_mapped_io;
-  // (FP32 shapes that keep their registers at 20 warps per SM; the FP64
-  // shapes and PCR on 16 rows per thread would spill)
-  if constexpr (WARP && sizeof(T) == 4 && !(K == 16 && LSTRIDE == 1)) {
+  // (PCR on 16 rows per thread would spill at 20 warps per SM)
+  if constexpr (WARP && !(K == 16 && LSTRIDE == 1)) {
     if (tma_ok && tunable(TRIDI_TUNE_WARP_STREAMS) != 2) return launch_warp_streams<T, K, LSTRIDE>(p, dev, stream);
   }
-  if constexpr (!WARP && sizeof(T) == 4 && !(K == 16 && LSTRIDE == 1)) {
+  if constexpr (!WARP && !(K == 16 && LSTRIDE == 1)) {
     if (tma_ok && p.ct == 128 && tunable(TRIDI_TUNE_WARP_STREAMS) != 2)
       return launch_block_streams<T, K, LSTRIDE>(p, dev, stream);
   }
@@ -154,20 +144,23 @@ cudaError_t launch_pcr_twophase(const HybridParams& p, const DeviceInfo& dev, cu
   return cudaGetLastError();
 }
 
-template <class T>
 bool pcr_twophase_applies(const HybridParams& p) {
-  if constexpr (sizeof(T) != 4) return false;
   return p.stride == 1 && (p.n == 64 || p.n == 128 || p.n == 256 || p.n == 512 || p.n == 1024) && aligned16(p.a) &&
          aligned16(p.b) && aligned16(p.c) && aligned16(p.d) && (long)p.m * p.n / 32 < (1L << 31) &&
          tunable(TRIDI_TUNE_PCR_KERNEL) != 2 && !g_host_mapped_io;
 }
 
-template <class T>
-tridi_status solve_hybrid(const T* a, const T* b, const T* c, const T* d, T* x, int n, int m, int stride,
-                          tridi_stream_t stream) {
+tridi_status solve_hybrid(const double* a, const double* b, const double* c, const double* d, double* x, int n, int m,
+                          int stride, tridi_stream_t stream) {
+  if (!a || !b || !c || !d || !x || m <= 0) return TRIDI_ERROR_INVALID_VALUE;
+  return cr64_solve(a, b, c, d, x, n, m, stride, as_stream(stream));
+}
+
+tridi_status solve_hybrid(const float* a, const float* b, const float* c, const float* d, float* x, int n, int m,
+                          int stride, tridi_stream_t stream) {
   if (!a || !b || !c || !d || !x || m <= 0) return TRIDI_ERROR_INVALID_VALUE;
   Shape sh;
-  if (!choose_shape<T>(n, &sh)) return TRIDI_ERROR_UNSUPPORTED_SIZE;
+  if (!choose_shape(n, &sh)) return TRIDI_ERROR_UNSUPPORTED_SIZE;
   const DeviceInfo* dev = current_device();
   if (!dev) return TRIDI_ERROR_CUDA;
   HybridParams p{};
@@ -180,40 +173,33 @@ tridi_status solve_hybrid(const T* a, const T* b, const T* c, const T* d, T* x, 
   p.status = dev->status;
   cudaStream_t s = as_stream(stream);
   cudaError_t e = cudaErrorInvalidValue;
-  if constexpr (sizeof(T) == 4) {
-    if (crpcr_regs_applies(a, b, c, d, x, n, m, stride)) return crpcr_regs_solve(a, b, c, d, x, n, m, stride, s);
-    if (pcr_twophase_applies<T>(p)) {
-      const bool paired = tunable(TRIDI_TUNE_PCR_KERNEL) != 3;
-      switch (n) {
-        case 64: return cuda_status(paired ? launch_pcr_twophase<64, true>(p, *dev, s)
-                                           : launch_pcr_twophase<64, false>(p, *dev, s));
-        case 128: return cuda_status(paired ? launch_pcr_twophase<128, true>(p, *dev, s)
-                                            : launch_pcr_twophase<128, false>(p, *dev, s));
-        case 256: return cuda_status(paired ? launch_pcr_twophase<256, true>(p, *dev, s)
-                                            : launch_pcr_twophase<256, false>(p, *dev, s));
-        case 512: return cuda_status(paired ? launch_pcr_twophase<512, true>(p, *dev, s)
-                                            : launch_pcr_twophase<512, false>(p, *dev, s));
-        default: return cuda_status(paired ? launch_pcr_twophase<1024, true>(p, *dev, s)
-                                           : launch_pcr_twophase<1024, false>(p, *dev, s));
-      }
+  if (crpcr_regs_applies(a, b, c, d, x, n, m, stride)) return crpcr_regs_solve(a, b, c, d, x, n, m, stride, s);
+  if (pcr_twophase_applies(p)) {
+    const bool paired = tunable(TRIDI_TUNE_PCR_KERNEL) != 3;
+    switch (n) {
+      case 64: return cuda_status(paired ? launch_pcr_twophase<64, true>(p, *dev, s)
+                                         : launch_pcr_twophase<64, false>(p, *dev, s));
+      case 128: return cuda_status(paired ? launch_pcr_twophase<128, true>(p, *dev, s)
+                                          : launch_pcr_twophase<128, false>(p, *dev, s));
+      case 256: return cuda_status(paired ? launch_pcr_twophase<256, true>(p, *dev, s)
+                                          : launch_pcr_twophase<256, false>(p, *dev, s));
+      case 512: return cuda_status(paired ? launch_pcr_twophase<512, true>(p, *dev, s)
+                                          : launch_pcr_twophase<512, false>(p, *dev, s));
+      default: return cuda_status(paired ? launch_pcr_twophase<1024, true>(p, *dev, s)
+                                         : launch_pcr_twophase<1024, false>(p, *dev, s));
     }
   }
   const int ls = stride < sh.K ? stride : 0;
 #define TRIDI_LAUNCH_LS(KK, WW, LS) \
-  if (sh.K == KK && sh.warp == WW && ls == LS) e = launch_one<T, KK, WW, LS>(p, *dev, s);
+  if (sh.K == KK && sh.warp == WW && ls == LS) e = launch_one<float, KK, WW, LS>(p, *dev, s);
 #define TRIDI_LAUNCH(KK, WW)                                                             \
   TRIDI_LAUNCH_LS(KK, WW, 0)                                                              \
   if constexpr (KK > 1) { TRIDI_LAUNCH_LS(KK, WW, 1) }                                    \
   if constexpr (KK > 2) { TRIDI_LAUNCH_LS(KK, WW, (KK > 2 ? 2 : 1)) }                     \
   if constexpr (KK > 4) { TRIDI_LAUNCH_LS(KK, WW, (KK > 4 ? 4 : 1)) }                     \
   if constexpr (KK > 8) { TRIDI_LAUNCH_LS(KK, WW, (KK > 8 ? 8 : 1)) }
-  if constexpr (sizeof(T) == 4) {
-    TRIDI_LAUNCH(1, true) TRIDI_LAUNCH(2, true) TRIDI_LAUNCH(4, true) TRIDI_LAUNCH(8, true)
-    TRIDI_LAUNCH(16, true) TRIDI_LAUNCH(8, false) TRIDI_LAUNCH(16, false)
-  } else {
-    TRIDI_LAUNCH(1, true) TRIDI_LAUNCH(2, true) TRIDI_LAUNCH(4, true) TRIDI_LAUNCH(4, false)
-    TRIDI_LAUNCH(8, false)
-  }
+  TRIDI_LAUNCH(1, true) TRIDI_LAUNCH(2, true) TRIDI_LAUNCH(4, true) TRIDI_LAUNCH(8, true)
+  TRIDI_LAUNCH(16, true) TRIDI_LAUNCH(8, false) TRIDI_LAUNCH(16, false)
 #undef TRIDI_LAUNCH
 #undef TRIDI_LAUNCH_LS
   return cuda_status(e);
@@ -225,7 +211,7 @@ tridi_status solve_hybrid(const T* a, const T* b, const T* c, const T* d, T* x, 
 template <class T>
 tridi_status hybrid_solve_device(const T* a, const T* b, const T* c, const T* d, T* x, int n, int m, int stride,
                                  tridi_stream_t stream) {
-  return solve_hybrid<T>(a, b, c, d, x, n, m, stride, stream);
+  return solve_hybrid(a, b, c, d, x, n, m, stride, stream);
 }
 template tridi_status hybrid_solve_device<float>(const float*, const float*, const float*, const float*, float*,
                                                  int, int, int, tridi_stream_t);
@@ -242,7 +228,7 @@ tridi_status crpcr_checked(const T* a, const T* b, const T* c, const T* d, T* x,
                            tridi_stream_t s) {
   if (n < 4 || !tridi::is_pow2(rest) || rest < 2 || rest > n / 2 || !tridi::is_pow2(n))
     return TRIDI_ERROR_UNSUPPORTED_SIZE;
-  return solve_hybrid<T>(a, b, c, d, x, n, m, n / rest, s);
+  return solve_hybrid(a, b, c, d, x, n, m, n / rest, s);
 }
 }  // namespace
 
@@ -250,20 +236,20 @@ extern "C" {
 
 tridi_status tridi_cr_f32(const float* a, const float* b, const float* c, const float* d, float* x, int n, int m,
                           tridi_stream_t s) {
-  return solve_hybrid<float>(a, b, c, d, x, n, m, n / 2 > 0 ? n / 2 : 1, s);
+  return solve_hybrid(a, b, c, d, x, n, m, n / 2 > 0 ? n / 2 : 1, s);
 }
 tridi_status tridi_cr_f64(const double* a, const double* b, const double* c, const double* d, double* x, int n,
                           int m, tridi_stream_t s) {
-  return solve_hybrid<double>(a, b, c, d, x, n, m, n / 2 > 0 ? n / 2 : 1, s);
+  return solve_hybrid(a, b, c, d, x, n, m, n / 2 > 0 ? n / 2 : 1, s);
 }
 tridi_status tridi_pcr_f32(const float* a, const float* b, const float* c, const float* d, float* x, int n, int m,
                            tridi_stream_t s) {
   if (n > 4096) return TRIDI_ERROR_UNSUPPORTED_SIZE;
-  return solve_hybrid<float>(a, b, c, d, x, n, m, 1, s);
+  return solve_hybrid(a, b, c, d, x, n, m, 1, s);
 }
 tridi_status tridi_pcr_f64(const double* a, const double* b, const double* c, const double* d, double* x, int n,
                            int m, tridi_stream_t s) {
-  return solve_hybrid<double>(a, b, c, d, x, n, m, 1, s);
+  return solve_hybrid(a, b, c, d, x, n, m, 1, s);
 }
 tridi_status tridi_crpcr_f32(const float* a, const float* b, const float* c, const float* d, float* x, int n,
                              int m, int rest, tridi_stream_t s) {

@@ -3,7 +3,7 @@
 // arithmetic, results bit-identical to the shared-memory kernel for crNBC,
 // within a few ulp for crpcrNBC, about twice its speed), the
 // shared-memory CR of nbc.cuh on request (TRIDI_TUNE_NBC_KERNEL = 2) or where
-// the register kernel has no shape.  Replaces the device work of crNBC()
+// the register kernel has no shape; FP64 runs cr64.cu.  Replaces the device work of crNBC()
 // (crNBC.cu:123), crNBC32() (crNBC32banks.cu:123) and crpcrNBC()
 // (crNBC.cu:344).
 #include "nbc.cuh"
@@ -15,22 +15,18 @@ namespace {
 
 constexpr int kMaxThreads = 4 * 32 + 32;
 
-template <class T>
-tridi_status solve_nbc(const T* a, const T* b, const T* c, const T* d, T* x, int n, int m, int rest,
+tridi_status solve_nbc(const float* a, const float* b, const float* c, const float* d, float* x, int n, int m, int rest,
                        tridi_stream_t stream) {
+  using T = float;
   if (!a || !b || !c || !d || !x || m <= 0) return TRIDI_ERROR_INVALID_VALUE;
-  const int nmax = sizeof(T) == 4 ? 4096 : 2048;
-  if (!is_pow2(n) || n < 2 || n > nmax) return TRIDI_ERROR_UNSUPPORTED_SIZE;
+  if (!is_pow2(n) || n < 2 || n > 4096) return TRIDI_ERROR_UNSUPPORTED_SIZE;
   if (!is_pow2(rest) || rest < 2 || rest > (n > 2 ? n / 2 : 2)) return TRIDI_ERROR_UNSUPPORTED_SIZE;
   if (tunable(TRIDI_TUNE_NBC_KERNEL) != 2) {
     // the register kernels: the same CR arithmetic (bit-identical results at
     // rest 2; the PCR of crpcr's register kernels at 1024 unknowns works on
     // normalised rows, a few ulp apart), no shared-memory bank traffic
-    tridi_status st;
-    if constexpr (sizeof(T) == 4)
-      st = rest == 2 ? tridi_cr_f32(a, b, c, d, x, n, m, stream) : tridi_crpcr_f32(a, b, c, d, x, n, m, rest, stream);
-    else
-      st = rest == 2 ? tridi_cr_f64(a, b, c, d, x, n, m, stream) : tridi_crpcr_f64(a, b, c, d, x, n, m, rest, stream);
+    const tridi_status st =
+        rest == 2 ? tridi_cr_f32(a, b, c, d, x, n, m, stream) : tridi_crpcr_f32(a, b, c, d, x, n, m, rest, stream);
     if (st != TRIDI_ERROR_UNSUPPORTED_SIZE) return st;
   }
   const DeviceInfo* dev = current_device();
@@ -63,7 +59,7 @@ tridi_status solve_nbc(const T* a, const T* b, const T* c, const T* d, T* x, int
   p.stages = S;
   p.ntiles = (int)(((long)m + G - 1) / G);
   const size_t smem = NbcSmem<T>::bytes(S, G, n, rest);
-  auto kern = nbc_kernel<T, kMaxThreads, sizeof(T) == 4 ? 5 : 1>;  // FP32: 5 CTAs (20 solving warps) per SM
+  auto kern = nbc_kernel<T, kMaxThreads, 5>;  // 5 CTAs (20 solving warps) per SM
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_status(e);
   const int threads = 32 * G + 32;
@@ -77,6 +73,16 @@ tridi_status solve_nbc(const T* a, const T* b, const T* c, const T* d, T* x, int
   return cuda_status(cudaGetLastError());
 }
 
+// FP64: the shared-memory CR of cr64.cu (dense arrays at every level across
+// threads), whatever TRIDI_TUNE_NBC_KERNEL says.
+tridi_status solve_nbc(const double* a, const double* b, const double* c, const double* d, double* x, int n, int m,
+                       int rest, tridi_stream_t stream) {
+  if (!a || !b || !c || !d || !x || m <= 0) return TRIDI_ERROR_INVALID_VALUE;
+  if (!is_pow2(n) || n < 2 || n > 2048) return TRIDI_ERROR_UNSUPPORTED_SIZE;
+  if (!is_pow2(rest) || rest < 2 || rest > (n > 2 ? n / 2 : 2)) return TRIDI_ERROR_UNSUPPORTED_SIZE;
+  return rest == 2 ? tridi_cr_f64(a, b, c, d, x, n, m, stream) : tridi_crpcr_f64(a, b, c, d, x, n, m, rest, stream);
+}
+
 }  // namespace
 }  // namespace tridi
 
@@ -86,21 +92,21 @@ extern "C" {
 
 tridi_status tridi_cr_nbc_f32(const float* a, const float* b, const float* c, const float* d, float* x, int n,
                               int m, tridi_stream_t s) {
-  return solve_nbc<float>(a, b, c, d, x, n, m, 2, s);
+  return solve_nbc(a, b, c, d, x, n, m, 2, s);
 }
 tridi_status tridi_cr_nbc_f64(const double* a, const double* b, const double* c, const double* d, double* x,
                               int n, int m, tridi_stream_t s) {
-  return solve_nbc<double>(a, b, c, d, x, n, m, 2, s);
+  return solve_nbc(a, b, c, d, x, n, m, 2, s);
 }
 tridi_status tridi_crpcr_nbc_f32(const float* a, const float* b, const float* c, const float* d, float* x, int n,
                                  int m, int rest, tridi_stream_t s) {
   if (n < 4) return TRIDI_ERROR_UNSUPPORTED_SIZE;
-  return solve_nbc<float>(a, b, c, d, x, n, m, rest, s);
+  return solve_nbc(a, b, c, d, x, n, m, rest, s);
 }
 tridi_status tridi_crpcr_nbc_f64(const double* a, const double* b, const double* c, const double* d, double* x,
                                  int n, int m, int rest, tridi_stream_t s) {
   if (n < 4) return TRIDI_ERROR_UNSUPPORTED_SIZE;
-  return solve_nbc<double>(a, b, c, d, x, n, m, rest, s);
+  return solve_nbc(a, b, c, d, x, n, m, rest, s);
 }
 
 }  // extern "C"

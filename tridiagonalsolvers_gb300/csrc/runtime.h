@@ -56,6 +56,10 @@ bool crpcr_regs_applies(const void* a, const void* b, const void* c, const void*
 tridi_status crpcr_regs_solve(const float* a, const float* b, const float* c, const float* d, float* x, int n,
                               int m, int stride, cudaStream_t stream);
 
+// cr, pcr and crpcr at every switch level in FP64 (cr64.cu); stride = n / rest.
+tridi_status cr64_solve(const double* a, const double* b, const double* c, const double* d, double* x, int n, int m,
+                        int stride, cudaStream_t stream);
+
 inline int ilog2(long v) {
   int k = 0;
   while (v > 1) {
