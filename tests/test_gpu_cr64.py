@@ -62,3 +62,32 @@ def test_misaligned_and_isolated(cuda, n, rest):
     ends[0][:, 0] = np.nan
     ends[2][:, -1] = np.nan
     assert np.array_equal(x, _solve(cuda, ends, n, rest))
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 8, 9, 16, 17, 63, 257, 1000, 1025, 2047, 2049, 4096, 4097, 4607, 4608])
+def test_any_size(cuda, n):
+    """tg.solve in FP64: the same kernel on n rows, whatever n: the sizes
+    around a thread's 8 rows, a CTA's and the largest, in batches of one
+    system, an odd count and more tiles than CTAs; an odd pointer offset and a
+    non-finite neighbour change no bit."""
+    import torch
+
+    for m in (1, 6, 2 * 152 * 5 + 7 if n in (1, 257, 1000) else 19):
+        arrs = workloads.dominant(m, n, seed=7 * n + m, dtype=np.float64)
+        t = [torch.from_numpy(v).to(cuda) for v in arrs]
+        x = tg.solve(*t).cpu().numpy()
+        check_against_oracle(*arrs, x, dtype=np.float64)
+        off = []
+        for v in arrs:
+            buf = torch.zeros(v.size + 1, dtype=torch.float64, device=cuda)
+            buf[1:] = torch.from_numpy(v.ravel())
+            off.append(buf[1:].view(m, n))
+        assert np.array_equal(x, tg.solve(*off).cpu().numpy())
+        if m > 1:
+            bad = [v.copy() for v in arrs]
+            bad[1][m // 2] = np.nan
+            bad[3][m // 2] = np.inf
+            y = tg.solve(*(torch.from_numpy(v).to(cuda) for v in bad)).cpu().numpy()
+            keep = np.arange(m) != m // 2
+            assert np.array_equal(x[keep], y[keep])
+    assert tg.device_status() == 0

@@ -1,5 +1,6 @@
-// The cyclic-reduction family in FP64 (cr, pcr, crpcr, crNBC, crpcrNBC):
-// one kernel, the reference's algorithms (crpcr_kernel.cu:40-141).
+// The cyclic-reduction family in FP64 (cr, pcr, crpcr, crNBC, crpcrNBC:
+// the reference's algorithms, crpcr_kernel.cu:40-141) and the any-size solve
+// in FP64 (cyclic reduction on n rows, whatever n): one kernel.
 //
 // What bounds it: the FP64 pipe.  The GB300 issues a DFMA of a warp in 16
 // cycles of the SM's FP64 pipe, so the kernel is built to issue few of them:
@@ -39,10 +40,10 @@ struct Cr64Params {
   const double* d;
   double* x;
   int n, m;
-  int tps;     // threads per system, n / K (a power of two, <= blockDim.x)
+  int tps;     // threads per system, ceil(n / K) <= blockDim.x; G = blockDim.x / tps systems a tile
   int rest;    // rows of the PCR-solved intermediate system (2 = plain CR, n = PCR)
-  int ntiles;  // ceil(m / (blockDim.x / tps))
-  int vec;     // all five pointers 16-byte aligned
+  int ntiles;  // ceil(m / G)
+  int vec;     // all five pointers 16-byte aligned and n even
 };
 
 // A row divided by its diagonal.
@@ -161,41 +162,128 @@ __device__ __forceinline__ void pcr64(Row<double> (&y)[R], double (&xs)[R], int 
   }
 }
 
+// Shared arrays of the levels across threads (a, b, c, d; x takes the place
+// of b) and the barrier of a step that `items` threads take part in: one
+// warp's worth and less stays in the first warp.
+struct Levels64 {
+  double *A, *B, *C, *D;
+};
+__device__ __forceinline__ bool level_takes_part(int items) { return items >= 32 || threadIdx.x < 32; }
+__device__ __forceinline__ void level_sync(int items) {
+  if (items > 32) __syncthreads();
+  else __syncwarp();
+}
+
+// Cyclic reduction of G systems of `per` rows each (any count), side by side
+// in the level arrays, down to one row a system, and back: B[g * per + j]
+// ends as x.  Level arrays of decreasing size follow one another; a level of
+// `per` rows keeps its floor(per / 2) odd rows.  tid / pairs by the rounded
+// reciprocal: exact for these ranges (tid < 1024).
+__device__ __forceinline__ void cr_levels_any(const Levels64& v, int G, int per0) {
+  const int tid = threadIdx.x;
+  int per = per0, o = 0;
+  while (per > 1) {
+    const int pp = (per + 1) / 2, items = G * pp, on = o + G * per;
+    if (level_takes_part(items)) {
+      Row<double> me{};
+      N64 L{};
+      const int g = (int)(((float)tid + 0.5f) * __frcp_rn((float)pp)), p = tid - g * pp, e = o + g * per + 2 * p;
+      const bool odd = 2 * p + 1 < per;
+      if (tid < items) {
+        L = normalize64(v.A[e], v.B[e], v.C[e], v.D[e]);
+        if (odd) me = Row<double>{v.A[e + 1], v.B[e + 1], v.C[e + 1], v.D[e + 1]};
+        v.A[e] = L.a; v.C[e] = L.c; v.D[e] = L.d;
+      }
+      level_sync(items);
+      if (tid < items && odd) {
+        eliminate_left(me, L);
+        if (2 * p + 2 < per) eliminate_right(me, N64{v.A[e + 2], v.C[e + 2], v.D[e + 2]});
+        const int w = on + g * (per / 2) + p;
+        v.A[w] = me.a; v.B[w] = me.b; v.C[w] = me.c; v.D[w] = me.d;
+      }
+      level_sync(items);
+    }
+    o = on;
+    per /= 2;
+  }
+  if (level_takes_part(G)) {
+    if (tid < G) v.B[o + tid] = tdiv(v.D[o + tid], v.B[o + tid]);
+    level_sync(G);
+  }
+  bool one_warp = G <= 32;
+  int depth = 31 - __clz(per0);  // levels above the last: per = per0 >> l
+  for (int l = depth - 1; l >= 0; --l) {
+    per = per0 >> l;
+    const int pp = (per + 1) / 2, items = G * pp, half = per / 2;
+    const int on = o;
+    o = on - G * per;
+    if (items > 32 && one_warp) {  // the first warp's levels are done
+      __syncthreads();
+      one_warp = false;
+    }
+    if (level_takes_part(items)) {
+      if (tid < items) {
+        const int g = (int)(((float)tid + 0.5f) * __frcp_rn((float)pp)), p = tid - g * pp, e = o + g * per + 2 * p;
+        const int w = on + g * half + p;
+        const double xl = p > 0 ? v.B[w - 1] : 0.0;
+        const double xo = 2 * p + 1 < per ? v.B[w] : 0.0;
+        const double al = p > 0 ? v.A[e] : 0.0, cr = 2 * p + 1 < per ? v.C[e] : 0.0;
+        v.B[e] = fma(-cr, xo, fma(-al, xl, v.D[e]));
+        if (2 * p + 1 < per) v.B[e + 1] = xo;
+      }
+      level_sync(items);
+    }
+  }
+}
+
 // LS = 0: the intermediate system has at most one row a thread (n / rest >=
-// K); else LS = n / rest < K, K / LS rows a thread.
+// K); LS > 0: LS = n / rest < K, K / LS rows a thread; LS = -1: any n, cyclic
+// reduction throughout (rows past the system's end are identity rows).
 template <int K, int LS, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) cr64_kernel(Cr64Params p) {
-  constexpr int SMAX = LS == 0 ? K : LS;  // last in-thread CR level
+  constexpr bool ANY = LS < 0;
+  constexpr int SMAX = LS <= 0 ? K : LS;  // last in-thread CR level
   extern __shared__ __align__(16) double sm[];
   const int ct = blockDim.x, tid = threadIdx.x, tps = p.tps;
   double* ex = sm;  // [3 * level + word][thread]
   double* lv = sm + kExportWords * ct;
   double* xlast = lv + cr64_level_words(LS > 0 ? K / (LS > 0 ? LS : 1) : 1) * ct;
-  const int g = tid / tps, t = tid & (tps - 1);
+  const int g = tid / tps, t = tid - g * tps;
   const int G = ct / tps;
 
   for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x) {
     const long sys = (long)tile * G + g;
-    const bool in = sys < p.m;
+    const bool in = sys < p.m && (!ANY || g < G);
     const long at = sys * p.n + (long)t * K;
     Row<double> r[K];
+    const bool whole = in && (!ANY || (t + 1) * K <= p.n);
     {
       double v[K];
-      load_rows<K>(p.a, at, in, p.vec, 0.0, v);
+      load_rows<K>(p.a, at, whole, p.vec, 0.0, v);
 #pragma unroll
       for (int i = 0; i < K; ++i) r[i].a = v[i];
-      load_rows<K>(p.b, at, in, p.vec, 1.0, v);
+      load_rows<K>(p.b, at, whole, p.vec, 1.0, v);
 #pragma unroll
       for (int i = 0; i < K; ++i) r[i].b = v[i];
-      load_rows<K>(p.c, at, in, p.vec, 0.0, v);
+      load_rows<K>(p.c, at, whole, p.vec, 0.0, v);
 #pragma unroll
       for (int i = 0; i < K; ++i) r[i].c = v[i];
-      load_rows<K>(p.d, at, in, p.vec, 0.0, v);
+      load_rows<K>(p.d, at, whole, p.vec, 0.0, v);
 #pragma unroll
       for (int i = 0; i < K; ++i) r[i].d = v[i];
     }
+    if constexpr (ANY) {
+      if (in && !whole) {  // the system's last thread
+#pragma unroll
+        for (int i = 0; i < K; ++i)
+          if (t * K + i < p.n) r[i] = Row<double>{p.a[at + i], p.b[at + i], p.c[at + i], p.d[at + i]};
+      }
+#pragma unroll
+      for (int i = 0; i < K; ++i)
+        if (t * K + i == p.n - 1) r[i].c = 0.0;
+    }
     if (t == 0) r[0].a = 0.0;            // a[0] and c[n-1] are not part of the system
-    if (t == tps - 1) r[K - 1].c = 0.0;
+    if (!ANY && t == tps - 1) r[K - 1].c = 0.0;
 
     // 1. In-thread CR levels; the last row's right neighbours belong to the
     //    next thread and follow below.  Even rows end as (a/b, -, c/b, d/b).
@@ -245,8 +333,18 @@ __global__ void __launch_bounds__(MAXT, MINB) cr64_kernel(Cr64Params p) {
         __syncthreads();
         if (t > 0) xprev = xlast[tid - 1];
       }
+    } else if constexpr (ANY) {
+      // 2b. One row a thread, tps of them a system: cyclic reduction to the end
+      const Levels64 v{lv, lv + 2 * ct, lv + 4 * ct, lv + 6 * ct};
+      const int w = g * tps + t;  // == tid for the threads of a system
+      v.A[w] = r[K - 1].a; v.B[w] = r[K - 1].b; v.C[w] = r[K - 1].c; v.D[w] = r[K - 1].d;
+      __syncthreads();
+      cr_levels_any(v, G, tps);
+      __syncthreads();
+      xr[K - 1] = v.B[w];
+      if (t > 0) xprev = v.B[w - 1];
     } else {
-      // 2b. One row a thread: the CR levels across threads, compacted.  Level
+      // 2c. One row a thread: the CR levels across threads, compacted.  Level
       //     rows / 2 pairs; thread i takes rows 2i (even) and 2i + 1 (odd).
       double* A = lv;
       double* B = lv + 2 * ct;
@@ -332,7 +430,11 @@ __global__ void __launch_bounds__(MAXT, MINB) cr64_kernel(Cr64Params p) {
         xr[i] = fma(-r[i].c, xr[(i + h) % K], fma(-r[i].a, xl, r[i].d));
       }
     }
-    if (in) {
+    if (ANY && in && !whole) {
+#pragma unroll
+      for (int i = 0; i < K; ++i)
+        if (t * K + i < p.n) p.x[at + i] = xr[i];
+    } else if (in) {
       if (K % 2 == 0 && p.vec) {
 #pragma unroll
         for (int i = 0; i < K / 2; ++i)
@@ -346,14 +448,14 @@ __global__ void __launch_bounds__(MAXT, MINB) cr64_kernel(Cr64Params p) {
   }
 }
 
-template <int K, int LS>
+template <int K, int LS, int MAXT = 256>
 cudaError_t launch_cr64(Cr64Params p, const DeviceInfo& dev, cudaStream_t stream) {
-  auto kern = cr64_kernel<K, LS, 256, K == 4 ? 3 : 2>;
+  auto kern = cr64_kernel<K, LS, MAXT, (MAXT > 256 ? 1 : K == 4 ? 3 : 2)>;
   // 128 threads a CTA (a system of 2048 rows takes 256; 256 threads throughout
   // measured 410 us against 371 us at 16384 x 1024, 64 threads no gain), fewer
   // where that would leave SMs without one
-  int ct = p.tps > 128 ? p.tps : 128;
-  while (ct > 32 && ct > p.tps && (long)p.m * p.tps < 2L * dev.sm_count * ct) ct /= 2;
+  int ct = p.tps > 128 ? (p.tps + 31) / 32 * 32 : 128;
+  while (ct > 32 && ct / 2 >= p.tps && (long)p.m * p.tps < 2L * dev.sm_count * ct) ct /= 2;
   const size_t smem = cr64_smem(ct, LS > 0 ? K / (LS > 0 ? LS : 1) : 1);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -402,6 +504,27 @@ tridi_status cr64_solve(const double* a, const double* b, const double* c, const
     default: break;
   }
   return cuda_status(e);
+}
+
+// Any n, 1 <= n <= 4608.  (The partition method that did this before, a chunk
+// per lane and PCR on the 32 to 512 separators, issued 90 FP64 instructions a
+// row at 1000 rows, 15 of them with the integer division: 4096 x 1000 684 and
+// 257 us, cyclic reduction 106 us; 100000 x 20 1571 us, 48 us; 800 x 4608
+// 394 us, 147 us.)
+tridi_status cr64_solve_any(const double* a, const double* b, const double* c, const double* d, double* x, int n, int m,
+                            cudaStream_t stream) {
+  const DeviceInfo* dev = current_device();
+  if (!dev) return TRIDI_ERROR_CUDA;
+  constexpr int K = 8;
+  static_assert(576L * K == partition_max_rows<double>(), "any-size cap");
+  if (n < 1 || n > 576 * K) return TRIDI_ERROR_UNSUPPORTED_SIZE;
+  Cr64Params p{};
+  p.a = a; p.b = b; p.c = c; p.d = d; p.x = x;
+  p.n = n; p.m = m; p.tps = (n + K - 1) / K; p.rest = 1;
+  p.vec = aligned16(a) && aligned16(b) && aligned16(c) && aligned16(d) && aligned16(x) && n % 2 == 0;
+  return cuda_status(p.tps <= 256   ? launch_cr64<K, -1>(p, *dev, stream)
+                     : p.tps <= 512 ? launch_cr64<K, -1, 512>(p, *dev, stream)
+                                    : launch_cr64<K, -1, 576>(p, *dev, stream));
 }
 
 }  // namespace tridi

@@ -3,6 +3,7 @@
 // CTA mode: one CTA of ct threads per system; the ct separators form a
 // second tridiagonal system, solved by PCR across the CTA in shared memory.
 // Inputs arrive through the cp.async.bulk + mbarrier ring of hybrid.cuh.
+// FP64 runs the cyclic reduction of cr64.cu instead.
 #include "partition.cuh"
 #include "runtime.h"
 
@@ -186,40 +187,43 @@ int odd_ceil(int v) { return (v % 2) ? v : v + 1; }
 template <class T>
 tridi_status partition_solve_device(const T* a, const T* b, const T* c, const T* d, T* x, int n, int m,
                                     tridi_stream_t stream) {
-  constexpr bool F32 = sizeof(T) == 4;
-  constexpr int kWarpMax = F32 ? 31 : 15;  // rows per lane in warp mode
-  constexpr int kCtaMax = F32 ? 17 : 9;    // rows per thread in CTA mode (512 threads)
+  constexpr int kWarpMax = 31;  // rows per lane in warp mode
+  constexpr int kCtaMax = 17;   // rows per thread in CTA mode (512 threads)
   if (!a || !b || !c || !d || !x || m <= 0) return TRIDI_ERROR_INVALID_VALUE;
-  static_assert(512L * kCtaMax == partition_max_rows<T>(), "partition size cap");
+  static_assert(512L * kCtaMax == partition_max_rows<float>(), "partition size cap");
   if (n < 1 || n > partition_max_rows<T>()) return TRIDI_ERROR_UNSUPPORTED_SIZE;
-  const DeviceInfo* dev = current_device();
-  if (!dev) return TRIDI_ERROR_CUDA;
-  PartParams p{};
-  p.a = a; p.b = b; p.c = c; p.d = d; p.x = x;
-  p.n = n; p.m = m; p.status = dev->status;
-  cudaStream_t s = as_stream(stream);
-  cudaError_t e;
-  if (n <= 32 * kWarpMax) {
-    p.kk = odd_ceil((n + 31) / 32);
-    p.ct = 128;
-    p.G = 4;
-    p.ntiles = (int)(((long)m + 3) / 4);
-    if (p.kk <= 3) e = launch_part<T, 3, false>(p, *dev, s);
-    else if (p.kk <= 7) e = launch_part<T, 7, false>(p, *dev, s);
-    else if (p.kk <= 9) e = launch_part<T, 9, false>(p, *dev, s);
-    else if (p.kk <= 15) e = launch_part<T, 15, false>(p, *dev, s);
-    else e = launch_part<T, (F32 ? 31 : 15), false>(p, *dev, s);
+  if constexpr (sizeof(T) == 8) {
+    return cr64_solve_any(a, b, c, d, x, n, m, as_stream(stream));
   } else {
-    int ct = 128;
-    while (ct < 512 && odd_ceil((n + ct - 1) / ct) > 7) ct *= 2;
-    p.ct = ct;
-    p.kk = odd_ceil((n + ct - 1) / ct);
-    p.G = 1;
-    p.ntiles = m;
-    if (p.kk <= 7) e = launch_part<T, 7, true>(p, *dev, s);
-    else e = launch_part<T, kCtaMax, true>(p, *dev, s);
+    const DeviceInfo* dev = current_device();
+    if (!dev) return TRIDI_ERROR_CUDA;
+    PartParams p{};
+    p.a = a; p.b = b; p.c = c; p.d = d; p.x = x;
+    p.n = n; p.m = m; p.status = dev->status;
+    cudaStream_t s = as_stream(stream);
+    cudaError_t e;
+    if (n <= 32 * kWarpMax) {
+      p.kk = odd_ceil((n + 31) / 32);
+      p.ct = 128;
+      p.G = 4;
+      p.ntiles = (int)(((long)m + 3) / 4);
+      if (p.kk <= 3) e = launch_part<T, 3, false>(p, *dev, s);
+      else if (p.kk <= 7) e = launch_part<T, 7, false>(p, *dev, s);
+      else if (p.kk <= 9) e = launch_part<T, 9, false>(p, *dev, s);
+      else if (p.kk <= 15) e = launch_part<T, 15, false>(p, *dev, s);
+      else e = launch_part<T, 31, false>(p, *dev, s);
+    } else {
+      int ct = 128;
+      while (ct < 512 && odd_ceil((n + ct - 1) / ct) > 7) ct *= 2;
+      p.ct = ct;
+      p.kk = odd_ceil((n + ct - 1) / ct);
+      p.G = 1;
+      p.ntiles = m;
+      if (p.kk <= 7) e = launch_part<T, 7, true>(p, *dev, s);
+      else e = launch_part<T, kCtaMax, true>(p, *dev, s);
+    }
+    return cuda_status(e);
   }
-  return cuda_status(e);
 }
 
 template tridi_status partition_solve_device<float>(const float*, const float*, const float*, const float*, float*,

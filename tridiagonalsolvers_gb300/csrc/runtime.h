@@ -59,6 +59,9 @@ tridi_status crpcr_regs_solve(const float* a, const float* b, const float* c, co
 // cr, pcr and crpcr at every switch level in FP64 (cr64.cu); stride = n / rest.
 tridi_status cr64_solve(const double* a, const double* b, const double* c, const double* d, double* x, int n, int m,
                         int stride, cudaStream_t stream);
+// The any-size solve in FP64 (cr64.cu).
+tridi_status cr64_solve_any(const double* a, const double* b, const double* c, const double* d, double* x, int n, int m,
+                            cudaStream_t stream);
 
 inline int ilog2(long v) {
   int k = 0;
