@@ -1,229 +1,257 @@
-// Uniform-size batched partition solve (partition.cuh): tridi_solve_*.
-// Warp mode: one warp per system (n <= 32*K), G = 4 systems per tile.
-// CTA mode: one CTA of ct threads per system; the ct separators form a
-// second tridiagonal system, solved by PCR across the CTA in shared memory.
-// Inputs arrive through the cp.async.bulk + mbarrier ring of hybrid.cuh.
-// FP64 runs the cyclic reduction of cr64.cu instead.
-#include "partition.cuh"
+// Uniform-size batched solve of any n (partition.cuh, strip.cuh): tridi_solve_*.
+// FP32: the partition method.  Up to 992 rows a system is solved by 4 to 32
+// lanes of a warp (part_warp_kernel), above by a CTA (part_cta_kernel), up to
+// 8704 rows.  FP64 runs the cyclic reduction of cr64.cu instead.
+//
+// Both kernels stream: while a tile is solved in registers, the bulk copies
+// of the next one fill the staging buffer it came from; x leaves through a
+// shared buffer of its own in whole 16-byte groups.  Tiles start at any
+// element (strip.cuh), so an n that is no multiple of four is staged like the
+// others.  What bounds them is HBM: 55-56 us at 65536 x 250, 32768 x 500 and
+// 8192 x 2000 (86-88 % of the copy rate), 62 us at 4096 x 4000; 82 us at 2048 x
+// 8000, where one CTA fills an SM's shared memory and its loads wait for its
+// eliminations.  The kernels before these (a producer warp and PCR over a
+// CTA's separators in shared memory, one system a warp, rows off the grid read
+// by each lane from global memory): 72, 171, 168, 162 and 131 us; 500000 x 20
+// 239 us (37 us here, four systems and more a warp).
 #include "runtime.h"
+#include "strip.cuh"
 
 namespace tridi {
 
+namespace {
+
 struct PartParams {
-  const void* a;
-  const void* b;
-  const void* c;
-  const void* d;
-  void* x;
+  StripIn<float> in;
+  float* x;
   int n, m;
-  int G;       // systems per tile
-  int ntiles;
-  int stages;  // 0: read rows straight from global memory
-  int kk;      // rows per lane (odd)
-  int ct;      // consumer threads
+  int lps;     // warp kernel: lanes per system (a power of two)
+  int bulk;    // inputs staged by bulk copies
+  int vec;     // x 16-byte aligned
+  long cap;    // floats per array in a staging buffer
+  long total;  // n * m
   unsigned* status;
 };
 
-template <class T>
-__host__ __device__ inline size_t part_smem_bytes(int stages, int G, int n, int ct, bool cta) {
-  size_t s = 128 + (size_t)stages * 4 * G * n * sizeof(T);
-  if (cta) s += ((size_t)ct * 5 + (size_t)(ct / 32) * 3) * sizeof(T);
-  return s;
+// One warp per tile of 32 / lps systems, K rows a lane.
+template <int K, int MINB>
+__global__ void __launch_bounds__(128, MINB) part_warp_kernel(PartParams p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem) + warp;
+  float* buf = reinterpret_cast<float*>(smem + 128) + (size_t)warp * 5 * p.cap;
+  float* xs = buf + 4 * p.cap;
+  const int lps = p.lps, G = 32 / lps, g = lane / lps, t = lane - g * lps, n = p.n;
+  const long tiles = ((long)p.m + G - 1) / G;
+  const long first = (long)blockIdx.x * 4 + warp, step = (long)gridDim.x * 4;
+  const bool bulk = p.bulk != 0;
+  const auto strip = [&](long tile) {
+    const long s0 = tile * G, s1 = s0 + G < p.m ? s0 + G : p.m;
+    return Strip<float>(s0 * n, s1 * n, p.total, bulk);
+  };
+  if (lane == 0) {
+    mbar_init(bar, 1);
+    mbar_fence_init();
+    if (bulk && first < tiles) strip_issue(strip(first), p.in, buf, p.cap, bar);
+  }
+  __syncwarp();
+  int ph = 0;
+  for (long tile = first; tile < tiles; tile += step, ph ^= 1) {
+    const Strip<float> s = strip(tile);
+    if (bulk && !mbar_wait(bar, ph, p.status)) break;
+    if (s.hi < s.e1) strip_rest(s, p.in, buf, p.cap, lane, 32);
+    __syncwarp();
+    const bool in = tile * G + g < p.m;
+    int k = n - t * K;
+    k = !in || k < 0 ? 0 : (k > K ? K : k);
+    const int off = (int)(s.e0 - s.lo) + g * n + t * K;
+    Chunk<float, K> ch;
+    chunk_eliminate<float, K>(ch, k, t == 0, k > 0 && t * K + k == n, buf + off, buf + p.cap + off,
+                              buf + 2 * p.cap + off, buf + 3 * p.cap + off);
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (bulk && lane == 0 && tile + step < tiles) strip_issue(strip(tile + step), p.in, buf, p.cap, bar);
+    const float nD = __shfl_down_sync(kFull, ch.fD, 1, lps);
+    const float nC = __shfl_down_sync(kFull, ch.fC, 1, lps);
+    const float nA = __shfl_down_sync(kFull, ch.fA, 1, lps);
+    const float sj = group_pcr(separator_row<float, K>(ch, nD, nC, nA), lps);
+    const float up = __shfl_up_sync(kFull, sj, 1, lps);
+    float x[K];
+    chunk_back<float, K>(ch, k, sj, t == 0 ? 0.0f : up, x);
+#pragma unroll
+    for (int i = 0; i < K; ++i)
+      if (i < k) xs[off + i] = x[i];
+    __syncwarp();
+    strip_store(xs, s.lo, p.x, s.e0, s.e1, p.vec != 0, lane);
+    __syncwarp();
+  }
 }
 
-template <class T, int K, bool CTA, int MAXT, int MINB>
-__global__ void __launch_bounds__(MAXT, MINB) partition_kernel(PartParams p) {
+// One CTA of W warps per system, K rows a lane.
+template <int K, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) part_cta_kernel(PartParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem);
-  uint64_t* empty = full + 8;
-  const int S = p.stages, n = p.n, G = p.G, ct = p.ct, kk = p.kk;
-  T* stages = reinterpret_cast<T*>(smem + 128);
-  const size_t stage_elems = (size_t)4 * G * n;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-
-  if (tid == 0 && S > 0) {
-    for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], ct / 32);
-    }
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, W = blockDim.x >> 5, n = p.n;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
+  float* scratch = reinterpret_cast<float*>(smem + 16);
+  float* buf = reinterpret_cast<float*>(smem + 512);
+  float* xs = buf + 4 * p.cap;
+  const bool bulk = p.bulk != 0;
+  const auto strip = [&](long sys) { return Strip<float>(sys * n, (sys + 1) * n, p.total, bulk); };
+  if (tid == 0) {
+    mbar_init(bar, 1);
     mbar_fence_init();
+    if (bulk && (int)blockIdx.x < p.m) strip_issue(strip(blockIdx.x), p.in, buf, p.cap, bar);
   }
   __syncthreads();
-  const T* ga = static_cast<const T*>(p.a);
-  const T* gb = static_cast<const T*>(p.b);
-  const T* gc = static_cast<const T*>(p.c);
-  const T* gd = static_cast<const T*>(p.d);
-  T* gx = static_cast<T*>(p.x);
-
-  if (tid >= ct) {  // producer warp
-    if (S > 0 && lane == 0) {
-      int k = 0;
-      for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x, ++k) {
-        const int s = k % S;
-        if (k >= S && !mbar_wait(&empty[s], ((k / S) - 1) & 1, p.status)) break;
-        const long sys0 = (long)tile * G;
-        const long nsys = (p.m - sys0) < G ? (p.m - sys0) : G;
-        const uint32_t bytes = (uint32_t)(nsys * n * sizeof(T));
-        T* st = stages + s * stage_elems;
-        mbar_arrive_expect_tx(&full[s], 4 * bytes);
-        bulk_g2s(st + 0 * (size_t)G * n, ga + sys0 * n, bytes, &full[s]);
-        bulk_g2s(st + 1 * (size_t)G * n, gb + sys0 * n, bytes, &full[s]);
-        bulk_g2s(st + 2 * (size_t)G * n, gc + sys0 * n, bytes, &full[s]);
-        bulk_g2s(st + 3 * (size_t)G * n, gd + sys0 * n, bytes, &full[s]);
-      }
-    }
-    return;
-  }
-
-  // CTA-mode scratch: separator rows R (4 ct), their solution Xs (ct), and
-  // each warp's lane-0 first-row coefficients (3 per warp).
-  T* Ra = stages + (size_t)S * stage_elems;
-  T* Rb = Ra + ct;
-  T* Rc = Rb + ct;
-  T* Rd = Rc + ct;
-  T* Xs = Rd + ct;
-  T* F0 = Xs + ct;
-
-  const int g = CTA ? 0 : warp;  // system within the tile
-  int k = 0;
-  for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x, ++k) {
-    const long sys = (long)tile * G + g;
-    const T *sa, *sb, *sc, *sd;
-    int s = 0;
-    if (S > 0) {
-      s = k % S;
-      bool ok = mbar_wait(&full[s], (k / S) & 1, p.status);
-      if constexpr (CTA) ok = consumer_sync_and(ct, ok);
-      if (!ok) break;
-      const T* st = stages + s * stage_elems + (size_t)g * n;
-      sa = st; sb = st + (size_t)G * n; sc = st + 2 * (size_t)G * n; sd = st + 3 * (size_t)G * n;
-    } else {
-      const long sc0 = (sys < p.m ? sys : p.m - 1) * (long)n;
-      sa = ga + sc0; sb = gb + sc0; sc = gc + sc0; sd = gd + sc0;
-    }
-    T x[K];
-    int kl = 0;
-    int r0;
-    if constexpr (!CTA) {
-      r0 = lane * kk;
-      kl = warp_partition_solve<T, K>(n, kk, sa, sb, sc, sd, x);
-    } else {
-      r0 = tid * kk;
-      int kr = n - r0;
-      kr = kr < 0 ? 0 : (kr > kk ? kk : kr);
-      kl = kr;
-      Chunk<T, K> ch;
-      chunk_eliminate<T, K>(ch, kr, tid == 0, r0 + kr == n && kr > 0, sa + r0, sb + r0, sc + r0, sd + r0);
-      if (lane == 0) {
-        F0[warp * 3 + 0] = ch.fD; F0[warp * 3 + 1] = ch.fC; F0[warp * 3 + 2] = ch.fA;
-      }
-      consumer_sync(ct);
-      T nD = __shfl_down_sync(kFull, ch.fD, 1);
-      T nC = __shfl_down_sync(kFull, ch.fC, 1);
-      T nA = __shfl_down_sync(kFull, ch.fA, 1);
-      if (lane == 31 && warp + 1 < ct / 32) {
-        nD = F0[(warp + 1) * 3 + 0]; nC = F0[(warp + 1) * 3 + 1]; nA = F0[(warp + 1) * 3 + 2];
-      }
-      // The ct separators form a tridiagonal system: PCR across the CTA in
-      // shared memory, one row per thread, identity rows past either end.
-      Row<T> sr = separator_row<T, K>(ch, nD, nC, nA);
-      const Row<T> id{T(0), T(1), T(0), T(0)};
-      for (int dl = 1; dl < ct; dl *= 2) {
-        Ra[tid] = sr.a; Rb[tid] = sr.b; Rc[tid] = sr.c; Rd[tid] = sr.d;
-        consumer_sync(ct);
-        const Row<T> L = tid >= dl ? Row<T>{Ra[tid - dl], Rb[tid - dl], Rc[tid - dl], Rd[tid - dl]} : id;
-        const Row<T> R = tid + dl < ct ? Row<T>{Ra[tid + dl], Rb[tid + dl], Rc[tid + dl], Rd[tid + dl]} : id;
-        sr = reduce_row(sr, L, R);
-        consumer_sync(ct);
-      }
-      Xs[tid] = tdiv(sr.d, sr.b);
-      consumer_sync(ct);
-      const T sj = Xs[tid];
-      const T sl = tid > 0 ? Xs[tid - 1] : T(0);
-      chunk_back<T, K>(ch, kr, sj, sl, x);
-    }
-    if (S > 0) {
-      release_stage(&empty[s]);
-    }
-    if (sys < p.m) {
-      T* dst = gx + sys * (long)n + r0;
+  int k = n - tid * K;
+  k = k < 0 ? 0 : (k > K ? K : k);
+  int ph = 0;
+  for (long sys = blockIdx.x; sys < p.m; sys += gridDim.x, ph ^= 1) {
+    const Strip<float> s = strip(sys);
+    bool ok = true;
+    if (bulk) ok = mbar_wait(bar, ph, p.status);
+    if (s.hi < s.e1) strip_rest(s, p.in, buf, p.cap, tid, blockDim.x);
+    if (!__syncthreads_and(ok)) break;
+    const int off = (int)(s.e0 - s.lo) + tid * K;
+    Chunk<float, K> ch;
+    chunk_eliminate<float, K>(ch, k, tid == 0, k > 0 && tid * K + k == n, buf + off, buf + p.cap + off,
+                              buf + 2 * p.cap + off, buf + 3 * p.cap + off);
+    fence_proxy_async_smem();
+    const BlockForward<float> f = block_forward<float, K>(ch, W, scratch);  // (its barrier: every row is read)
+    if (bulk && tid == 0 && sys + gridDim.x < p.m) strip_issue(strip(sys + gridDim.x), p.in, buf, p.cap, bar);
+    float x[K];
+    block_back<float, K>(f, ch, k, W, 0.0f, tdiv(f.last.d, f.last.b), x);
 #pragma unroll
-      for (int i = 0; i < K; ++i)
-        if (i < kl) dst[i] = x[i];
-    }
-    if constexpr (CTA) consumer_sync(ct);  // Xs / F0 reused by the next tile
+    for (int i = 0; i < K; ++i)
+      if (i < k) xs[off + i] = x[i];
+    __syncwarp();
+    const long w0 = s.e0 + (long)warp * 32 * K, w1 = w0 + 32 * K < s.e1 ? w0 + 32 * K : s.e1;
+    strip_store(xs, s.lo, p.x, w0, w1, p.vec != 0, lane);
+    __syncwarp();
   }
 }
 
-namespace {
-
-template <class T, int K, bool CTA>
-cudaError_t launch_part(PartParams p, const DeviceInfo& dev, cudaStream_t stream) {
-  constexpr int MAXT = CTA ? 512 + 32 : 128 + 32;
-  constexpr int MINB = CTA ? 1 : 4;
-  auto kern = partition_kernel<T, K, CTA, MAXT, MINB>;
-  const bool tma_ok = aligned16(p.a) && aligned16(p.b) && aligned16(p.c) && aligned16(p.d) &&
-                      ((size_t)p.n * sizeof(T)) % 16 == 0 && !g_host_mapped_io;
-  const size_t stage = (size_t)4 * p.G * p.n * sizeof(T);
-  const size_t fixed = part_smem_bytes<T>(0, p.G, p.n, p.ct, CTA);
-  const int S = tma_ok ? pick_stages(fixed, stage, 2, dev) : 0;
-  p.stages = S;
-  const size_t smem = part_smem_bytes<T>(S, p.G, p.n, p.ct, CTA);
+template <int K>
+cudaError_t launch_warp(PartParams p, const DeviceInfo& dev, cudaStream_t stream) {
+  constexpr int MINB = K <= 9 ? 5 : K <= 15 ? 4 : K <= 21 ? 3 : 2;
+  auto kern = part_warp_kernel<K, MINB>;
+  const int G = 32 / p.lps;
+  p.cap = strip_cap<float>((long)G * p.n);
+  const size_t smem = 128 + (size_t)4 * 5 * p.cap * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, p.ct + 32, smem)) != cudaSuccess) return e;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem)) != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
+  const long tiles = ((long)p.m + G - 1) / G;
   long grid = (long)per_sm * dev.sm_count;
-  if (grid > p.ntiles) grid = p.ntiles;
-  kern<<<(unsigned)grid, p.ct + 32, smem, stream>>>(p);
+  if (grid * 4 > tiles) grid = (tiles + 3) / 4;
+  kern<<<(unsigned)grid, 128, smem, stream>>>(p);
   return cudaGetLastError();
 }
 
-int odd_ceil(int v) { return (v % 2) ? v : v + 1; }
+template <int K, int MAXT>
+cudaError_t launch_cta(PartParams p, int threads, const DeviceInfo& dev, cudaStream_t stream) {
+  auto kern = part_cta_kernel<K, MAXT, 512 / MAXT>;  // 128 registers a thread
+  p.cap = strip_cap<float>(p.n);
+  const size_t smem = 512 + (size_t)5 * p.cap * sizeof(float);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem)) != cudaSuccess) return e;
+  if (per_sm < 1) per_sm = 1;
+  long grid = (long)per_sm * dev.sm_count;
+  if (grid > p.m) grid = p.m;
+  kern<<<(unsigned)grid, threads, smem, stream>>>(p);
+  return cudaGetLastError();
+}
+
+// Lanes per system and rows a lane of the warp kernel for a system of n rows:
+// the cheapest of the shapes that hold it, by the shared-memory wavefronts and
+// instructions of a row slot and of a group's separator solve (their sums
+// order the shapes as timed at 20, 61, 100, 250 and 333 rows); lanes of
+// different systems n words apart may share banks, which counts.
+constexpr int kWarpRows[] = {3, 5, 7, 9, 11, 13, 15, 17, 21, 25, 31};
+
+void warp_shape(int n, int* lps, int* rows) {
+  double best = 1e30;
+  for (int l = 1, steps = 0; l <= 32; l *= 2, ++steps) {
+    for (int K : kWarpRows) {
+      if (l * K < n || (long)(32 / l) * n > 1100) continue;
+      int hits[32] = {};
+      int conflict = 0;
+      for (int lane = 0; lane < 32; ++lane) {
+        const int g = lane / l, t = lane % l;
+        if (t * K >= n) continue;
+        const int h = ++hits[(g * n + t * K) % 32];
+        conflict = h > conflict ? h : conflict;
+      }
+      const double slot = 24.0 + 5.0 * (conflict - 1);
+      const double cost = ((double)K * slot + 60.0 + 25.0 * steps) / ((double)(32 / l) * n);
+      if (cost < best) {
+        best = cost;
+        *lps = l;
+        *rows = K;
+      }
+    }
+  }
+}
+
+tridi_status solve_f32(const float* a, const float* b, const float* c, const float* d, float* x, int n, int m,
+                       cudaStream_t s) {
+  const DeviceInfo* dev = current_device();
+  if (!dev) return TRIDI_ERROR_CUDA;
+  PartParams p{};
+  p.in = StripIn<float>{a, b, c, d};
+  p.x = x;
+  p.n = n; p.m = m; p.total = (long)n * m; p.status = dev->status;
+  p.bulk = aligned16(a) && aligned16(b) && aligned16(c) && aligned16(d) && !g_host_mapped_io;
+  p.vec = aligned16(x);
+  if (n <= 32 * 31) {
+    int K = 31;
+    warp_shape(n, &p.lps, &K);
+    switch (K) {
+      case 3: return cuda_status(launch_warp<3>(p, *dev, s));
+      case 5: return cuda_status(launch_warp<5>(p, *dev, s));
+      case 7: return cuda_status(launch_warp<7>(p, *dev, s));
+      case 9: return cuda_status(launch_warp<9>(p, *dev, s));
+      case 11: return cuda_status(launch_warp<11>(p, *dev, s));
+      case 13: return cuda_status(launch_warp<13>(p, *dev, s));
+      case 15: return cuda_status(launch_warp<15>(p, *dev, s));
+      case 17: return cuda_status(launch_warp<17>(p, *dev, s));
+      case 21: return cuda_status(launch_warp<21>(p, *dev, s));
+      case 25: return cuda_status(launch_warp<25>(p, *dev, s));
+      default: return cuda_status(launch_warp<31>(p, *dev, s));
+    }
+  }
+  // the smallest of 4, 8 or 16 warps that hold the system at 17 rows a lane,
+  // then as few rows a lane as that takes
+  const int warps = n <= 128 * 17 ? 4 : n <= 256 * 17 ? 8 : 16;
+  const int rows = (n + warps * 32 - 1) / (warps * 32);
+  const auto by_rows = [&](auto maxt) {
+    constexpr int MAXT = decltype(maxt)::value;
+    if (rows <= 9) return launch_cta<9, MAXT>(p, warps * 32, *dev, s);
+    if (rows <= 11) return launch_cta<11, MAXT>(p, warps * 32, *dev, s);
+    if (rows <= 13) return launch_cta<13, MAXT>(p, warps * 32, *dev, s);
+    if (rows <= 15) return launch_cta<15, MAXT>(p, warps * 32, *dev, s);
+    return launch_cta<17, MAXT>(p, warps * 32, *dev, s);
+  };
+  return cuda_status(warps == 4   ? by_rows(std::integral_constant<int, 128>{})
+                     : warps == 8 ? by_rows(std::integral_constant<int, 256>{})
+                                  : by_rows(std::integral_constant<int, 512>{}));
+}
 
 }  // namespace
 
 template <class T>
 tridi_status partition_solve_device(const T* a, const T* b, const T* c, const T* d, T* x, int n, int m,
                                     tridi_stream_t stream) {
-  constexpr int kWarpMax = 31;  // rows per lane in warp mode
-  constexpr int kCtaMax = 17;   // rows per thread in CTA mode (512 threads)
   if (!a || !b || !c || !d || !x || m <= 0) return TRIDI_ERROR_INVALID_VALUE;
-  static_assert(512L * kCtaMax == partition_max_rows<float>(), "partition size cap");
   if (n < 1 || n > partition_max_rows<T>()) return TRIDI_ERROR_UNSUPPORTED_SIZE;
-  if constexpr (sizeof(T) == 8) {
-    return cr64_solve_any(a, b, c, d, x, n, m, as_stream(stream));
-  } else {
-    const DeviceInfo* dev = current_device();
-    if (!dev) return TRIDI_ERROR_CUDA;
-    PartParams p{};
-    p.a = a; p.b = b; p.c = c; p.d = d; p.x = x;
-    p.n = n; p.m = m; p.status = dev->status;
-    cudaStream_t s = as_stream(stream);
-    cudaError_t e;
-    if (n <= 32 * kWarpMax) {
-      p.kk = odd_ceil((n + 31) / 32);
-      p.ct = 128;
-      p.G = 4;
-      p.ntiles = (int)(((long)m + 3) / 4);
-      if (p.kk <= 3) e = launch_part<T, 3, false>(p, *dev, s);
-      else if (p.kk <= 7) e = launch_part<T, 7, false>(p, *dev, s);
-      else if (p.kk <= 9) e = launch_part<T, 9, false>(p, *dev, s);
-      else if (p.kk <= 15) e = launch_part<T, 15, false>(p, *dev, s);
-      else e = launch_part<T, 31, false>(p, *dev, s);
-    } else {
-      int ct = 128;
-      while (ct < 512 && odd_ceil((n + ct - 1) / ct) > 7) ct *= 2;
-      p.ct = ct;
-      p.kk = odd_ceil((n + ct - 1) / ct);
-      p.G = 1;
-      p.ntiles = m;
-      if (p.kk <= 7) e = launch_part<T, 7, true>(p, *dev, s);
-      else e = launch_part<T, kCtaMax, true>(p, *dev, s);
-    }
-    return cuda_status(e);
-  }
+  static_assert(partition_max_rows<float>() == 512L * 17, "partition size cap");
+  if constexpr (sizeof(T) == 8) return cr64_solve_any(a, b, c, d, x, n, m, as_stream(stream));
+  else return solve_f32(a, b, c, d, x, n, m, as_stream(stream));
 }
 
 template tridi_status partition_solve_device<float>(const float*, const float*, const float*, const float*, float*,
