@@ -131,4 +131,14 @@ __host__ __device__ __forceinline__ void div64x3(double a, double c, double d, d
   }
 }
 
+// Two quotients by one divisor.
+__host__ __device__ __forceinline__ void div64x2(double c, double d, double b, double& qc, double& qd) {
+  const Inv64 v = invert64(b);
+  const bool fc = quotient_fast(c, v, qc), fd = quotient_fast(d, v, qd);
+  if (!(fc && fd)) {
+    qc = quotient_ieee(c, b);
+    qd = quotient_ieee(d, b);
+  }
+}
+
 }  // namespace tridi

@@ -1,21 +1,25 @@
-// Large systems (any n, contiguous or interleaved layout): the partition
-// method across the whole GPU, in three steps on one stream.
+// Large systems (any n, contiguous or interleaved layout).  Contiguous
+// systems that one CTA holds take the uniform solver (partition.cu), longer
+// ones the block passes of large_rows.cu.  Interleaved systems (element i of
+// system s at i*m + s): the partition method across the whole GPU, in three
+// steps on one stream.
 //
 //   1. large_reduce: one thread per chunk of L rows of one system.  The chunk
 //      is eliminated in registers (partition.cuh) and its interface -- first
 //      and last interior row coefficients and the separator row, 10 values --
-//      is written out.  In the interleaved layout (element i of system s at
-//      i*m + s) a warp covers 32 consecutive systems at the same rows, so
-//      every row load is one 128-byte line.
+//      is written out.  A warp covers 32 consecutive systems at the same
+//      rows, so every row load is one 128-byte line.
 //   2. large_assemble: separator row j of system s from chunk j's interface
 //      and chunk j+1's first interior row, in the layout of the data.  The
 //      P = ceil(n/L) separators per system form a batch of the same kind,
-//      solved by the uniform partition solver (contiguous, P <= 8704 in FP32,
-//      4608 in FP64) or by
-//      this scheme again (interleaved, or larger P), down to a one-thread-
-//      per-system Thomas kernel for interleaved batches of <= 32 rows.
-//   3. large_back: each chunk is read and eliminated again and its rows
-//      recovered from the two separators around it.
+//      solved by this scheme again, down to a one-thread-per-system Thomas
+//      kernel for batches of <= 32 rows.
+//   3. large_back: each chunk is read again and solved between the two
+//      separators around it, a Thomas sweep (in FP64 3 FP64 instructions a row
+//      where the elimination has 8).
+// Steps 1 and 3 run in blocks of 128 threads (160 registers in FP64: three
+// blocks an SM; one block of 256 there: 128 x 100001 FP64 568 us, 452 us now,
+// 850 us before the Thomas sweep and the integer divisions).
 // For the interleaved FP32 layout with m a multiple of 32, steps 1 and 3 run
 // as TMA-tiled persistent kernels (large_tma.cu) on the same chunks.
 // Memory traffic per unknown: inputs read twice (2 x 16 B FP32), x written
@@ -30,6 +34,11 @@ namespace tridi {
 template <class T>
 tridi_status partition_solve_device(const T* a, const T* b, const T* c, const T* d, T* x, int n, int m,
                                     tridi_stream_t stream);
+template <class T>
+tridi_status large_rows_solve(const T* a, const T* b, const T* c, const T* d, T* x, long n, long m, void* ws,
+                              cudaStream_t st);
+template <class T>
+size_t large_rows_bytes(long n, long m);
 bool large_tma_ok(const float* a, const float* b, const float* c, const float* d, long n, long m);
 tridi_status large_tma_pass(bool back, const float* a, const float* b, const float* c, const float* d, long n,
                             long m, long P, long PMp, float* red, float* bnd, const float* sol, float* x,
@@ -43,40 +52,31 @@ struct LargeParams {
   void* x;
   long n, m;
   long P;       // chunks per system
-  int layout;   // 0 contiguous, 1 interleaved
   void* iface;  // 10 arrays of P*m interface values (stride PMp), same layout as the data
   void* red;    // 4 arrays (stride PMp): the separator system, same layout as the data
   long PMp;     // P*m rounded up to 64 elements: keeps each array 256-byte aligned
   void* sol;    // the separator solution (aliases iface), same layout
 };
 
-// Thread -> (system, chunk).  Interleaved: systems fastest; contiguous:
-// chunks fastest.  Either way consecutive threads touch consecutive
-// addresses of the interface and separator arrays, whose layout follows the
-// data's: index j*m + s (interleaved) or s*P + j (contiguous).
+// Thread -> (system, chunk), systems fastest: consecutive threads touch
+// consecutive addresses of the data and of the interface and separator
+// arrays, whose index is j*m + s.
 __device__ __forceinline__ void large_coords(const LargeParams& p, long gid, long* s, long* j) {
-  if (p.layout == 1) {
-    *s = gid % p.m;
-    *j = gid / p.m;
-  } else {
-    *j = gid % p.P;
-    *s = gid / p.P;
-  }
+  *s = gid % p.m;
+  *j = gid / p.m;
 }
-__device__ __forceinline__ long sep_index(const LargeParams& p, long s, long j) {
-  return p.layout == 1 ? j * p.m + s : s * p.P + j;
-}
+__device__ __forceinline__ long sep_index(const LargeParams& p, long s, long j) { return j * p.m + s; }
 
 template <class T, int L>
-__global__ void __launch_bounds__(256) large_reduce_kernel(LargeParams p) {
+__global__ void __launch_bounds__(128) large_reduce_kernel(LargeParams p) {
   const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= p.P * p.m) return;
   long s, j;
   large_coords(p, gid, &s, &j);
   const long r0 = j * L;
   const int k = (int)((p.n - r0) < L ? (p.n - r0) : L);
-  const long rs = p.layout == 1 ? p.m : 1;
-  const long base = p.layout == 1 ? r0 * p.m + s : s * p.n + r0;
+  const long rs = p.m;
+  const long base = r0 * p.m + s;
   Chunk<T, L> ch;
   chunk_eliminate<T, L, true>(ch, k, j == 0, j == p.P - 1, static_cast<const T*>(p.a) + base,
                         static_cast<const T*>(p.b) + base, static_cast<const T*>(p.c) + base,
@@ -111,24 +111,21 @@ __global__ void __launch_bounds__(256) large_assemble_kernel(LargeParams p) {
 }
 
 template <class T, int L>
-__global__ void __launch_bounds__(256) large_back_kernel(LargeParams p) {
+__global__ void __launch_bounds__(128) large_back_kernel(LargeParams p) {
   const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= p.P * p.m) return;
   long s, j;
   large_coords(p, gid, &s, &j);
   const long r0 = j * L;
   const int k = (int)((p.n - r0) < L ? (p.n - r0) : L);
-  const long rs = p.layout == 1 ? p.m : 1;
-  const long base = p.layout == 1 ? r0 * p.m + s : s * p.n + r0;
-  Chunk<T, L> ch;
-  chunk_eliminate<T, L, true>(ch, k, j == 0, j == p.P - 1, static_cast<const T*>(p.a) + base,
-                        static_cast<const T*>(p.b) + base, static_cast<const T*>(p.c) + base,
-                        static_cast<const T*>(p.d) + base, rs);
+  const long rs = p.m;
+  const long base = r0 * p.m + s;
   const T* sol = static_cast<const T*>(p.sol);
   const T sj = sol[sep_index(p, s, j)];
   const T sl = j > 0 ? sol[sep_index(p, s, j - 1)] : T(0);
   T x[L];
-  chunk_back<T, L>(ch, k, sj, sl, x);
+  chunk_between<T, L, true>(k, j == 0, sl, sj, static_cast<const T*>(p.a) + base, static_cast<const T*>(p.b) + base,
+                            static_cast<const T*>(p.c) + base, static_cast<const T*>(p.d) + base, rs, x);
   T* gx = static_cast<T*>(p.x) + base;
 #pragma unroll
   for (int i = 0; i < L; ++i)
@@ -151,9 +148,7 @@ __global__ void __launch_bounds__(256) thomas_interleaved_kernel(const T* __rest
     const long k = i * m + s;
     const T ai = i == 0 ? T(0) : a[k];
     const T ci = i == n - 1 ? T(0) : c[k];
-    const T inv = tdiv(T(1), b[k] - ai * cprev);
-    cprev = ci * inv;
-    dprev = (d[k] - ai * dprev) * inv;
+    tdiv2(ci, d[k] - ai * dprev, b[k] - ai * cprev, cprev, dprev);
     cp[k] = cprev;
     dp[k] = dprev;
   }
@@ -175,7 +170,8 @@ constexpr long kThomasMax = 32;
 
 long round64(long v) { return (v + 63) & ~63L; }
 
-// Workspace of one level plus the levels below it.
+// Workspace of one level plus the levels below it (for the contiguous layout
+// more than its block passes use).
 template <class T>
 size_t large_ws_bytes(long n, long m, int layout) {
   if (layout == 1 && n <= kThomasMax) return (size_t)2 * round64(n * m) * sizeof(T) + 256;
@@ -203,7 +199,12 @@ tridi_status large_solve_device(const T* a, const T* b, const T* c, const T* d, 
   if (!current_device()) return TRIDI_ERROR_CUDA;
   cudaStream_t st = as_stream(stream);
   char* w = static_cast<char*>(ws);
-  if (layout == 1 && n <= kThomasMax) {
+  if (layout == 0) {
+    if (n <= partition_max_rows<T>()) return partition_solve_device<T>(a, b, c, d, x, (int)n, (int)m, stream);
+    if (ws_bytes < large_rows_bytes<T>(n, m)) return TRIDI_ERROR_WORKSPACE_TOO_SMALL;
+    return large_rows_solve<T>(a, b, c, d, x, n, m, ws, st);
+  }
+  if (n <= kThomasMax) {
     T* cp = reinterpret_cast<T*>(w);
     T* dp = cp + round64(n * m);
     thomas_interleaved_kernel<T><<<(unsigned)((m + 255) / 256), 256, 0, st>>>(a, b, c, d, x, n, m, cp, dp);
@@ -211,7 +212,7 @@ tridi_status large_solve_device(const T* a, const T* b, const T* c, const T* d, 
   }
   LargeParams p{};
   p.a = a; p.b = b; p.c = c; p.d = d; p.x = x;
-  p.n = n; p.m = m; p.layout = layout;
+  p.n = n; p.m = m;
   p.P = (n + kChunk - 1) / kChunk;
   const long PM = p.P * m;
   p.PMp = round64(PM);
@@ -224,7 +225,7 @@ tridi_status large_solve_device(const T* a, const T* b, const T* c, const T* d, 
   // interleaved FP32 with m a multiple of 32: the TMA-tiled passes (large_tma.cu)
   bool tma = false;
   if constexpr (sizeof(T) == 4)
-    tma = layout == 1 && tunable(TRIDI_TUNE_LARGE_TMA) != 2 && !g_host_mapped_io && large_tma_ok(a, b, c, d, n, m);
+    tma = tunable(TRIDI_TUNE_LARGE_TMA) != 2 && !g_host_mapped_io && large_tma_ok(a, b, c, d, n, m);
   if (tma) {
     // the separator rows assembled in the pass (the interface area holds the
     // tile-boundary arrays only)
@@ -234,25 +235,20 @@ tridi_status large_solve_device(const T* a, const T* b, const T* c, const T* d, 
                                           nullptr, nullptr, st);
     if (t != TRIDI_SUCCESS) return t;
   } else {
-    large_reduce_kernel<T, kChunk><<<blocks, 256, 0, st>>>(p);
+    large_reduce_kernel<T, kChunk><<<(unsigned)((PM + 127) / 128), 128, 0, st>>>(p);
     large_assemble_kernel<T><<<blocks, 256, 0, st>>>(p);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_status(e);
   const T* r = static_cast<const T*>(p.red);
-  tridi_status ts;
-  if (layout == 0 && p.P <= partition_max_rows<T>())
-    ts = partition_solve_device<T>(r, r + p.PMp, r + 2 * p.PMp, r + 3 * p.PMp, static_cast<T*>(p.sol), (int)p.P,
-                                   (int)m, stream);
-  else
-    ts = large_solve_device<T>(r, r + p.PMp, r + 2 * p.PMp, r + 3 * p.PMp, static_cast<T*>(p.sol), p.P, m, layout,
-                               inner, inner_bytes, stream);
+  const tridi_status ts = large_solve_device<T>(r, r + p.PMp, r + 2 * p.PMp, r + 3 * p.PMp, static_cast<T*>(p.sol),
+                                                p.P, m, layout, inner, inner_bytes, stream);
   if (ts != TRIDI_SUCCESS) return ts;
   if (tma)
     return large_tma_pass(true, reinterpret_cast<const float*>(a), reinterpret_cast<const float*>(b),
                           reinterpret_cast<const float*>(c), reinterpret_cast<const float*>(d), n, m, p.P, p.PMp,
                           nullptr, nullptr, static_cast<const float*>(p.sol), reinterpret_cast<float*>(x), st);
-  large_back_kernel<T, kChunk><<<blocks, 256, 0, st>>>(p);
+  large_back_kernel<T, kChunk><<<(unsigned)((PM + 127) / 128), 128, 0, st>>>(p);
   return cuda_status(cudaGetLastError());
 }
 

@@ -58,10 +58,7 @@ __device__ __forceinline__ void chunk_eliminate(Chunk<T, K>& ch, int k, bool fir
                                          qd[PREFETCH ? i : 0]}
                                 : Row<T>{pa[i * rs], pb[i * rs], pc[i * rs], pd[i * rs]};
       const T a = (i == 0 && first) ? T(0) : r.a;
-      const T inv = tdiv(T(1), r.b - a * cprev);
-      ch.cp[i] = r.c * inv;
-      ch.ap[i] = (i == 0 ? a : -a * aprev) * inv;
-      ch.dp[i] = (r.d - a * dprev) * inv;
+      tdiv3(r.c, i == 0 ? a : -a * aprev, r.d - a * dprev, r.b - a * cprev, ch.cp[i], ch.ap[i], ch.dp[i]);
       cprev = ch.cp[i];
       aprev = ch.ap[i];
       dprev = ch.dp[i];
@@ -130,10 +127,8 @@ __device__ __forceinline__ void chunk_eliminate_smem(ChunkSummary<T>& cs, int k,
   T cprev = T(0), aprev = T(0), dprev = T(0);
   const auto step = [&](int i, T a0, T b0, T c0, T r) {
     const T a = (i == 0 && first) ? T(0) : a0;
-    const T inv = tdiv(T(1), b0 - a * cprev);
-    const T cn = c0 * inv;
-    const T an = (i == 0 ? a : -a * aprev) * inv;
-    const T dn = (r - a * dprev) * inv;
+    T cn, an, dn;
+    tdiv3(c0, i == 0 ? a : -a * aprev, r - a * dprev, b0 - a * cprev, cn, an, dn);
     sa[i] = an; sc[i] = cn; sd[i] = dn;
     cprev = cn; aprev = an; dprev = dn;
   };
@@ -216,6 +211,47 @@ __device__ __forceinline__ void chunk_back_smem_over_d(int k, T sj, T sl, const 
   for (int i = k - 2; i >= 0; --i) {
     xn = sd[i] - sc[i] * xn - sa[i] * sl;
     sd[i] = xn;
+  }
+}
+
+// The chunk's unknowns between its known neighbours -- sl the row before it, sj
+// its last row -- from its rows as they were read: a Thomas sweep over the
+// interior rows (the coupling to sl goes to the right-hand side), 3 operations
+// and 2 quotients a row where the elimination above takes 8 and 3.
+template <class T, int K, bool PREFETCH = false>
+__device__ __forceinline__ void chunk_between(int k, bool first, T sl, T sj, const T* pa, const T* pb, const T* pc,
+                                              const T* pd, long rs, T (&x)[K]) {
+  T qa[PREFETCH ? K : 1], qb[PREFETCH ? K : 1], qc[PREFETCH ? K : 1], qd[PREFETCH ? K : 1];
+  if constexpr (PREFETCH) {
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      if (i < k - 1) {
+        qa[i] = pa[i * rs]; qb[i] = pb[i * rs]; qc[i] = pc[i * rs]; qd[i] = pd[i * rs];
+      }
+    }
+  }
+  T cp[K], cprev = T(0), dprev = sl;  // row 0's left neighbour: x = sl - 0 x
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    if (i < k - 1) {
+      const Row<T> r = PREFETCH ? Row<T>{qa[PREFETCH ? i : 0], qb[PREFETCH ? i : 0], qc[PREFETCH ? i : 0],
+                                         qd[PREFETCH ? i : 0]}
+                                : Row<T>{pa[i * rs], pb[i * rs], pc[i * rs], pd[i * rs]};
+      const T a = (i == 0 && first) ? T(0) : r.a;
+      tdiv2(r.c, r.d - a * dprev, i == 0 ? r.b : r.b - a * cprev, cp[i], x[i]);
+      cprev = cp[i];
+      dprev = x[i];
+    }
+  }
+  T xn = sj;
+#pragma unroll
+  for (int i = K - 1; i >= 0; --i) {
+    if (i <= k - 2) {
+      xn = x[i] - cp[i] * xn;
+      x[i] = xn;
+    } else {
+      x[i] = sj;
+    }
   }
 }
 

@@ -113,11 +113,9 @@ __device__ __forceinline__ T group_pcr(Row<T> r, int width) {
 // PCR over lanes 0 .. count-1 of a warp (count <= 31) with the couplings of
 // lane 0 to the row before it and of lane count-1 to the row after it kept:
 // afterwards x = d - a (row before) - c (row after) in each of these lanes.
-// WIDTH: a power of two > count - 1.
-template <int WIDTH, class T>
+template <class T>
 __device__ __forceinline__ NRow<T> open_pcr(Row<T> r, int lane, int count) {
-#pragma unroll
-  for (int dl = 1; dl < WIDTH; dl *= 2) {
+  for (int dl = 1; dl < count; dl *= 2) {
     const NRow<T> w = normalize_row(r);
     const NRow<T> L = shfl_up(w, dl, 32), R = shfl_down(w, dl, 32);
     const bool inl = lane >= dl, inr = lane + dl < count;
@@ -151,7 +149,7 @@ __device__ __forceinline__ BlockForward<T> block_forward(const Chunk<T, K>& ch, 
   const T nA = __shfl_down_sync(kFull, ch.fA, 1);
   BlockForward<T> o;
   // lanes 0..30: separators as usual; lane 31's right side belongs to the next warp
-  o.lane = open_pcr<32>(separator_row<T, K>(ch, nD, nC, nA), lane, 31);
+  o.lane = open_pcr(separator_row<T, K>(ch, nD, nC, nA), lane, 31);
   const T pa = __shfl_up_sync(kFull, o.lane.a, 1), pc = __shfl_up_sync(kFull, o.lane.c, 1),
           pd = __shfl_up_sync(kFull, o.lane.d, 1);
   if (lane == 0) {  // the warp's first row: x = fD - fC s - fA (row before), s = lane 0's separator
@@ -176,7 +174,7 @@ __device__ __forceinline__ BlockForward<T> block_forward(const Chunk<T, K>& ch, 
     r.d -= c0 * fd;
     r.c = -c0 * fc;
   }
-  o.warp = open_pcr<16>(r, lane, W - 1);
+  o.warp = open_pcr(r, lane, W - 1);
   const T qa = __shfl_sync(kFull, o.warp.a, W - 2), qc = __shfl_sync(kFull, o.warp.c, W - 2),
           qd = __shfl_sync(kFull, o.warp.d, W - 2);
   const T la = __shfl_sync(kFull, r.a, W - 1);

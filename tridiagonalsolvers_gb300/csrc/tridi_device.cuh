@@ -27,6 +27,21 @@ __device__ __forceinline__ float rcp_approx(float v) {
 __device__ __forceinline__ float tdiv(float a, float b) { return a * rcp_approx(b); }
 __device__ __forceinline__ double tdiv(double a, double b) { return div64(a, invert64(b)); }
 
+// Several quotients by one divisor: one reciprocal (FP32: times it; FP64: each
+// quotient to nearest, div64.cuh).
+__device__ __forceinline__ void tdiv3(float x, float y, float z, float b, float& qx, float& qy, float& qz) {
+  const float inv = tdiv(1.0f, b);
+  qx = x * inv; qy = y * inv; qz = z * inv;
+}
+__device__ __forceinline__ void tdiv3(double x, double y, double z, double b, double& qx, double& qy, double& qz) {
+  div64x3(x, y, z, b, qx, qy, qz);
+}
+__device__ __forceinline__ void tdiv2(float x, float y, float b, float& qx, float& qy) {
+  const float inv = tdiv(1.0f, b);
+  qx = x * inv; qy = y * inv;
+}
+__device__ __forceinline__ void tdiv2(double x, double y, double b, double& qx, double& qy) { div64x2(x, y, b, qx, qy); }
+
 // One equation a*x[i-1] + b*x[i] + c*x[i+1] = d.
 template <class T>
 struct Row {
@@ -59,8 +74,9 @@ struct NRow {
 };
 template <class T>
 __device__ __forceinline__ NRow<T> normalize_row(const Row<T>& r) {
-  const T ib = tdiv(T(1), r.b);
-  return {r.a * ib, r.c * ib, r.d * ib};
+  NRow<T> w;
+  tdiv3(r.a, r.c, r.d, r.b, w.a, w.c, w.d);
+  return w;
 }
 
 // reduce_row with the neighbours given as normalised rows:
