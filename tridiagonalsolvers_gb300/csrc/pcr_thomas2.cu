@@ -1,5 +1,5 @@
 // PCR-then-Thomas ("pcrGauss", pcrGauss_kernel.cu:1-126, pcrGauss_app.cu:164)
-// for FP32 systems of 64..1024 unknowns (power of two) in registers, on the
+// for FP32 systems of 32..1024 unknowns (power of two) in registers, on the
 // two-phase layout of pcr_twophase.cuh.
 //
 // log2(G) PCR steps (distances 1, 2, ..., G/2) leave G independent chains of
@@ -13,6 +13,9 @@
 // lane's registers, two chains per paired FP32 instruction where a lane holds
 // more than one, and x leaves from them as the two-phase kernel's does.
 //
+// (32 unknowns, two lanes a system: 524288 systems, g = 8, 71 us; 257 us on the
+// shared-memory kernel.)
+//
 // G is the caller's split g where g >= LPS.  A smaller g would leave chains
 // spread over several lanes; there G = LPS: the extra PCR steps keep the
 // solution exact (after any number of PCR steps the chains solve the same
@@ -20,6 +23,7 @@
 // reference's own tables often take fewer steps than log2(g), and its result
 // is then an approximation: pcrGauss_app.cu:12-96.)
 #include "hybrid.cuh"
+#include "pcr_thomas2.cuh"
 #include "pcr_twophase.cuh"
 #include "runtime.h"
 
@@ -28,60 +32,6 @@ namespace tridi {
 namespace {
 
 using namespace pcr2;
-
-// Thomas on the lane's chains: KG chains of R / KG rows, chain s0 in slots
-// s0 + KG * k (normalised rows: a x_prev + x + c x_next = d).  dst: the
-// lane's first unknown; slot s is unknown LPS * s.
-template <int R, int KG, int LPS>
-__device__ __forceinline__ void thomas_pairs(NR2 (&P)[R / 2], float* dst, bool store) {
-  constexpr int KP = KG / 2;  // chain pairs (slots 2 j', 2 j' + 1 of pair j')
-  constexpr int L = R / KG;   // rows per chain
-#pragma unroll
-  for (int jp = 0; jp < KP; ++jp) {
-    float2 cp = P[jp].c, dp = P[jp].d;
-#pragma unroll
-    for (int k = 1; k < L; ++k) {
-      NR2& r = P[jp + KP * k];
-      const float2 na = neg2(r.a);
-      const float2 inv = rcp_approx2(__ffma2_rn(na, cp, make_float2(1.0f, 1.0f)));
-      cp = __fmul2_rn(r.c, inv);
-      dp = __fmul2_rn(__ffma2_rn(na, dp, r.d), inv);
-      r.c = cp;
-      r.d = dp;
-    }
-    float2 x = dp;
-#pragma unroll
-    for (int k = L - 1; k >= 0; --k) {
-      const int j = jp + KP * k;
-      if (k < L - 1) x = __ffma2_rn(neg2(P[j].c), x, P[j].d);
-      if (store) {
-        dst[LPS * (2 * j)] = x.x;
-        dst[LPS * (2 * j + 1)] = x.y;
-      }
-    }
-  }
-}
-
-// One chain a lane (G = LPS): slots 0 .. R-1 in order.
-template <int R, int LPS>
-__device__ __forceinline__ void thomas_single(NR (&w)[R], float* dst, bool store) {
-  float cp = w[0].c, dp = w[0].d;
-#pragma unroll
-  for (int s = 1; s < R; ++s) {
-    const float inv = rcp_approx(fmaf(-w[s].a, cp, 1.0f));
-    cp = w[s].c * inv;
-    dp = fmaf(-w[s].a, dp, w[s].d) * inv;
-    w[s].c = cp;
-    w[s].d = dp;
-  }
-  float x = dp;
-  if (store) dst[LPS * (R - 1)] = x;
-#pragma unroll
-  for (int s = R - 2; s >= 0; --s) {
-    x = fmaf(-w[s].c, x, w[s].d);
-    if (store) dst[LPS * s] = x;
-  }
-}
 
 // One launch: every warp streams its own tiles of 32/LPS systems (the tile
 // pipeline of pcr_twophase_kernel).
@@ -94,7 +44,7 @@ __global__ void __launch_bounds__(Pcr2Shape<N>::WARPS * 32, 3)
   constexpr int BUF = 4 * TF;
   constexpr int SYS_STRIDE = S::SYS_STRIDE;
   constexpr int KG = G / LPS;  // chains a lane
-  static_assert(N >= 64 && N <= 1024 && SPW * N == TF, "pcr_thomas2: 64 <= n <= 1024");
+  static_assert(N >= 32 && N <= 1024 && SPW * N == TF, "pcr_thomas2: 32 <= n <= 1024");
   static_assert(G >= LPS && G % LPS == 0 && G <= N / 4 && (KG == 1 || KG % 2 == 0), "pcr_thomas2: split");
   extern __shared__ __align__(128) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -158,9 +108,10 @@ __global__ void __launch_bounds__(Pcr2Shape<N>::WARPS * 32, 3)
                  __fmul2_rn(make_float2(v[3][2 * j], v[3][2 * j + 1]), ib)};
     }
     // ---- phase A: distances 1 .. min(G, R) / 2 ----
-    phase_a_step1_pairs<LPS, R>(P);
-    if constexpr (2 <= G / 2) phase_a_step_pairs<1, LPS, R>(P);
-    if constexpr (4 <= G / 2) phase_a_step_pairs<2, LPS, R>(P);
+    constexpr bool FINE = N == 32;  // no further from FP64 than the shared-memory kernel it stands in for
+    phase_a_step1_pairs<LPS, R, FINE>(P);
+    if constexpr (2 <= G / 2) phase_a_step_pairs<1, LPS, R, FINE>(P);
+    if constexpr (4 <= G / 2) phase_a_step_pairs<2, LPS, R, FINE>(P);
     if constexpr (8 <= G / 2 && 8 <= R / 2) phase_a_step_pairs<4, LPS, R>(P);
     if constexpr (16 <= G / 2 && 16 <= R / 2) phase_a_step_pairs<8, LPS, R>(P);
     // ---- transpose: lane t of system g takes rows t + LPS * s ----
@@ -186,6 +137,9 @@ __global__ void __launch_bounds__(Pcr2Shape<N>::WARPS * 32, 3)
       if constexpr (4 * R <= G / 2) phase_b_pairs<4 * R / LPS, R>(P);
     }
     // ---- Thomas on the lane's chains ----
+    const auto emit = [&](int s, float v) {
+      if (store) dst[LPS * s] = v;
+    };
     if constexpr (KG == 1) {
       NR w[R];
 #pragma unroll
@@ -193,9 +147,9 @@ __global__ void __launch_bounds__(Pcr2Shape<N>::WARPS * 32, 3)
         w[2 * j] = row_x(P[j]);
         w[2 * j + 1] = row_y(P[j]);
       }
-      thomas_single<R, LPS>(w, dst, store);
+      thomas_single<R>(w, emit);
     } else {
-      thomas_pairs<R, KG, LPS>(P, dst, store);
+      thomas_pairs<R, KG>(P, emit);
     }
   }
 }
@@ -244,11 +198,13 @@ cudaError_t launch_for_n(const HybridParams& p, int g, const DeviceInfo& dev, cu
 }  // namespace
 
 // True when the register kernel takes this FP32 call: n a power of two in
-// 64 .. 1024, g < n/2 (g >= n/2 is the full PCR kernel's), 16-byte aligned
-// contiguous arrays, the batch within the tensor maps' 32-bit row count.
+// 32 .. 1024, g < n/2 (g >= n/2 is the full PCR kernel's; 32 rows: from four
+// chains on, with one or two the shared-memory kernel's Thomas on unreduced
+// rows rounds less), 16-byte aligned contiguous arrays, the batch within the
+// tensor maps' 32-bit row count.
 bool pcr_thomas2_applies(const void* a, const void* b, const void* c, const void* d, int n, long m, int g) {
-  return (n == 64 || n == 128 || n == 256 || n == 512 || n == 1024) && g >= 1 && g < n / 2 && aligned16(a) &&
-         aligned16(b) && aligned16(c) && aligned16(d) && m * n / 32 < (1L << 31) &&
+  return ((n == 32 && g >= 4) || n == 64 || n == 128 || n == 256 || n == 512 || n == 1024) && g >= 1 && g < n / 2 &&
+         aligned16(a) && aligned16(b) && aligned16(c) && aligned16(d) && m * n / 32 < (1L << 31) &&
          tunable(TRIDI_TUNE_PCR_KERNEL) != 2 && !g_host_mapped_io;
 }
 
@@ -262,6 +218,7 @@ tridi_status pcr_thomas2_solve(const float* a, const float* b, const float* c, c
   p.status = dev->status;
   cudaError_t e = cudaErrorInvalidValue;
   switch (n) {
+    case 32: e = launch_for_n<32>(p, g, *dev, stream); break;
     case 64: e = launch_for_n<64>(p, g, *dev, stream); break;
     case 128: e = launch_for_n<128>(p, g, *dev, stream); break;
     case 256: e = launch_for_n<256>(p, g, *dev, stream); break;

@@ -87,6 +87,26 @@ __device__ __forceinline__ NR2 step_both2(const NR2& me, const NR2& L, const NR2
   const float2 ib = rcp_approx2(b);
   return {__fmul2_rn(__fmul2_rn(na, L.a), ib), __fmul2_rn(__fmul2_rn(nc, R.c), ib), __fmul2_rn(d, ib)};
 }
+// step_both / step_both2 with less rounding.  The new diagonal is 1 - u, u =
+// me.a L.c + me.c R.a; the row is divided by it as row + row * e, e = u / (1 -
+// u), so that the reciprocal's rounding enters scaled by u (below 1/2 for
+// dominant rows) and not in full.
+__device__ __forceinline__ NR fine_step(const NR& me, const NR& L, const NR& R) {
+  const float u = fmaf(me.c, R.a, me.a * L.c);
+  const float e = u * rcp_approx(1.0f - u);
+  const float d = fmaf(-me.c, R.d, fmaf(-me.a, L.d, me.d));
+  const float ta = -me.a * L.a, tc = -me.c * R.c;
+  return {fmaf(ta, e, ta), fmaf(tc, e, tc), fmaf(d, e, d)};
+}
+__device__ __forceinline__ NR2 fine_step2(const NR2& me, const NR2& L, const NR2& R) {
+  const float2 na = neg2(me.a), nc = neg2(me.c);
+  const float2 u = __ffma2_rn(me.c, R.a, __fmul2_rn(me.a, L.c));
+  const float2 e = __fmul2_rn(u, rcp_approx2(__fadd2_rn(make_float2(1.0f, 1.0f), neg2(u))));
+  const float2 d = __ffma2_rn(nc, R.d, __ffma2_rn(na, L.d, me.d));
+  const float2 ta = __fmul2_rn(na, L.a), tc = __fmul2_rn(nc, R.c);
+  return {__ffma2_rn(ta, e, ta), __ffma2_rn(tc, e, tc), __ffma2_rn(d, e, d)};
+}
+
 __device__ __forceinline__ NR2 step_right2(const NR2& me, const NR2& R) {
   const float2 nc = neg2(me.c);
   const float2 b = __ffma2_rn(nc, R.a, make_float2(1.0f, 1.0f));
@@ -188,7 +208,7 @@ __device__ __forceinline__ void phase_b_xor16(NR (&w)[R], int lane) {
 // ---- row pairs P[j] = rows (2j, 2j+1) -------------------------------------
 // Distance 1 (phase A) and slot distance 1 (phase B) pair a row with halves
 // of two different pairs; those steps run on single rows.
-template <int LPS, int R>
+template <int LPS, int R, bool FINE = false>
 __device__ __forceinline__ void phase_a_step1_pairs(NR2 (&P)[R / 2]) {
   constexpr int NP = R / 2;
   const NR fromL = shfl_up_nr(row_y(P[NP - 1]), LPS);  // previous lane's last row
@@ -196,15 +216,16 @@ __device__ __forceinline__ void phase_a_step1_pairs(NR2 (&P)[R / 2]) {
   NR2 o[NP];
 #pragma unroll
   for (int j = 0; j < NP; ++j) {
-    const NR lo = step_both(row_x(P[j]), j > 0 ? row_y(P[j - 1]) : fromL, row_y(P[j]));
-    const NR hi = step_both(row_y(P[j]), row_x(P[j]), j + 1 < NP ? row_x(P[j + 1]) : fromR);
+    const NR l = j > 0 ? row_y(P[j - 1]) : fromL, r = j + 1 < NP ? row_x(P[j + 1]) : fromR;
+    const NR lo = FINE ? fine_step(row_x(P[j]), l, row_y(P[j])) : step_both(row_x(P[j]), l, row_y(P[j]));
+    const NR hi = FINE ? fine_step(row_y(P[j]), row_x(P[j]), r) : step_both(row_y(P[j]), row_x(P[j]), r);
     o[j] = pair_of(lo, hi);
   }
 #pragma unroll
   for (int j = 0; j < NP; ++j) P[j] = o[j];
 }
 // Distance 2*DP rows (DP whole pairs) on contiguous rows.
-template <int DP, int LPS, int R>
+template <int DP, int LPS, int R, bool FINE = false>
 __device__ __forceinline__ void phase_a_step_pairs(NR2 (&P)[R / 2]) {
   constexpr int NP = R / 2;
   NR2 o[NP];
@@ -216,7 +237,7 @@ __device__ __forceinline__ void phase_a_step_pairs(NR2 (&P)[R / 2]) {
     for (int q = j; q < NP; q += DP) {
       const NR2& L = q >= DP ? P[q - DP] : fromL;
       const NR2& Rr = q + DP < NP ? P[q + DP] : fromR;
-      o[q] = step_both2(P[q], L, Rr);
+      o[q] = FINE ? fine_step2(P[q], L, Rr) : step_both2(P[q], L, Rr);
     }
   }
 #pragma unroll
@@ -309,7 +330,10 @@ struct Pcr2Shape {
   static constexpr int SPW = 32 / LPS;           // systems per warp tile
   static constexpr int TF = 32 * R;              // values of one array in a warp tile (= SPW * N)
   static constexpr int WARPS = R == 32 ? 2 : 4;  // warps per CTA
-  static constexpr int SYS_STRIDE = N + LPS;     // transpose scratch per system (padded: no bank conflicts)
+  // transpose scratch per system (padded: no bank conflicts; whole 16-byte
+  // groups, which its stores move)
+  static constexpr int SYS_STRIDE = N + (LPS < 4 ? 4 : LPS);
+  static_assert(SYS_STRIDE % 4 == 0, "16-byte stores into the transpose scratch");
   static constexpr int SCRATCH = SPW * SYS_STRIDE;  // floats per warp
   static constexpr size_t SMEM = 128 + (size_t)WARPS * SCRATCH * sizeof(float) + 1024 +
                                  (size_t)WARPS * 4 * TF * sizeof(float);

@@ -49,6 +49,10 @@ long ragged_team_max_rows();
 bool pcr_thomas2_applies(const void* a, const void* b, const void* c, const void* d, int n, long m, int g);
 tridi_status pcr_thomas2_solve(const float* a, const float* b, const float* c, const float* d, float* x, int n,
                                int m, int g, cudaStream_t stream);
+// PCR (g >= n/2) and PCR-then-Thomas at 2048 and 4096 unknowns (pcr_wide.cu).
+bool pcr_wide_applies(const void* a, const void* b, const void* c, const void* d, int n, long m, int g);
+tridi_status pcr_wide_solve(const float* a, const float* b, const float* c, const float* d, float* x, int n, int m,
+                            int g, cudaStream_t stream);
 // cr and crpcr at every switch level for 512 and 1024 unknowns, in registers
 // (crpcr2.cu); stride = n / rest.
 bool crpcr_regs_applies(const void* a, const void* b, const void* c, const void* d, const void* x, int n, long m,
