@@ -457,18 +457,14 @@ cudaError_t launch_cr64(Cr64Params p, const DeviceInfo& dev, cudaStream_t stream
   int ct = p.tps > 128 ? (p.tps + 31) / 32 * 32 : 128;
   while (ct > 32 && ct / 2 >= p.tps && (long)p.m * p.tps < 2L * dev.sm_count * ct) ct /= 2;
   const size_t smem = cr64_smem(ct, LS > 0 ? K / (LS > 0 ? LS : 1) : 1);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ct, smem);
+  const cudaError_t e = resident_blocks(kern, ct, smem, dev, &per_sm);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
   const int G = ct / p.tps;
   p.ntiles = (int)(((long)p.m + G - 1) / G);
   long grid = (long)per_sm * dev.sm_count;
   if (grid > p.ntiles) grid = p.ntiles;
-  kern<<<(unsigned)grid, ct, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_kernel(kern, (unsigned)grid, ct, smem, stream, p);
 }
 
 }  // namespace

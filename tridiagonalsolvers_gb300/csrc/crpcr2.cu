@@ -475,17 +475,13 @@ using TileKernel = void (*)(HybridParams, CUtensorMap, CUtensorMap, CUtensorMap,
 tridi_status launch_tiles(TileKernel kern, size_t smem, int max_per_sm, const HybridParams& p,
                           const CUtensorMap* tm, const DeviceInfo* dev, cudaStream_t stream) {
   if (smem > (size_t)dev->max_smem_optin) return TRIDI_ERROR_UNSUPPORTED_SIZE;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_status(e);
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarps * 32, smem);
+  const cudaError_t e = resident_blocks(kern, kWarps * 32, smem, *dev, &per_sm);
   if (e != cudaSuccess) return cuda_status(e);
-  if (per_sm < 1) per_sm = 1;
   if (per_sm > max_per_sm) per_sm = max_per_sm;
   long grid = (long)per_sm * dev->sm_count;
   if (grid * kWarps > p.m) grid = (p.m + kWarps - 1) / kWarps;
-  kern<<<(unsigned)grid, kWarps * 32, smem, stream>>>(p, tm[0], tm[1], tm[2], tm[3]);
-  return cuda_status(cudaGetLastError());
+  return cuda_status(launch_kernel(kern, (unsigned)grid, kWarps * 32, smem, stream, p, tm[0], tm[1], tm[2], tm[3]));
 }
 
 template <int N>

@@ -47,17 +47,13 @@ cudaError_t launch_warp_streams(const HybridParams& p, const DeviceInfo& dev, cu
   const int warps = kWarpKernelThreads / 32;
   const size_t smem = HybridSmem<T>::barrier_bytes() + (size_t)warps * 2 * HybridSmem<T>::stage_elems(32 / p.tps, p.n) * sizeof(T);
   if (smem > (size_t)dev.max_smem_optin) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarpKernelThreads, smem);
+  const cudaError_t e = resident_blocks(kern, kWarpKernelThreads, smem, dev, &per_sm);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
   const long tiles = ((long)p.m + 32 / p.tps - 1) / (32 / p.tps);
   long grid = (long)per_sm * dev.sm_count;
   if (grid * warps > tiles) grid = (tiles + warps - 1) / warps;
-  kern<<<(unsigned)grid, kWarpKernelThreads, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_kernel(kern, (unsigned)grid, kWarpKernelThreads, smem, stream, p);
 }
 
 // Block shapes with one 128-thread CTA of groups (tps 64 or 128) and
@@ -68,16 +64,12 @@ cudaError_t launch_block_streams(const HybridParams& p, const DeviceInfo& dev, c
   auto kern = hybrid_block_stream_kernel<T, K, LSTRIDE, 128, MINB>;
   const size_t smem = HybridSmem<T>::bytes(2, p.G, p.n, p.scratch_rows, false, p.ct, Log2<K>::value);
   if (smem > (size_t)dev.max_smem_optin) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, p.ct, smem);
+  const cudaError_t e = resident_blocks(kern, p.ct, smem, dev, &per_sm);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
   long grid = (long)per_sm * dev.sm_count;
   if (grid > p.ntiles) grid = p.ntiles;
-  kern<<<(unsigned)grid, p.ct, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_kernel(kern, (unsigned)grid, p.ct, smem, stream, p);
 }
 
 template <class T, int K, bool WARP, int LSTRIDE>
@@ -102,17 +94,13 @@ cudaError_t launch_one(const HybridParams& p0, const DeviceInfo& dev, cudaStream
   const int S = tma_ok ? pick_stages(fixed, stage_bytes, 2, dev) : 0;
   p.stages = S;
   const size_t smem = HybridSmem<T>::bytes(S, p.G, p.n, p.scratch_rows, WARP, p.ct, logk);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   const int threads = p.ct + 32;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+  const cudaError_t e = resident_blocks(kern, threads, smem, dev, &per_sm);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
   long grid = (long)per_sm * dev.sm_count;
   if (grid > p.ntiles) grid = p.ntiles;
-  kern<<<(unsigned)grid, threads, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_kernel(kern, (unsigned)grid, threads, smem, stream, p);
 }
 
 // FP32 PCR on 64..1024 unknowns: the two-phase kernel (pcr_twophase.cuh).
@@ -131,17 +119,13 @@ cudaError_t launch_pcr_twophase(const HybridParams& p, const DeviceInfo& dev, cu
       !make_tensor_map_2d(&md, static_cast<const float*>(p.d), 32, rows, 128, 32, S::R, true))
     return cudaErrorInvalidValue;
   if (S::SMEM > (size_t)dev.max_smem_optin) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-  if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, S::SMEM);
+  const cudaError_t e = resident_blocks(kern, kThreads, S::SMEM, dev, &per_sm);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
   const long tiles = ((long)p.m + S::SPW - 1) / S::SPW;
   long grid = (long)per_sm * dev.sm_count;
   if (grid * S::WARPS > tiles) grid = (tiles + S::WARPS - 1) / S::WARPS;
-  kern<<<(unsigned)grid, kThreads, S::SMEM, stream>>>(p, ma, mb, mc, md);
-  return cudaGetLastError();
+  return launch_kernel(kern, (unsigned)grid, kThreads, S::SMEM, stream, p, ma, mb, mc, md);
 }
 
 bool pcr_twophase_applies(const HybridParams& p) {

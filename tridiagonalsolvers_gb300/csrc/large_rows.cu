@@ -182,15 +182,12 @@ cudaError_t launch_rows(const RowsParams<T>& p, const DeviceInfo& dev, cudaStrea
   using S = RowsShape<T, K>;
   auto kern = rows_kernel<T, K, BACK, MINB>;
   const size_t smem = S::smem(BACK);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   int per_sm = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarps, smem)) != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
+  const cudaError_t e = resident_blocks(kern, 32 * kWarps, smem, dev, &per_sm);
+  if (e != cudaSuccess) return e;
   long grid = (long)per_sm * dev.sm_count;
   if (grid > p.NB * p.m) grid = p.NB * p.m;
-  kern<<<(unsigned)grid, 32 * kWarps, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_kernel(kern, (unsigned)grid, 32 * kWarps, smem, st, p);
 }
 
 template <class T>

@@ -294,18 +294,15 @@ tridi_status large_tma_pass(bool back, const float* a, const float* b, const flo
   const long ntiles = (long)p.row_tiles * p.col_tiles;
   int grid = dev->sm_count;
   if (grid > ntiles) grid = (int)ntiles;
-  cudaError_t e;
+  int per_sm = 0;
+  cudaError_t e = back ? resident_blocks(large_tile_kernel<true>, 32 * (kLtWarps + 1), smem, *dev, &per_sm)
+                       : resident_blocks(large_tile_kernel<false>, 32 * (kLtWarps + 1), smem, *dev, &per_sm);
+  if (e != cudaSuccess) return cuda_status(e);
   if (back) {
-    if ((e = cudaFuncSetAttribute(large_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)kLtSmem)) != cudaSuccess)
-      return cuda_status(e);
-    large_tile_kernel<true><<<grid, 32 * (kLtWarps + 1), kLtSmem, st>>>(p, ma, mb, mc, md);
+    return cuda_status(launch_kernel(large_tile_kernel<true>, (unsigned)grid, 32 * (kLtWarps + 1), smem, st, p, ma, mb, mc, md));
   } else {
-    if ((e = cudaFuncSetAttribute(large_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem)) != cudaSuccess)
-      return cuda_status(e);
-    large_tile_kernel<false><<<grid, 32 * (kLtWarps + 1), smem, st>>>(p, ma, mb, mc, md);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
+    e = launch_kernel(large_tile_kernel<false>, (unsigned)grid, 32 * (kLtWarps + 1), smem, st, p, ma, mb, mc, md);
+    if (e != cudaSuccess) return cuda_status(e);
     const long cnt = (long)p.row_tiles * m;
     large_tile_boundary_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(p);
   }

@@ -60,17 +60,13 @@ tridi_status solve_nbc(const float* a, const float* b, const float* c, const flo
   p.ntiles = (int)(((long)m + G - 1) / G);
   const size_t smem = NbcSmem<T>::bytes(S, G, n, rest);
   auto kern = nbc_kernel<T, kMaxThreads, 5>;  // 5 CTAs (20 solving warps) per SM
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_status(e);
   const int threads = 32 * G + 32;
   int per_sm = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem)) != cudaSuccess)
-    return cuda_status(e);
-  if (per_sm < 1) per_sm = 1;
+  const cudaError_t e = resident_blocks(kern, threads, smem, *dev, &per_sm);
+  if (e != cudaSuccess) return cuda_status(e);
   long grid = (long)per_sm * dev->sm_count;
   if (grid > p.ntiles) grid = p.ntiles;
-  kern<<<(unsigned)grid, threads, smem, as_stream(stream)>>>(p);
-  return cuda_status(cudaGetLastError());
+  return cuda_status(launch_kernel(kern, (unsigned)grid, threads, smem, as_stream(stream), p));
 }
 
 // FP64: the shared-memory CR of cr64.cu (dense arrays at every level across

@@ -139,16 +139,13 @@ cudaError_t launch_warp(PartParams p, const DeviceInfo& dev, cudaStream_t stream
   const int G = 32 / p.lps;
   p.cap = strip_cap<float>((long)G * p.n);
   const size_t smem = 128 + (size_t)4 * 5 * p.cap * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   int per_sm = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem)) != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
+  const cudaError_t e = resident_blocks(kern, 128, smem, dev, &per_sm);
+  if (e != cudaSuccess) return e;
   const long tiles = ((long)p.m + G - 1) / G;
   long grid = (long)per_sm * dev.sm_count;
   if (grid * 4 > tiles) grid = (tiles + 3) / 4;
-  kern<<<(unsigned)grid, 128, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_kernel(kern, (unsigned)grid, 128, smem, stream, p);
 }
 
 template <int K, int MAXT>
@@ -156,15 +153,12 @@ cudaError_t launch_cta(PartParams p, int threads, const DeviceInfo& dev, cudaStr
   auto kern = part_cta_kernel<K, MAXT, 512 / MAXT>;  // 128 registers a thread
   p.cap = strip_cap<float>(p.n);
   const size_t smem = 512 + (size_t)5 * p.cap * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   int per_sm = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem)) != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
+  const cudaError_t e = resident_blocks(kern, threads, smem, dev, &per_sm);
+  if (e != cudaSuccess) return e;
   long grid = (long)per_sm * dev.sm_count;
   if (grid > p.m) grid = p.m;
-  kern<<<(unsigned)grid, threads, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_kernel(kern, (unsigned)grid, threads, smem, stream, p);
 }
 
 // Lanes per system and rows a lane of the warp kernel for a system of n rows:

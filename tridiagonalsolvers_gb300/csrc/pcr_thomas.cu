@@ -257,16 +257,12 @@ tridi_status pcr_thomas_device(const T* a, const T* b, const T* c, const T* d, T
               : rows <= 4 ? pcr_thomas_kernel<T, 288, 4>
               : rows <= 8 ? pcr_thomas_kernel<T, 288, 8>
                           : pcr_thomas_kernel<T, 288, 16>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_status(e);
   int per_sm = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, p.ct + 32, smem)) != cudaSuccess)
-    return cuda_status(e);
-  if (per_sm < 1) per_sm = 1;
+  const cudaError_t e = resident_blocks(kern, p.ct + 32, smem, *dev, &per_sm);
+  if (e != cudaSuccess) return cuda_status(e);
   long grid = (long)per_sm * dev->sm_count;
   if (grid > p.ntiles) grid = p.ntiles;
-  kern<<<(unsigned)grid, p.ct + 32, smem, as_stream(stream)>>>(p);
-  return cuda_status(cudaGetLastError());
+  return cuda_status(launch_kernel(kern, (unsigned)grid, p.ct + 32, smem, as_stream(stream), p));
 }
 
 template tridi_status pcr_thomas_device<float>(const float*, const float*, const float*, const float*, float*, int,

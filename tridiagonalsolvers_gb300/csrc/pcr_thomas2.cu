@@ -167,17 +167,13 @@ cudaError_t launch_pcr_thomas2(const HybridParams& p, const DeviceInfo& dev, cud
       !make_tensor_map_2d(&md, static_cast<const float*>(p.d), 32, rows, 128, 32, S::R, true))
     return cudaErrorInvalidValue;
   if (S::SMEM > (size_t)dev.max_smem_optin) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-  if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, S::SMEM);
+  const cudaError_t e = resident_blocks(kern, kThreads, S::SMEM, dev, &per_sm);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
   const long tiles = ((long)p.m + S::SPW - 1) / S::SPW;
   long grid = (long)per_sm * dev.sm_count;
   if (grid * S::WARPS > tiles) grid = (tiles + S::WARPS - 1) / S::WARPS;
-  kern<<<(unsigned)grid, kThreads, S::SMEM, stream>>>(p, ma, mb, mc, md);
-  return cudaGetLastError();
+  return launch_kernel(kern, (unsigned)grid, kThreads, S::SMEM, stream, p, ma, mb, mc, md);
 }
 
 // G from the caller's g (raised to LPS), for n and G with an instantiated kernel.

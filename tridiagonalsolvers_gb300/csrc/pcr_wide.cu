@@ -270,16 +270,12 @@ cudaError_t launch_wide(const HybridParams& p, const DeviceInfo& dev, cudaStream
       !make_tensor_map_2d(&md, static_cast<const float*>(p.d), 32, rows, 128, 32, kR, true))
     return cudaErrorInvalidValue;
   if (S::SMEM > (size_t)dev.max_smem_optin) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-  if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, M * 32, S::SMEM);
+  const cudaError_t e = resident_blocks(kern, M * 32, S::SMEM, dev, &per_sm);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
   long grid = (long)per_sm * dev.sm_count;
   if (grid > p.m) grid = p.m;
-  kern<<<(unsigned)grid, M * 32, S::SMEM, stream>>>(p, ma, mb, mc, md);
-  return cudaGetLastError();
+  return launch_kernel(kern, (unsigned)grid, M * 32, S::SMEM, stream, p, ma, mb, mc, md);
 }
 
 template <int M>

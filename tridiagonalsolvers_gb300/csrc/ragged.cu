@@ -1263,9 +1263,9 @@ tridi_status ragged_launch(const RaggedPlan* plan, void* dev_plan, RagParams& p,
   const size_t smem = rag_smem_bytes(MODE);
   if (smem > (size_t)dev->max_smem_optin) return TRIDI_ERROR_UNSUPPORTED_SIZE;
   const auto kernel = plan->needs_big(ring_rows(MODE)) ? ragged_kernel<MODE, true> : ragged_kernel<MODE, false>;
-  cudaError_t e;
-  if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
-    return cuda_status(e);
+  int per_sm = 0;
+  const cudaError_t e = resident_blocks(kernel, kRagThreads + 32, smem, *dev, &per_sm);
+  if (e != cudaSuccess) return cuda_status(e);
   char* dp = static_cast<char*>(dev_plan);
   p.items = reinterpret_cast<const RagItem*>(dp + 64);
   p.sys = reinterpret_cast<const RagSys*>(dp + 64 + plan->items.size() * sizeof(RagItem));
@@ -1273,8 +1273,7 @@ tridi_status ragged_launch(const RaggedPlan* plan, void* dev_plan, RagParams& p,
   p.status = dev->status;
   int grid = dev->sm_count;
   if (grid > p.nitems) grid = p.nitems;
-  kernel<<<grid, kRagThreads + 32, smem, st>>>(p);
-  return cuda_status(cudaGetLastError());
+  return cuda_status(launch_kernel(kernel, (unsigned)grid, kRagThreads + 32, smem, st, p));
 }
 
 long pad4(long v) { return (v + 3) & ~3L; }

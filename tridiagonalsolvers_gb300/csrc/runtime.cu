@@ -73,6 +73,36 @@ const DeviceInfo* current_device() {
   return &d;
 }
 
+cudaError_t raise_smem_limit(const void* kern, size_t smem, const DeviceInfo& dev) {
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.max_smem_optin) == cudaSuccess)
+    return cudaSuccess;
+  cudaGetLastError();
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
+cudaError_t resident_blocks(const void* kern, int threads, size_t smem, const DeviceInfo& dev, int* per_sm) {
+  struct Entry {
+    const void* kern;
+    size_t smem;
+    int threads, device, per_sm;
+  };
+  static thread_local Entry table[256] = {};
+  const size_t h = (reinterpret_cast<uintptr_t>(kern) >> 4) * 31 + smem / 16 * 7 + (size_t)threads / 32 + (size_t)dev.device * 13;
+  Entry& t = table[(h ^ (h >> 8)) % 256];
+  if (t.kern == kern && t.smem == smem && t.threads == threads && t.device == dev.device && t.per_sm > 0) {
+    *per_sm = t.per_sm;
+    return cudaSuccess;
+  }
+  cudaError_t e = raise_smem_limit(kern, smem, dev);
+  if (e != cudaSuccess) return e;
+  int n = 0;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem)) != cudaSuccess) return e;
+  if (n < 1) n = 1;
+  t = Entry{kern, smem, threads, dev.device, n};
+  *per_sm = n;
+  return cudaSuccess;
+}
+
 namespace {
 // The driver's tensor-map encoder, looked up through the runtime once (the
 // library does not link the driver library itself, so it loads on machines

@@ -29,6 +29,35 @@ tridi_status cuda_status(cudaError_t e);
 
 inline cudaStream_t as_stream(tridi_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// CTAs of `threads` threads and `smem` bytes of dynamic shared memory that one
+// SM holds of the kernel (at least 1).  The first call of a thread for a shape
+// raises the kernel's shared-memory limit to the device's and asks the
+// runtime; later ones find the answer in a table of the thread (the two calls
+// took 1 to 2 us of each launch).
+cudaError_t resident_blocks(const void* kern, int threads, size_t smem, const DeviceInfo& dev, int* per_sm);
+template <class... P>
+cudaError_t resident_blocks(void (*kern)(P...), int threads, size_t smem, const DeviceInfo& dev, int* per_sm) {
+  return resident_blocks(reinterpret_cast<const void*>(kern), threads, smem, dev, per_sm);
+}
+// Raises the kernel's dynamic shared-memory limit to the device's (or to
+// `smem`, where it has static shared memory too).
+cudaError_t raise_smem_limit(const void* kern, size_t smem, const DeviceInfo& dev);
+
+// Launch of a kernel that resident_blocks() has seen.  A device reset drops
+// the raised limit; the launch then fails and is repeated with the limit set.
+template <class... P, class... A>
+cudaError_t launch_kernel(void (*kern)(P...), unsigned grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+  kern<<<grid, threads, smem, stream>>>(args...);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaErrorInvalidValue && smem > 48 * 1024) {
+    const DeviceInfo* dev = current_device();
+    if (!dev || raise_smem_limit(reinterpret_cast<const void*>(kern), smem, *dev) != cudaSuccess) return e;
+    kern<<<grid, threads, smem, stream>>>(args...);
+    e = cudaGetLastError();
+  }
+  return e;
+}
+
 // Launch-shape tunables (tridi_set_tunable); 0 means "choose automatically".
 int tunable(int key);
 

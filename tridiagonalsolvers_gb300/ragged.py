@@ -14,6 +14,7 @@ import ctypes
 import numpy as np
 
 from ._lib import check, lib
+from .solvers import _raw_stream
 
 
 def padded(total_rows: int) -> int:
@@ -53,10 +54,12 @@ class RaggedPlan:
             if t.dtype != torch.float32 or not t.is_cuda or not t.is_contiguous() or t.numel() < need:
                 raise ValueError(f"a, b, c, d must be contiguous float32 CUDA tensors of >= {need} elements")
         if x is None:
-            x = torch.zeros(need, dtype=torch.float32, device=a.device)
-        stream = ctypes.c_void_p(torch.cuda.current_stream(a.device).cuda_stream)
+            x = torch.empty(need, dtype=torch.float32, device=a.device)
+            if need > self.total_rows:
+                x[self.total_rows:].zero_()  # the padding; every row is written
         check(lib().tridi_ragged_solve_f32(a.data_ptr(), b.data_ptr(), c.data_ptr(), d.data_ptr(), x.data_ptr(),
-                                           self._h, self._dev.data_ptr(), stream), "tridi_ragged_solve_f32")
+                                           self._h, self._dev.data_ptr(), _raw_stream(torch, a)),
+              "tridi_ragged_solve_f32")
         return x
 
     def __del__(self):

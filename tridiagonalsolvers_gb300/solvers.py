@@ -10,47 +10,67 @@ Inputs are never modified.
 from __future__ import annotations
 
 import ctypes
+import functools
 
 from ._lib import check, lib
 
+_torch_module = None
+
 
 def _torch():
-    import torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
 
-    return torch
+        _torch_module = torch
+    return _torch_module
+
+
+def _raw_stream(torch, t) -> int:
+    """Handle of the current stream on t's device (without building a Stream
+    object, which costs more than the launch it is for)."""
+    get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return get(t.get_device()) if get is not None else torch.cuda.current_stream(t.device).cuda_stream
+
+
+@functools.lru_cache(maxsize=None)
+def _function(name, suf):
+    return getattr(lib(), f"tridi_{name}_{suf}")
 
 
 def _prep(a, b, c, d, x, system_size):
     torch = _torch()
-    ts = (a, b, c, d)
     dt = a.dtype
-    if dt not in (torch.float32, torch.float64):
+    if dt is torch.float32:
+        suf = "f32"
+    elif dt is torch.float64:
+        suf = "f64"
+    else:
         raise TypeError(f"unsupported dtype {dt}")
-    for t in ts:
+    count = a.numel()
+    for t in (a, b, c, d):
         if not t.is_cuda:
             raise ValueError("inputs must be CUDA tensors")
-        if t.dtype != dt or t.numel() != a.numel():
+        if t.dtype is not dt or t.numel() != count:
             raise ValueError("a, b, c, d must share dtype and size")
         if not t.is_contiguous():
             raise ValueError("inputs must be contiguous")
     n = int(system_size if system_size is not None else a.shape[-1])
-    if n <= 0 or a.numel() % n:
-        raise ValueError(f"numel {a.numel()} is not a multiple of system_size {n}")
-    m = a.numel() // n
+    if n <= 0 or count % n:
+        raise ValueError(f"numel {count} is not a multiple of system_size {n}")
     if x is None:
         x = torch.empty_like(a)
-    elif x.dtype != dt or x.numel() != a.numel() or not x.is_cuda or not x.is_contiguous():
+    elif x.dtype is not dt or x.numel() != count or not x.is_cuda or not x.is_contiguous():
         raise ValueError("x must be a contiguous CUDA tensor like a")
-    suf = "f32" if dt == torch.float32 else "f64"
-    stream = ctypes.c_void_p(torch.cuda.current_stream(a.device).cuda_stream)
-    return ts, x, n, m, suf, stream
+    return x, n, count // n, suf, _raw_stream(torch, a)
 
 
 def _call(name, a, b, c, d, x, system_size, *extra):
-    ts, x, n, m, suf, stream = _prep(a, b, c, d, x, system_size)
-    fn = getattr(lib(), f"tridi_{name}_{suf}")
-    ptrs = [t.data_ptr() for t in ts]
-    check(fn(*ptrs, x.data_ptr(), n, m, *extra, stream), f"tridi_{name}_{suf}(n={n}, m={m})")
+    x, n, m, suf, stream = _prep(a, b, c, d, x, system_size)
+    st = _function(name, suf)(a.data_ptr(), b.data_ptr(), c.data_ptr(), d.data_ptr(), x.data_ptr(), n, m, *extra,
+                              stream)
+    if st:
+        check(st, f"tridi_{name}_{suf}(n={n}, m={m})")
     return x
 
 
@@ -104,21 +124,30 @@ def solve_large(a, b, c, d, system_size, num_systems, layout="contiguous", x=Non
     torch = _torch()
     lay = {"contiguous": 0, "interleaved": 1}[layout]
     n, m = int(system_size), int(num_systems)
-    ts = (a, b, c, d)
-    for t in ts:
-        if not t.is_cuda or t.numel() != n * m or not t.is_contiguous() or t.dtype != a.dtype:
+    dt = a.dtype
+    for t in (a, b, c, d):
+        if not t.is_cuda or t.numel() != n * m or not t.is_contiguous() or t.dtype is not dt:
             raise ValueError("a, b, c, d must be contiguous CUDA tensors of n*m elements")
     if x is None:
         x = torch.empty_like(a)
-    suf = "f32" if a.dtype == torch.float32 else "f64"
-    L = lib()
-    ws_bytes = L.tridi_large_workspace_bytes(n, m, a.element_size())
+    suf = "f32" if dt is torch.float32 else "f64"
+    ws_bytes = _large_workspace_bytes(n, m, a.element_size())
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device)
-    stream = ctypes.c_void_p(torch.cuda.current_stream(a.device).cuda_stream)
-    fn = getattr(L, f"tridi_solve_large_{suf}")
-    check(fn(*(t.data_ptr() for t in ts), x.data_ptr(), n, m, lay, ws.data_ptr(), ws_bytes, stream),
-          f"tridi_solve_large_{suf}(n={n}, m={m}, {layout})")
+    st = _function("solve_large", suf)(a.data_ptr(), b.data_ptr(), c.data_ptr(), d.data_ptr(), x.data_ptr(), n, m, lay,
+                                       ws.data_ptr(), ws_bytes, _raw_stream(torch, a))
+    if st:
+        check(st, f"tridi_solve_large_{suf}(n={n}, m={m}, {layout})")
     return x
+
+
+@functools.lru_cache(maxsize=1024)
+def _large_workspace_bytes(n, m, elem_size):
+    return lib().tridi_large_workspace_bytes(n, m, elem_size)
+
+
+@functools.lru_cache(maxsize=1024)
+def _refine_workspace_bytes(n, m, lay):
+    return lib().tridi_refine_workspace_bytes(n, m, lay)
 
 
 def refine(a, b, c, d, system_size, num_systems, layout="contiguous", tol=1e-10, max_sweeps=10, x=None,
@@ -137,11 +166,11 @@ def refine(a, b, c, d, system_size, num_systems, layout="contiguous", tol=1e-10,
     if x is None:
         x = torch.empty(n * m, dtype=torch.float64, device=a.device)
     L = lib()
-    wsb = L.tridi_refine_workspace_bytes(n, m, lay)
+    wsb = _refine_workspace_bytes(n, m, lay)
     ws = torch.empty(wsb, dtype=torch.uint8, device=a.device)
     sweeps = ctypes.c_int(0)
     rel = ctypes.c_double(0.0)
-    stream = ctypes.c_void_p(torch.cuda.current_stream(a.device).cuda_stream)
+    stream = _raw_stream(torch, a)
     mode = {"df": 1, "fp64": 2}[residual]  # TRIDI_RESIDUAL_DF / TRIDI_RESIDUAL_FP64
     prev = L.tridi_get_tunable(4)  # TRIDI_TUNE_RESIDUAL
     check(L.tridi_set_tunable(4, mode), "tridi_set_tunable")
