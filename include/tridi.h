@@ -116,7 +116,9 @@ tridi_status tridi_pcr_f64(const double *a, const double *b, const double *c, co
                            int n, int num_systems, tridi_stream_t stream);
 
 /* Hybrid CR -> PCR -> CR with switch level `rest_system_size` (the size of the
-   intermediate system solved by PCR: a power of two, 2 <= rest <= n/2).
+   intermediate system solved by PCR: a power of two, 2 <= rest <= n/2; FP32
+   at n = 2048 and 4096 switches at n/32 rows for a larger rest, with the same
+   solution up to rounding).
    Replaces crpcr() of crpcr_app.cu:5 / crpcrKernel (crpcr_kernel.cu:1). */
 tridi_status tridi_crpcr_f32(const float *a, const float *b, const float *c, const float *d, float *x, int n,
                              int num_systems, int rest_system_size, tridi_stream_t stream);

@@ -158,6 +158,7 @@ tridi_status solve_hybrid(const float* a, const float* b, const float* c, const 
   cudaStream_t s = as_stream(stream);
   cudaError_t e = cudaErrorInvalidValue;
   if (stride == 1 && pcr_wide_applies(a, b, c, d, n, m, n)) return pcr_wide_solve(a, b, c, d, x, n, m, n, s);
+  if (crpcr_wide_applies(a, b, c, d, x, n, m, stride)) return crpcr_wide_solve(a, b, c, d, x, n, m, stride, s);
   if (crpcr_regs_applies(a, b, c, d, x, n, m, stride)) return crpcr_regs_solve(a, b, c, d, x, n, m, stride, s);
   if (pcr_twophase_applies(p)) {
     const bool paired = tunable(TRIDI_TUNE_PCR_KERNEL) != 3;

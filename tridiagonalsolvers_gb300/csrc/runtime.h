@@ -89,6 +89,11 @@ bool crpcr_regs_applies(const void* a, const void* b, const void* c, const void*
 tridi_status crpcr_regs_solve(const float* a, const float* b, const float* c, const float* d, float* x, int n,
                               int m, int stride, cudaStream_t stream);
 
+// cr and crpcr for 2048 and 4096 unknowns in registers (crpcr_wide.cu).
+bool crpcr_wide_applies(const void* a, const void* b, const void* c, const void* d, const void* x, int n, long m,
+                        int stride);
+tridi_status crpcr_wide_solve(const float* a, const float* b, const float* c, const float* d, float* x, int n, int m,
+                              int stride, cudaStream_t stream);
 // cr, pcr and crpcr at every switch level in FP64 (cr64.cu); stride = n / rest.
 tridi_status cr64_solve(const double* a, const double* b, const double* c, const double* d, double* x, int n, int m,
                         int stride, cudaStream_t stream);
