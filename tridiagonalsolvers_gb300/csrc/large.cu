@@ -26,6 +26,7 @@
 // once (4 B), plus ~20/L B of interface data.  No reference kernel
 // corresponds; the reference's large-system path is pcrGauss's global-memory
 // PCR steps (pcrGauss_kernel.cu:272-386).  Oracle: the gold Thomas solver.
+#include "large_tma.h"
 #include "partition.cuh"
 #include "runtime.h"
 
@@ -39,10 +40,6 @@ tridi_status large_rows_solve(const T* a, const T* b, const T* c, const T* d, T*
                               cudaStream_t st);
 template <class T>
 size_t large_rows_bytes(long n, long m);
-bool large_tma_ok(const float* a, const float* b, const float* c, const float* d, long n, long m);
-tridi_status large_tma_pass(bool back, const float* a, const float* b, const float* c, const float* d, long n,
-                            long m, long P, long PMp, float* red, float* bnd, const float* sol, float* x,
-                            cudaStream_t st);
 
 struct LargeParams {
   const void* a;
@@ -132,41 +129,56 @@ __global__ void __launch_bounds__(128) large_back_kernel(LargeParams p) {
     if (i < k) gx[i * rs] = x[i];
 }
 
-// Base case for interleaved systems: one thread per system runs the gold
-// Thomas recurrence (tridiagonal_gold.h:26-44, a[0] and c[n-1] ignored),
-// keeping c' and d' in a scratch array; a warp reads 32 consecutive systems,
-// so every row access is coalesced.
+// Base case for interleaved systems of at most kThomasMax rows: one thread per
+// system runs the gold Thomas recurrence (tridiagonal_gold.h:26-44, a[0] and
+// c[n-1] ignored) in registers; a warp reads 32 consecutive systems, so every
+// row access is coalesced.  The loads of eight rows are issued together: with
+// one row at a time the 16-row systems of a 65536-row solve took 12 us of
+// memory latency.
+constexpr long kThomasMax = 32;
 template <class T>
-__global__ void __launch_bounds__(256) thomas_interleaved_kernel(const T* __restrict__ a, const T* __restrict__ b,
-                                                                 const T* __restrict__ c, const T* __restrict__ d,
-                                                                 T* __restrict__ x, long n, long m,
-                                                                 T* __restrict__ cp, T* __restrict__ dp) {
+__global__ void __launch_bounds__(32) thomas_interleaved_kernel(const T* __restrict__ a, const T* __restrict__ b,
+                                                                const T* __restrict__ c, const T* __restrict__ d,
+                                                                T* __restrict__ x, int n, long m) {
+  constexpr int N = (int)kThomasMax, B = 8;
   const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= m) return;
-  T cprev = T(0), dprev = T(0);
-  for (long i = 0; i < n; ++i) {
-    const long k = i * m + s;
-    const T ai = i == 0 ? T(0) : a[k];
-    const T ci = i == n - 1 ? T(0) : c[k];
-    tdiv2(ci, d[k] - ai * dprev, b[k] - ai * cprev, cprev, dprev);
-    cp[k] = cprev;
-    dp[k] = dprev;
+  T cp[N], dp[N], cprev = T(0), dprev = T(0);
+#pragma unroll
+  for (int i0 = 0; i0 < N; i0 += B) {
+    if (i0 < n) {
+      T ra[B], rb[B], rc[B], rd[B];
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const int i = i0 + q;
+        const bool in = i < n;
+        const long k = (long)i * m + s;
+        ra[q] = in && i > 0 ? a[k] : T(0);
+        rb[q] = in ? b[k] : T(1);
+        rc[q] = in && i < n - 1 ? c[k] : T(0);
+        rd[q] = in ? d[k] : T(0);
+      }
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        tdiv2(rc[q], rd[q] - ra[q] * dprev, rb[q] - ra[q] * cprev, cprev, dprev);
+        cp[i0 + q] = cprev;
+        dp[i0 + q] = dprev;
+      }
+    }
   }
-  T xn = dprev;
-  x[(n - 1) * m + s] = xn;
-  for (long i = n - 2; i >= 0; --i) {
-    const long k = i * m + s;
-    xn = dp[k] - cp[k] * xn;
-    x[k] = xn;
+  // (rows past n are identity rows: x = 0, and row n - 1 has c = 0)
+  T xn = T(0);
+#pragma unroll
+  for (int i = N - 1; i >= 0; --i) {
+    if (i < n) {
+      xn = dp[i] - cp[i] * xn;
+      x[(long)i * m + s] = xn;
+    }
   }
 }
 
 namespace {
 constexpr int kChunk = 16;
-// Interleaved base case: one thread per system, a serial chain over n rows
-// with only m threads in flight, so it is kept short (the recursion goes one
-// level further rather than run 256-row chains on 1024 threads).
-constexpr long kThomasMax = 32;
 
 long round64(long v) { return (v + 63) & ~63L; }
 
@@ -189,9 +201,14 @@ size_t large_workspace_bytes(long n, long m, int layout) {
 template size_t large_workspace_bytes<float>(long, long, int);
 template size_t large_workspace_bytes<double>(long, long, int);
 
+bool large_fusable(const float* a, const float* b, const float* c, const float* d, long n, long m) {
+  return n > kThomasMax && tunable(TRIDI_TUNE_LARGE_TMA) != 2 && !g_host_mapped_io && large_tma_ok(a, b, c, d, n, m);
+}
+
+namespace {
 template <class T>
-tridi_status large_solve_device(const T* a, const T* b, const T* c, const T* d, T* x, long n, long m, int layout,
-                                void* ws, size_t ws_bytes, tridi_stream_t stream) {
+tridi_status large_solve(const T* a, const T* b, const T* c, const T* d, T* x, long n, long m, int layout, void* ws,
+                         size_t ws_bytes, const LargeFused* fused, tridi_stream_t stream) {
   if (!a || !b || !c || !d || !x || m <= 0 || n <= 0 || (layout != 0 && layout != 1))
     return TRIDI_ERROR_INVALID_VALUE;
   if (n * m > (1L << 34)) return TRIDI_ERROR_UNSUPPORTED_SIZE;
@@ -205,9 +222,7 @@ tridi_status large_solve_device(const T* a, const T* b, const T* c, const T* d, 
     return large_rows_solve<T>(a, b, c, d, x, n, m, ws, st);
   }
   if (n <= kThomasMax) {
-    T* cp = reinterpret_cast<T*>(w);
-    T* dp = cp + round64(n * m);
-    thomas_interleaved_kernel<T><<<(unsigned)((m + 255) / 256), 256, 0, st>>>(a, b, c, d, x, n, m, cp, dp);
+    thomas_interleaved_kernel<T><<<(unsigned)((m + 31) / 32), 32, 0, st>>>(a, b, c, d, x, (int)n, m);
     return cuda_status(cudaGetLastError());
   }
   LargeParams p{};
@@ -224,15 +239,13 @@ tridi_status large_solve_device(const T* a, const T* b, const T* c, const T* d, 
   const unsigned blocks = (unsigned)((PM + 255) / 256);
   // interleaved FP32 with m a multiple of 32: the TMA-tiled passes (large_tma.cu)
   bool tma = false;
-  if constexpr (sizeof(T) == 4)
-    tma = tunable(TRIDI_TUNE_LARGE_TMA) != 2 && !g_host_mapped_io && large_tma_ok(a, b, c, d, n, m);
+  if constexpr (sizeof(T) == 4) tma = large_fusable(a, b, c, d, n, m);
   if (tma) {
     // the separator rows assembled in the pass (the interface area holds the
     // tile-boundary arrays only)
-    const tridi_status t = large_tma_pass(false, reinterpret_cast<const float*>(a), reinterpret_cast<const float*>(b),
-                                          reinterpret_cast<const float*>(c), reinterpret_cast<const float*>(d), n, m,
-                                          p.P, p.PMp, static_cast<float*>(p.red), static_cast<float*>(p.iface),
-                                          nullptr, nullptr, st);
+    const tridi_status t = large_tma_reduce(
+        reinterpret_cast<const float*>(a), reinterpret_cast<const float*>(b), reinterpret_cast<const float*>(c),
+        reinterpret_cast<const float*>(d), n, m, p.P, p.PMp, static_cast<float*>(p.red), static_cast<float*>(p.iface), st);
     if (t != TRIDI_SUCCESS) return t;
   } else {
     large_reduce_kernel<T, kChunk><<<(unsigned)((PM + 127) / 128), 128, 0, st>>>(p);
@@ -241,15 +254,27 @@ tridi_status large_solve_device(const T* a, const T* b, const T* c, const T* d, 
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_status(e);
   const T* r = static_cast<const T*>(p.red);
-  const tridi_status ts = large_solve_device<T>(r, r + p.PMp, r + 2 * p.PMp, r + 3 * p.PMp, static_cast<T*>(p.sol),
-                                                p.P, m, layout, inner, inner_bytes, stream);
+  const tridi_status ts = large_solve<T>(r, r + p.PMp, r + 2 * p.PMp, r + 3 * p.PMp, static_cast<T*>(p.sol), p.P, m,
+                                         layout, inner, inner_bytes, nullptr, stream);
   if (ts != TRIDI_SUCCESS) return ts;
   if (tma)
-    return large_tma_pass(true, reinterpret_cast<const float*>(a), reinterpret_cast<const float*>(b),
-                          reinterpret_cast<const float*>(c), reinterpret_cast<const float*>(d), n, m, p.P, p.PMp,
-                          nullptr, nullptr, static_cast<const float*>(p.sol), reinterpret_cast<float*>(x), st);
+    return large_tma_back(reinterpret_cast<const float*>(a), reinterpret_cast<const float*>(b),
+                          reinterpret_cast<const float*>(c), reinterpret_cast<const float*>(d), n, m,
+                          static_cast<const float*>(p.sol), reinterpret_cast<float*>(x), fused, st);
   large_back_kernel<T, kChunk><<<(unsigned)((PM + 127) / 128), 128, 0, st>>>(p);
   return cuda_status(cudaGetLastError());
+}
+
+}  // namespace
+
+template <class T>
+tridi_status large_solve_device(const T* a, const T* b, const T* c, const T* d, T* x, long n, long m, int layout,
+                                void* ws, size_t ws_bytes, tridi_stream_t stream) {
+  return large_solve<T>(a, b, c, d, x, n, m, layout, ws, ws_bytes, nullptr, stream);
+}
+tridi_status large_solve_fused(const float* a, const float* b, const float* c, const float* rhs, float* x, long n,
+                               long m, void* ws, size_t ws_bytes, const LargeFused& f, tridi_stream_t stream) {
+  return large_solve<float>(a, b, c, rhs, x, n, m, TRIDI_LAYOUT_INTERLEAVED, ws, ws_bytes, &f, stream);
 }
 
 template tridi_status large_solve_device<float>(const float*, const float*, const float*, const float*, float*, long,

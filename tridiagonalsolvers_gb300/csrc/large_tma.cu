@@ -25,6 +25,8 @@
 #include <cstring>
 #include <mutex>
 
+#include "dfloat.cuh"
+#include "large_tma.h"
 #include "partition.cuh"
 #include "runtime.h"
 
@@ -45,7 +47,12 @@ struct LtParams {
   float* bnd;       // reduce: tile-boundary interface, 10 arrays of row_tiles*m (stride BS)
   long BS;
   const float* sol; // back: separators
-  float* x;         // back: solution
+  void* x;          // back: solution (FP32, or FP64 in kBackSecond)
+  const float* d;   // kBackSecond: the refined system's right-hand side ...
+  const float* e0;  // ... and its first solution
+  float* r;         // kBackFirst: the residual
+  double* rr;       // kBackFirst, kBackSecond: per-system sums of r^2 ...
+  double* dd;       // ... and, kBackFirst, of d^2
   int row_tiles, col_tiles;
   unsigned* status;
 };
@@ -110,9 +117,8 @@ __device__ __forceinline__ void column_summary(ChunkSummary<float>& cs, int k, c
   }
 }
 
-template <bool BACK>
 __global__ void __launch_bounds__(32 * (kLtWarps + 1), 1)
-    large_tile_kernel(LtParams p, const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb,
+    large_reduce_tile_kernel(LtParams p, const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb,
                       const __grid_constant__ CUtensorMap mc, const __grid_constant__ CUtensorMap md) {
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
@@ -167,70 +173,295 @@ __global__ void __launch_bounds__(32 * (kLtWarps + 1), 1)
     const int kr = rem <= 0 ? 0 : (rem < kLtChunk ? (int)rem : kLtChunk);
     ChunkSummary<float> cs;
     // The eliminated column stays in registers and the stage goes back to
-    // the producer right after the elimination, so a stage is held for the
-    // elimination only (not for the separator wait and back substitution,
-    // nor for the interface exchange).
+    // the producer right after the elimination (not after the interface
+    // exchange).
     float cp[kLtChunk], ap[kLtChunk], dp[kLtChunk];
     float cl = 0.f, al = 0.f, dl = 0.f;
-    float sj = 0.f, sl = 0.f;
     if (kr > 0) {
-      if constexpr (BACK) {  // the separators' loads overlap the elimination
-        const long o = j * p.m + sys;
-        sj = p.sol[o];
-        sl = j > 0 ? p.sol[o - p.m] : 0.f;
-      }
       column_forward(kr, j == 0, sa, sb, sc, sd, cp, ap, dp, cl, al, dl);
-      if constexpr (!BACK) {
-        const int o = (kr - 1) * kTileCols;
-        cs.sep = Row<float>{sa[o], sb[o], sc[o], sd[o]};
-        if (kr == 1 && j == 0) cs.sep.a = 0.f;
-        if (j == p.P - 1) cs.sep.c = 0.f;
-      }
+      const int o = (kr - 1) * kTileCols;
+      cs.sep = Row<float>{sa[o], sb[o], sc[o], sd[o]};
+      if (kr == 1 && j == 0) cs.sep.a = 0.f;
+      if (j == p.P - 1) cs.sep.c = 0.f;
     }
     release_stage(&empty[s]);
-    if constexpr (BACK) {
-      if (kr > 0) {
-        float* gx = p.x + r0 * p.m + sys;
-        gx[(long)(kr - 1) * p.m] = sj;
-        float xn = sj;
-#pragma unroll
-        for (int i = kLtChunk - 2; i >= 0; --i) {
-          if (i <= kr - 2) {
-            xn = dp[i] - cp[i] * xn - ap[i] * sl;
-            gx[(long)i * p.m] = xn;
-          }
-        }
-      }
-      continue;
-    }
     if (kr > 0) column_summary(cs, kr, cp, ap, dp, cl, al, dl);
-    if constexpr (!BACK) {
-      // separator rows: warp w < 7 takes the next chunk's first row from warp
-      // w + 1 of the same tile; a tile's last chunk and its first chunk go to
-      // the boundary arrays, assembled by large_tile_boundary_kernel
-      float* ex = exch + (k & 1) * (kLtWarps * 32 * 3);
-      float* mine = ex + (warp * 32 + lane) * 3;
-      mine[0] = kr > 0 ? cs.fD : 0.f;
-      mine[1] = kr > 0 ? cs.fC : 0.f;
-      mine[2] = kr > 0 ? cs.fA : 0.f;
-      consumer_sync(32 * kLtWarps);
-      if (kr > 0) {
-        const long tr = t / p.col_tiles;
-        if (warp + 1 < kLtWarps) {
-          const float* nx = ex + ((warp + 1) * 32 + lane) * 3;
-          put_separator(p.red, p.PMp, j * p.m + sys, cs.sep, cs.lD, cs.lC, cs.lA, nx[0], nx[1], nx[2]);
-        } else {
-          float* b = p.bnd + tr * p.m + sys;
-          b[(kBndLast + 0) * p.BS] = cs.lD; b[(kBndLast + 1) * p.BS] = cs.lC; b[(kBndLast + 2) * p.BS] = cs.lA;
-          b[(kBndLast + 3) * p.BS] = cs.sep.a; b[(kBndLast + 4) * p.BS] = cs.sep.b;
-          b[(kBndLast + 5) * p.BS] = cs.sep.c; b[(kBndLast + 6) * p.BS] = cs.sep.d;
-        }
-        if (warp == 0) {
-          float* b = p.bnd + tr * p.m + sys;
-          b[(kBndFirst + 0) * p.BS] = cs.fD; b[(kBndFirst + 1) * p.BS] = cs.fC; b[(kBndFirst + 2) * p.BS] = cs.fA;
-        }
+    // separator rows: warp w < 7 takes the next chunk's first row from warp
+    // w + 1 of the same tile; a tile's last chunk and its first chunk go to
+    // the boundary arrays, assembled by large_tile_boundary_kernel
+    float* ex = exch + (k & 1) * (kLtWarps * 32 * 3);
+    float* mine = ex + (warp * 32 + lane) * 3;
+    mine[0] = kr > 0 ? cs.fD : 0.f;
+    mine[1] = kr > 0 ? cs.fC : 0.f;
+    mine[2] = kr > 0 ? cs.fA : 0.f;
+    consumer_sync(32 * kLtWarps);
+    if (kr > 0) {
+      const long tr = t / p.col_tiles;
+      if (warp + 1 < kLtWarps) {
+        const float* nx = ex + ((warp + 1) * 32 + lane) * 3;
+        put_separator(p.red, p.PMp, j * p.m + sys, cs.sep, cs.lD, cs.lC, cs.lA, nx[0], nx[1], nx[2]);
+      } else {
+        float* b = p.bnd + tr * p.m + sys;
+        b[(kBndLast + 0) * p.BS] = cs.lD; b[(kBndLast + 1) * p.BS] = cs.lC; b[(kBndLast + 2) * p.BS] = cs.lA;
+        b[(kBndLast + 3) * p.BS] = cs.sep.a; b[(kBndLast + 4) * p.BS] = cs.sep.b;
+        b[(kBndLast + 5) * p.BS] = cs.sep.c; b[(kBndLast + 6) * p.BS] = cs.sep.d;
+      }
+      if (warp == 0) {
+        float* b = p.bnd + tr * p.m + sys;
+        b[(kBndFirst + 0) * p.BS] = cs.fD; b[(kBndFirst + 1) * p.BS] = cs.fC; b[(kBndFirst + 2) * p.BS] = cs.fA;
       }
     }
+  }
+}
+
+// The back pass: each lane's column again, between the separators above and
+// below it, by a Thomas sweep.  MODE kBackPlain: x.  kBackFirst: x (FP32,
+// exact) and the residual r = d - T x in double-float, rounded to FP32, with
+// the sums of r^2 and d^2 per system: the first sweep of the refinement without
+// reading the system again.  kBackSecond: the solve was of a correction e1
+// (right-hand side r); x = e0 + e1 in FP64 and the sum of its residuals'
+// squares, d and e0 read beside the tiles.  A tile's last row needs x of the
+// next tile's first: large_tile_edge_kernel adds its share once the pass is
+// done.
+//
+// Three groups of four warps an SM, each with tiles of its own (64 rows x 32
+// systems), a private two-stage ring and its own barrier: a tile goes to
+// registers, its stage is refilled at once, and the groups cover one another's
+// dependent chains.  1024 x 65536: plain 188 us, kBackFirst 283 us, kBackSecond
+// 516 us; eight warps in step on 128-row tiles 208, 396 and 668 us; with two
+// rows' residuals in paired FP32 instructions 190, 319 and 530 us (the pairs'
+// registers).  kBackFirst and kBackSecond stand for a back pass and a pass over
+// the system of 330 and 560 us.
+constexpr int kBackGroups = 3, kBackWarps = 4;           // groups a CTA, warps a group
+constexpr int kBackRows = kBackWarps * kLtChunk;         // 64
+constexpr int kBackFloats = kBackRows * kTileCols;       // per array of a tile
+constexpr int kBackThreads = 32 * kBackGroups * kBackWarps;
+constexpr size_t kBackSmem = 128 + (size_t)kBackGroups * 2 * 4 * kBackFloats * sizeof(float);
+// per group: x of the warps' first rows (hi, lo) and the norms' partial sums (r^2, d^2), both for two tiles
+constexpr size_t kBackShare = 2 * 2 * kBackWarps * 32;
+constexpr size_t kBackResidual = kBackGroups * kBackShare * sizeof(float2);
+
+template <int MODE>
+__global__ void __launch_bounds__(kBackThreads, 1)
+    large_back_tile_kernel(LtParams p, const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb,
+                           const __grid_constant__ CUtensorMap mc, const __grid_constant__ CUtensorMap md) {
+  constexpr int L = kLtChunk;
+  constexpr int GT = 32 * kBackWarps;  // threads a group
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int lane = threadIdx.x & 31, grp = threadIdx.x / GT, warp = (threadIdx.x % GT) >> 5;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem) + 2 * grp;
+  float* ring = reinterpret_cast<float*>(smem + 128) + (size_t)grp * 2 * 4 * kBackFloats;
+  float2* exch = reinterpret_cast<float2*>(smem + kBackSmem) + grp * kBackShare;
+  float2* norms = exch + 2 * kBackWarps * 32;
+  const int row_tiles = (int)((p.n + kBackRows - 1) / kBackRows);
+  const int ntiles = row_tiles * p.col_tiles, step = (int)gridDim.x * kBackGroups;
+  const int first = (int)blockIdx.x * kBackGroups + grp;
+  const bool leader = threadIdx.x % GT == 0;
+  const auto issue = [&](int t, int s) {  // the group's leader
+    const int x0 = (t % p.col_tiles) * kTileCols, y0 = (t / p.col_tiles) * kBackRows;
+    float* st = ring + (size_t)s * 4 * kBackFloats;
+    mbar_arrive_expect_tx(&full[s], 4u * kBackFloats * sizeof(float));
+    tma_load_2d(st + 0 * kBackFloats, &ma, x0, y0, &full[s]);
+    tma_load_2d(st + 1 * kBackFloats, &mb, x0, y0, &full[s]);
+    tma_load_2d(st + 2 * kBackFloats, &mc, x0, y0, &full[s]);
+    tma_load_2d(st + 3 * kBackFloats, &md, x0, y0, &full[s]);
+  };
+  if (leader) {
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    mbar_fence_init();
+    if (first < ntiles) issue(first, 0);
+    if (first + step < ntiles) issue(first + step, 1);
+  }
+  __syncthreads();
+
+  // The lane's column of tile t: system, first row; its separators are loaded
+  // one tile ahead.
+  const auto column = [&](int t, long& sys, long& r0) {
+    sys = (long)(t % p.col_tiles) * kTileCols + lane;
+    r0 = (long)(t / p.col_tiles) * kBackRows + (long)warp * L;
+  };
+  const auto separators = [&](int t, float& above, float& below) {
+    above = below = 0.f;
+    if (t >= ntiles) return;
+    long sys, r0;
+    column(t, sys, r0);
+    if (r0 >= p.n) return;
+    const long o = (r0 / L) * p.m + sys;
+    below = __ldg(p.sol + o);
+    if (r0 > 0) above = __ldg(p.sol + o - p.m);
+  };
+  // sums of tile t's norms (the group's k-th) over its warps, by one of them
+  const auto flush = [&](int t, int k) {
+    if (warp != (k & (kBackWarps - 1))) return;
+    double rs = 0.0, ds = 0.0;
+    for (int w = 0; w < kBackWarps; ++w) {
+      const float2 v = norms[((k & 1) * kBackWarps + w) * 32 + lane];
+      rs += v.x;
+      ds += v.y;
+    }
+    const long sys = (long)(t % p.col_tiles) * kTileCols + lane;
+    atomicAdd(&p.rr[sys], rs);
+    if (MODE == kBackFirst) atomicAdd(&p.dd[sys], ds);
+  };
+  float sl_next, sj_next;
+  separators(first, sl_next, sj_next);
+  int k = 0;
+  for (int t = first; t < ntiles; t += step, ++k) {
+    const int s = k & 1;
+    long sys, r0;
+    column(t, sys, r0);
+    const float sl = sl_next, sj = sj_next;
+    separators(t + step, sl_next, sj_next);
+    const long rem = p.n - r0;
+    const int kr = rem <= 0 ? 0 : (rem < L ? (int)rem : L);
+    const long g0 = r0 * p.m + sys;
+    float dv[MODE == kBackSecond ? L : 1], e0[MODE == kBackSecond ? L : 1], e0m = 0.f;
+    if constexpr (MODE == kBackSecond) {
+#pragma unroll
+      for (int q = 0; q < L; ++q) {
+        dv[q] = q < kr ? __ldg(p.d + g0 + (long)q * p.m) : 0.f;
+        e0[q] = q < kr ? __ldg(p.e0 + g0 + (long)q * p.m) : 0.f;
+      }
+      if (kr > 0 && r0 > 0) e0m = __ldg(p.e0 + g0 - p.m);
+    }
+    const bool ok = mbar_wait(&full[s], (k >> 1) & 1, p.status);
+    const float* st = ring + (size_t)s * 4 * kBackFloats + warp * L * kTileCols + lane;
+    float a[L], b[L], c[L], d[L];
+#pragma unroll
+    for (int q = 0; q < L; ++q) {
+      a[q] = st[q * kTileCols];
+      b[q] = st[kBackFloats + q * kTileCols];
+      c[q] = st[2 * kBackFloats + q * kTileCols];
+      d[q] = st[3 * kBackFloats + q * kTileCols];
+    }
+    fence_proxy_async_smem();
+    if (!named_sync_and(1 + grp, GT, ok)) return;  // every column is read
+    if (leader && t + 2 * step < ntiles) issue(t + 2 * step, s);
+    if (MODE != kBackPlain && k > 0) flush(t - step, k - 1);
+    if (r0 == 0) a[0] = 0.f;
+    float cp[L], x[L], cprev = 0.f, dprev = sl;
+#pragma unroll
+    for (int q = 0; q < L; ++q) {
+      if (q < kr - 1) {
+        tdiv2(c[q], d[q] - a[q] * dprev, q == 0 ? b[q] : b[q] - a[q] * cprev, cp[q], x[q]);
+        cprev = cp[q];
+        dprev = x[q];
+      }
+    }
+    float xn = sj;
+    if constexpr (MODE == kBackPlain) {
+      float* gx = static_cast<float*>(p.x) + g0;
+#pragma unroll
+      for (int q = L - 1; q >= 0; --q) {
+        if (q <= kr - 1) {
+          if (q <= kr - 2) xn = x[q] - cp[q] * xn;
+          gx[(long)q * p.m] = xn;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int q = L - 1; q >= 0; --q) {
+        if (q <= kr - 2) xn = x[q] - cp[q] * xn;
+        x[q] = q <= kr - 1 ? xn : 0.f;
+      }
+      // x as pairs: the row above, the lane's rows, the row below
+      float lo[MODE == kBackSecond ? L : 1] = {};
+      float2 xm = make_float2(sl, 0.f);
+      if constexpr (MODE == kBackSecond) {
+        xm.x = two_sum(e0m, sl, xm.y);
+#pragma unroll
+        for (int q = 0; q < L; ++q) x[q] = two_sum(e0[q], x[q], lo[q]);
+      }
+      const auto pair = [&](int q) { return make_float2(x[q], MODE == kBackSecond ? lo[MODE == kBackSecond ? q : 0] : 0.f); };
+      float2* ex = exch + (k & 1) * kBackWarps * 32;
+      ex[warp * 32 + lane] = pair(0);
+      named_sync_and(1 + grp, GT, true);
+      // x below the lane's last row: zero past the system's end (that row's c
+      // counts as zero); past the tile it is not known here
+      const bool open = warp == kBackWarps - 1 && r0 + L < p.n;
+      const bool end = kr > 0 && r0 + kr == p.n;
+      const float2 below = warp + 1 < kBackWarps && !end ? ex[(warp + 1) * 32 + lane] : make_float2(0.f, 0.f);
+      float rs = 0.f, ds = 0.f;
+#pragma unroll
+      for (int q = 0; q < L; ++q) {
+        if (q < kr) {
+          const float2 xi = pair(q);
+          const bool lastrow = q == kr - 1;
+          const long o = g0 + (long)q * p.m;
+          if (MODE == kBackFirst) static_cast<float*>(p.x)[o] = xi.x;
+          else static_cast<double*>(p.x)[o] = df_to_double(xi.x, xi.y);
+          const float2 xp = lastrow ? below : pair(q + 1 < L ? q + 1 : q);
+          const float di = MODE == kBackSecond ? dv[MODE == kBackSecond ? q : 0] : d[q];
+          const float ci = lastrow && end ? 0.f : c[q];
+          const float r = MODE == kBackSecond ? df_residual(a[q], b[q], ci, di, xm, xi, xp)
+                                              : f_residual(a[q], b[q], ci, di, xm.x, xi.x, xp.x);
+          if (!(lastrow && open)) {
+            if (MODE == kBackFirst) p.r[o] = r;
+            rs = fmaf(r, r, rs);
+            ds = fmaf(di, di, ds);
+          }
+          xm = xi;
+        }
+      }
+      norms[((k & 1) * kBackWarps + warp) * 32 + lane] = make_float2(rs, ds);
+    }
+  }
+  if (MODE != kBackPlain && k > 0) {
+    named_sync_and(1 + grp, GT, true);
+    flush(first + (k - 1) * step, k - 1);
+  }
+}
+
+// v as hi + lo, hi its significand's upper 24 bits and lo the next 24, on the
+// integer units (three FP64 instructions a value bound the kernel below);
+// values outside FP32's normal range take those.
+__device__ __forceinline__ float2 double_to_pair(double v) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+  const int e = (int)((u >> 52) & 0x7ff) - 1023;  // v = +-1.f * 2^e
+  if (e < -60 || e > 120) {
+    const float hi = __double2float_rn(v);
+    return make_float2(hi, __double2float_rn(v - (double)hi));
+  }
+  const unsigned sign = (unsigned)(u >> 32) & 0x80000000u;
+  const float hi = __uint_as_float(sign | ((unsigned)(e + 127) << 23) | ((unsigned)(u >> 29) & 0x7fffffu));
+  const float ulp = __uint_as_float(sign | ((unsigned)(e + 127 - 52) << 23));  // 2^(e - 52)
+  return make_float2(hi, (float)((unsigned)u & 0x1fffffffu) * ulp);
+}
+
+// The rows that large_back_tile_kernel leaves open (the last of each tile but
+// the system's last row): their residuals and shares of the norms.  A warp
+// takes 32 systems of one tile row, a block eight tile rows.
+template <int MODE>
+__global__ void __launch_bounds__(256) large_tile_edge_kernel(LtParams p, const float* __restrict__ a,
+                                                              const float* __restrict__ b, const float* __restrict__ c,
+                                                              const float* __restrict__ d) {
+  __shared__ float2 part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long sys = (long)(blockIdx.x % p.col_tiles) * kTileCols + lane;
+  const long i = ((long)(blockIdx.x / p.col_tiles) * 8 + warp + 1) * kBackRows - 1;
+  const auto x_at = [&](long o) {
+    if constexpr (MODE == kBackFirst) return make_float2(static_cast<const float*>(p.x)[o], 0.f);
+    return double_to_pair(static_cast<const double*>(p.x)[o]);
+  };
+  float2 sums = make_float2(0.f, 0.f);
+  if (i < p.n - 1) {
+    const long o = i * p.m + sys;
+    const float di = d[o];
+    const float r = df_residual(a[o], b[o], c[o], di, x_at(o - p.m), x_at(o), x_at(o + p.m));
+    if (MODE == kBackFirst) p.r[o] = r;
+    sums = make_float2(r * r, di * di);
+  }
+  part[warp][lane] = sums;
+  __syncthreads();
+  if (warp == 0) {
+    float rs = 0.f, ds = 0.f;
+    for (int w = 0; w < 8; ++w) {
+      rs += part[w][lane].x;
+      ds += part[w][lane].y;
+    }
+    atomicAdd(&p.rr[sys], (double)rs);
+    if (MODE == kBackFirst) atomicAdd(&p.dd[sys], (double)ds);
   }
 }
 
@@ -254,9 +485,8 @@ __global__ void __launch_bounds__(256) large_tile_boundary_kernel(LtParams p) {
                 b[(kBndLast + 2) * p.BS], nD, nC, nA);
 }
 
-bool make_map(CUtensorMap* map, const float* base, long n, long m) {
-  return make_tensor_map_2d(map, base, (uint64_t)m, (uint64_t)n, (uint64_t)m * sizeof(float), kTileCols, kTileRows,
-                            false);
+bool make_map(CUtensorMap* map, const float* base, long n, long m, int rows) {
+  return make_tensor_map_2d(map, base, (uint64_t)m, (uint64_t)n, (uint64_t)m * sizeof(float), kTileCols, rows, false);
 }
 
 }  // namespace
@@ -272,39 +502,84 @@ bool large_tma_ok(const float* a, const float* b, const float* c, const float* d
 // interface floats the register kernels use).
 long large_tma_boundary_stride(long n, long m) { return ((((n + kTileRows - 1) / kTileRows) * m) + 63) & ~63L; }
 
-// One TMA pass: back = false -> the separator system (reduce, with the
-// assembly of separator rows fused in; bnd: scratch of 10 boundary arrays),
-// true -> x (back).
-tridi_status large_tma_pass(bool back, const float* a, const float* b, const float* c, const float* d, long n,
-                            long m, long P, long PMp, float* red, float* bnd, const float* sol, float* x,
-                            cudaStream_t st) {
-  const DeviceInfo* dev = current_device();
-  if (!dev) return TRIDI_ERROR_CUDA;
-  const size_t smem = back ? kLtSmem : kLtSmem + kLtExchange;
-  if ((size_t)dev->max_smem_optin < smem) return TRIDI_ERROR_UNSUPPORTED_SIZE;
-  CUtensorMap ma, mb, mc, md;
-  if (!make_map(&ma, a, n, m) || !make_map(&mb, b, n, m) || !make_map(&mc, c, n, m) || !make_map(&md, d, n, m))
-    return TRIDI_ERROR_INVALID_VALUE;
+// One TMA pass.  large_tma_reduce: the separator system (with the assembly of
+// separator rows fused in; bnd: scratch of 10 boundary arrays).
+// large_tma_back: the unknowns, and what f asks for beside them.
+namespace {
+tridi_status make_maps(CUtensorMap (&tm)[4], const float* a, const float* b, const float* c, const float* d, long n,
+                       long m, int rows) {
+  const float* src[4] = {a, b, c, d};
+  for (int i = 0; i < 4; ++i)
+    if (!make_map(&tm[i], src[i], n, m, rows)) return TRIDI_ERROR_INVALID_VALUE;
+  return TRIDI_SUCCESS;
+}
+LtParams tile_params(long n, long m, const DeviceInfo* dev) {
   LtParams p{};
-  p.n = n; p.m = m; p.P = P; p.PMp = PMp; p.red = red; p.bnd = bnd; p.sol = sol; p.x = x;
+  p.n = n; p.m = m;
   p.BS = large_tma_boundary_stride(n, m);
   p.row_tiles = (int)((n + kTileRows - 1) / kTileRows);
   p.col_tiles = (int)(m / kTileCols);
   p.status = dev->status;
-  const long ntiles = (long)p.row_tiles * p.col_tiles;
-  int grid = dev->sm_count;
-  if (grid > ntiles) grid = (int)ntiles;
+  return p;
+}
+using TileKernel = void (*)(LtParams, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap);
+// `groups` tiles a CTA at a time, one CTA an SM.
+cudaError_t launch_tiles(TileKernel kern, int threads, size_t smem, long tiles, int groups, const LtParams& p,
+                         const CUtensorMap (&tm)[4], const DeviceInfo& dev, cudaStream_t st) {
   int per_sm = 0;
-  cudaError_t e = back ? resident_blocks(large_tile_kernel<true>, 32 * (kLtWarps + 1), smem, *dev, &per_sm)
-                       : resident_blocks(large_tile_kernel<false>, 32 * (kLtWarps + 1), smem, *dev, &per_sm);
+  const cudaError_t e = resident_blocks(kern, threads, smem, dev, &per_sm);
+  if (e != cudaSuccess) return e;
+  const long ctas = (tiles + groups - 1) / groups;
+  return launch_kernel(kern, (unsigned)(dev.sm_count < ctas ? dev.sm_count : ctas), threads, smem, st, p, tm[0], tm[1],
+                       tm[2], tm[3]);
+}
+}  // namespace
+
+tridi_status large_tma_reduce(const float* a, const float* b, const float* c, const float* d, long n, long m, long P,
+                              long PMp, float* red, float* bnd, cudaStream_t st) {
+  const DeviceInfo* dev = current_device();
+  if (!dev) return TRIDI_ERROR_CUDA;
+  constexpr size_t smem = kLtSmem + kLtExchange;
+  if ((size_t)dev->max_smem_optin < smem) return TRIDI_ERROR_UNSUPPORTED_SIZE;
+  CUtensorMap tm[4];
+  const tridi_status ts = make_maps(tm, a, b, c, d, n, m, kTileRows);
+  if (ts != TRIDI_SUCCESS) return ts;
+  LtParams p = tile_params(n, m, dev);
+  p.P = P; p.PMp = PMp; p.red = red; p.bnd = bnd;
+  const cudaError_t e = launch_tiles(large_reduce_tile_kernel, 32 * (kLtWarps + 1), smem,
+                                     (long)p.row_tiles * p.col_tiles, 1, p, tm, *dev, st);
   if (e != cudaSuccess) return cuda_status(e);
-  if (back) {
-    return cuda_status(launch_kernel(large_tile_kernel<true>, (unsigned)grid, 32 * (kLtWarps + 1), smem, st, p, ma, mb, mc, md));
-  } else {
-    e = launch_kernel(large_tile_kernel<false>, (unsigned)grid, 32 * (kLtWarps + 1), smem, st, p, ma, mb, mc, md);
-    if (e != cudaSuccess) return cuda_status(e);
-    const long cnt = (long)p.row_tiles * m;
-    large_tile_boundary_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(p);
+  const long cnt = (long)p.row_tiles * m;
+  large_tile_boundary_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(p);
+  return cuda_status(cudaGetLastError());
+}
+
+tridi_status large_tma_back(const float* a, const float* b, const float* c, const float* d, long n, long m,
+                            const float* sol, float* x, const LargeFused* f, cudaStream_t st) {
+  const DeviceInfo* dev = current_device();
+  if (!dev) return TRIDI_ERROR_CUDA;
+  const int mode = f ? f->mode : kBackPlain;
+  const size_t smem = mode == kBackPlain ? kBackSmem : kBackSmem + kBackResidual;
+  if ((size_t)dev->max_smem_optin < smem) return TRIDI_ERROR_UNSUPPORTED_SIZE;
+  CUtensorMap tm[4];
+  const tridi_status ts = make_maps(tm, a, b, c, d, n, m, kBackRows);
+  if (ts != TRIDI_SUCCESS) return ts;
+  LtParams p = tile_params(n, m, dev);
+  const int row_tiles = (int)((n + kBackRows - 1) / kBackRows);
+  p.sol = sol;
+  p.x = x;
+  const auto run = [&](TileKernel kern) {
+    return launch_tiles(kern, kBackThreads, smem, (long)row_tiles * p.col_tiles, kBackGroups, p, tm, *dev, st);
+  };
+  if (mode == kBackPlain) return cuda_status(run(large_back_tile_kernel<kBackPlain>));
+  p.r = f->r; p.rr = f->rr; p.dd = f->dd; p.d = f->d; p.e0 = f->e0;
+  if (mode == kBackSecond) p.x = f->x;
+  const cudaError_t e = run(mode == kBackFirst ? large_back_tile_kernel<kBackFirst> : large_back_tile_kernel<kBackSecond>);
+  if (e != cudaSuccess) return cuda_status(e);
+  if (row_tiles > 1) {
+    const unsigned grid = (unsigned)(p.col_tiles * ((row_tiles + 7) / 8));
+    if (mode == kBackFirst) large_tile_edge_kernel<kBackFirst><<<grid, 256, 0, st>>>(p, a, b, c, d);
+    else large_tile_edge_kernel<kBackSecond><<<grid, 256, 0, st>>>(p, a, b, c, f->d);
   }
   return cuda_status(cudaGetLastError());
 }
