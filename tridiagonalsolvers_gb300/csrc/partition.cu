@@ -161,37 +161,6 @@ cudaError_t launch_cta(PartParams p, int threads, const DeviceInfo& dev, cudaStr
   return launch_kernel(kern, (unsigned)grid, threads, smem, stream, p);
 }
 
-// Lanes per system and rows a lane of the warp kernel for a system of n rows:
-// the cheapest of the shapes that hold it, by the shared-memory wavefronts and
-// instructions of a row slot and of a group's separator solve (their sums
-// order the shapes as timed at 20, 61, 100, 250 and 333 rows); lanes of
-// different systems n words apart may share banks, which counts.
-constexpr int kWarpRows[] = {3, 5, 7, 9, 11, 13, 15, 17, 21, 25, 31};
-
-void warp_shape(int n, int* lps, int* rows) {
-  double best = 1e30;
-  for (int l = 1, steps = 0; l <= 32; l *= 2, ++steps) {
-    for (int K : kWarpRows) {
-      if (l * K < n || (long)(32 / l) * n > 1100) continue;
-      int hits[32] = {};
-      int conflict = 0;
-      for (int lane = 0; lane < 32; ++lane) {
-        const int g = lane / l, t = lane % l;
-        if (t * K >= n) continue;
-        const int h = ++hits[(g * n + t * K) % 32];
-        conflict = h > conflict ? h : conflict;
-      }
-      const double slot = 24.0 + 5.0 * (conflict - 1);
-      const double cost = ((double)K * slot + 60.0 + 25.0 * steps) / ((double)(32 / l) * n);
-      if (cost < best) {
-        best = cost;
-        *lps = l;
-        *rows = K;
-      }
-    }
-  }
-}
-
 tridi_status solve_f32(const float* a, const float* b, const float* c, const float* d, float* x, int n, int m,
                        cudaStream_t s) {
   const DeviceInfo* dev = current_device();
@@ -204,7 +173,7 @@ tridi_status solve_f32(const float* a, const float* b, const float* c, const flo
   p.vec = aligned16(x);
   if (n <= 32 * 31) {
     int K = 31;
-    warp_shape(n, &p.lps, &K);
+    strip_warp_shape(n, 31, 1100, &p.lps, &K);
     switch (K) {
       case 3: return cuda_status(launch_warp<3>(p, *dev, s));
       case 5: return cuda_status(launch_warp<5>(p, *dev, s));

@@ -33,30 +33,17 @@ struct Chunk {
   T lD, lC, lA;           // last interior row (row k-2), same form
 };
 
-// Eliminates the lane's k rows (0 <= k <= K), row i of the chunk being
-// (pa[i*rs], pb[i*rs], pc[i*rs], pd[i*rs]).  first/last: the chunk holds the
-// system's first/last row.
-// PREFETCH (for global-memory rows): all k rows are loaded into registers
-// before the dependent elimination chain starts, so their loads overlap.
-template <class T, int K, bool PREFETCH = false>
-__device__ __forceinline__ void chunk_eliminate(Chunk<T, K>& ch, int k, bool first, bool last, const T* pa,
-                                                const T* pb, const T* pc, const T* pd, long rs = 1) {
-  T qa[PREFETCH ? K : 1], qb[PREFETCH ? K : 1], qc[PREFETCH ? K : 1], qd[PREFETCH ? K : 1];
-  if constexpr (PREFETCH) {
-#pragma unroll
-    for (int i = 0; i < K; ++i) {
-      if (i < k - 1) {
-        qa[i] = pa[i * rs]; qb[i] = pb[i * rs]; qc[i] = pc[i * rs]; qd[i] = pd[i * rs];
-      }
-    }
-  }
+// Eliminates the lane's k rows (0 <= k <= K), interior row i of the chunk being
+// row(i), its last row sep.  first/last: the chunk holds the system's
+// first/last row.
+template <class T, int K, class RowAt>
+__device__ __forceinline__ void chunk_eliminate_rows(Chunk<T, K>& ch, int k, bool first, bool last, const RowAt& row,
+                                                     const Row<T>& sep) {
   T cprev = T(0), aprev = T(0), dprev = T(0);
 #pragma unroll
   for (int i = 0; i < K; ++i) {
     if (i < k - 1) {
-      const Row<T> r = PREFETCH ? Row<T>{qa[PREFETCH ? i : 0], qb[PREFETCH ? i : 0], qc[PREFETCH ? i : 0],
-                                         qd[PREFETCH ? i : 0]}
-                                : Row<T>{pa[i * rs], pb[i * rs], pc[i * rs], pd[i * rs]};
+      const Row<T> r = row(i);
       const T a = (i == 0 && first) ? T(0) : r.a;
       tdiv3(r.c, i == 0 ? a : -a * aprev, r.d - a * dprev, r.b - a * cprev, ch.cp[i], ch.ap[i], ch.dp[i]);
       cprev = ch.cp[i];
@@ -84,13 +71,54 @@ __device__ __forceinline__ void chunk_eliminate(Chunk<T, K>& ch, int k, bool fir
     ch.lD = T(0); ch.lC = T(0); ch.lA = T(-1);
   }
   if (k >= 1) {
-    const long o = (long)(k - 1) * rs;
-    ch.sep = Row<T>{pa[o], pb[o], pc[o], pd[o]};
+    ch.sep = sep;
     if (k == 1 && first) ch.sep.a = T(0);
     if (last) ch.sep.c = T(0);
   } else {  // lane past the end of the system: identity separator
     ch.sep = Row<T>{T(0), T(1), T(0), T(0)};
   }
+}
+
+// Rows (pa[i*rs], pb[i*rs], pc[i*rs], pd[i*rs]).  PREFETCH (for global-memory
+// rows): all k rows are loaded into registers before the dependent elimination
+// chain starts, so their loads overlap.
+template <class T, int K, bool PREFETCH = false>
+__device__ __forceinline__ void chunk_eliminate(Chunk<T, K>& ch, int k, bool first, bool last, const T* pa,
+                                                const T* pb, const T* pc, const T* pd, long rs = 1) {
+  T qa[PREFETCH ? K : 1], qb[PREFETCH ? K : 1], qc[PREFETCH ? K : 1], qd[PREFETCH ? K : 1];
+  if constexpr (PREFETCH) {
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      if (i < k - 1) {
+        qa[i] = pa[i * rs]; qb[i] = pb[i * rs]; qc[i] = pc[i * rs]; qd[i] = pd[i * rs];
+      }
+    }
+  }
+  Row<T> sep{};
+  if (k >= 1) {
+    const long o = (long)(k - 1) * rs;
+    sep = Row<T>{pa[o], pb[o], pc[o], pd[o]};
+  }
+  chunk_eliminate_rows<T, K>(
+      ch, k, first, last,
+      [&](int i) {
+        if constexpr (PREFETCH) return Row<T>{qa[i], qb[i], qc[i], qd[i]};
+        else return Row<T>{pa[i * rs], pb[i * rs], pc[i * rs], pd[i * rs]};
+      },
+      sep);
+}
+
+// The same with the right-hand sides in registers (a correction's residuals).
+template <class T, int K>
+__device__ __forceinline__ void chunk_eliminate_rhs(Chunk<T, K>& ch, int k, bool first, bool last, const T* pa,
+                                                    const T* pb, const T* pc, const T (&rhs)[K]) {
+  Row<T> sep{};
+  if (k >= 1) sep = Row<T>{pa[k - 1], pb[k - 1], pc[k - 1], T(0)};
+#pragma unroll
+  for (int i = 0; i < K; ++i)
+    if (i == k - 1) sep.d = rhs[i];
+  chunk_eliminate_rows<T, K>(
+      ch, k, first, last, [&](int i) { return Row<T>{pa[i], pb[i], pc[i], rhs[i]}; }, sep);
 }
 
 // Summary of a chunk eliminated in shared memory: what the separator system

@@ -17,12 +17,15 @@
 // x_2 = e_0 + e_1 straight to FP64 (one correction: no pair buffer, no
 // assembly pass); further sweeps run on pairs, assembled into FP64 at the end.
 // Interleaved batches that take the TMA passes form these two residuals in the
-// solver's back pass (large_tma.cu): 1024 x 65536 1.82 -> 1.42 ms.
+// solver's back pass (large_tma.cu): 1024 x 65536 1.82 -> 1.42 ms.  Contiguous
+// systems of at most 8704 rows take the first solution and the correction in
+// one kernel (refine_rows.cu).
 #include <algorithm>
 #include <cmath>
 
 #include "dfloat.cuh"
 #include "large_tma.h"
+#include "refine_rows.h"
 #include "runtime.h"
 #include "tridi_device.cuh"
 
@@ -372,13 +375,36 @@ tridi_status refine_device(const float* a, const float* b, const float* c, const
   const bool fused = df && layout == TRIDI_LAYOUT_INTERLEAVED && large_fusable(a, b, c, d, n, m) &&
                      large_fusable(a, b, c, w.r, n, m);
   tridi_status ts = TRIDI_SUCCESS;
-  if (!fused && (ts = solve32(a, b, c, d, w.e, n, m, layout, w, stream)) != TRIDI_SUCCESS) return ts;
+  double rel = 0.0;
+  // Contiguous systems a warp or a CTA holds, double-float: the first solution
+  // and one correction in one kernel (refine_rows.cu).  A tolerance that an
+  // FP32 solution may reach (its residual is some 1e-7) goes through the
+  // sweeps one by one, and so does the first solution where it turns out to
+  // be within the tolerance.
+  bool rows = df && layout == TRIDI_LAYOUT_CONTIGUOUS && max_sweeps >= 1 && tol <= 1e-8 && refine_rows_applies(n, m);
+  if (rows) {
+    double rel2[2] = {0.0, 0.0};
+    if ((ts = refine_rows_device(a, b, c, d, x, (int)n, (int)m, w.scalar, st)) != TRIDI_SUCCESS) return ts;
+    if ((e = cudaMemcpyAsync(rel2, w.scalar, sizeof(rel2), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(st)) != cudaSuccess)
+      return cuda_status(e);
+    rel = std::sqrt(rel2[1]);
+    const double rel0 = std::sqrt(rel2[0]);
+    if (rel0 <= tol || !(rel0 == rel0)) {
+      rows = false;  // the first solution was the answer
+    } else if (rel <= tol || max_sweeps == 1 || !(rel == rel)) {
+      if (sweeps_out) *sweeps_out = 1;
+      if (res_out) *res_out = rel;
+      return rel <= tol ? TRIDI_SUCCESS : TRIDI_ERROR_NOT_CONVERGED;
+    }
+  }
+  const bool one_kernel = fused || rows;  // a first correction without a residual left in w.r
+  if (!one_kernel && (ts = solve32(a, b, c, d, w.e, n, m, layout, w, stream)) != TRIDI_SUCCESS) return ts;
   if ((e = cudaMemsetAsync(w.dd, 0, sizeof(double) * m, st)) != cudaSuccess) return cuda_status(e);
 
   RefineParams p{};
   p.a = a; p.b = b; p.c = c; p.d = d; p.e = w.e; p.r = w.r; p.rr = w.rr; p.dd = w.dd;
   p.n = n; p.m = m; p.layout = layout;
-  double rel = 0.0;
   // The scalar and rr cleared before a sweep; after it the maximum relative
   // residual read back into rel.
   const auto clear = [&]() { return cudaMemsetAsync(w.scalar, 0, 256 + sizeof(double) * m, st); };
@@ -438,7 +464,12 @@ tridi_status refine_device(const float* a, const float* b, const float* c, const
     // on pairs, assembled into FP64 at the end.
     p.first = 1;
     p.mode = 0;
-    if (fused) {
+    if (rows) {  // done above; ||d||^2 per system for the later sweeps: the residual of x = 0
+      if ((e = cudaMemsetAsync(w.e, 0, sizeof(float) * count, st)) != cudaSuccess) return cuda_status(e);
+      const double rel1 = rel;
+      if ((e = pass()) != cudaSuccess) return cuda_status(e);
+      rel = rel1;
+    } else if (fused) {
       if ((e = clear()) != cudaSuccess) return cuda_status(e);
       const LargeFused f{kBackFirst, nullptr, nullptr, nullptr, w.r, w.rr, w.dd};
       if ((ts = large_solve_fused(a, b, c, d, w.e, n, m, w.inner, w.inner_bytes, f, stream)) != TRIDI_SUCCESS)
@@ -447,13 +478,14 @@ tridi_status refine_device(const float* a, const float* b, const float* c, const
     } else if ((e = pass()) != cudaSuccess) {
       return cuda_status(e);
     }
-    if (done(0)) {
+    if (!rows && done(0)) {
       refine_f32_to_fp64_kernel<<<eblocks, 256, 0, st>>>(w.e, x, count);
       if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
     } else {
       sweep = 1;
       p.first = 0;
-      if (fused) {
+      if (rows) {  // x and rel are those of one correction
+      } else if (fused) {
         if ((e = clear()) != cudaSuccess) return cuda_status(e);
         const LargeFused f{kBackSecond, d, w.e, x, nullptr, w.rr, nullptr};
         if ((ts = large_solve_fused(a, b, c, w.r, w.e2, n, m, w.inner, w.inner_bytes, f, stream)) != TRIDI_SUCCESS)
@@ -475,7 +507,7 @@ tridi_status refine_device(const float* a, const float* b, const float* c, const
         double* bufs[2] = {x, w.xalt};
         int cur = 1;
         p.mode = 2;
-        if (fused) {  // the fused sweep wrote no residual: one more pass, with a zero correction
+        if (one_kernel) {  // no residual is left: one more pass, with a zero correction
           if ((e = cudaMemsetAsync(w.e2, 0, sizeof(float) * count, st)) != cudaSuccess) return cuda_status(e);
           p.e = w.e2;
           p.xin = bufs[cur];

@@ -202,4 +202,35 @@ __device__ __forceinline__ void block_back(const BlockForward<T>& o, const Chunk
   chunk_back<T, K>(ch, k, sj, lane == 0 ? wb : up, x);
 }
 
+// Lanes per system and rows a lane of a warp kernel for a system of n rows:
+// the cheapest of the shapes that hold it, by the shared-memory wavefronts and
+// instructions of a row slot and of a group's separator solve (their sums
+// order the shapes as timed at 20, 61, 100, 250 and 333 rows); lanes of
+// different systems n words apart may share banks, which counts.
+// max_rows: rows a lane at most; max_tile: rows a warp's tile at most.
+inline void strip_warp_shape(int n, int max_rows, long max_tile, int* lps, int* rows) {
+  constexpr int kWarpRows[] = {3, 5, 7, 9, 11, 13, 15, 17, 21, 25, 31};
+  double best = 1e30;
+  for (int l = 1, steps = 0; l <= 32; l *= 2, ++steps) {
+    for (int K : kWarpRows) {
+      if (K > max_rows || l * K < n || (long)(32 / l) * n > max_tile) continue;
+      int hits[32] = {};
+      int conflict = 0;
+      for (int lane = 0; lane < 32; ++lane) {
+        const int g = lane / l, t = lane % l;
+        if (t * K >= n) continue;
+        const int h = ++hits[(g * n + t * K) % 32];
+        conflict = h > conflict ? h : conflict;
+      }
+      const double slot = 24.0 + 5.0 * (conflict - 1);
+      const double cost = ((double)K * slot + 60.0 + 25.0 * steps) / ((double)(32 / l) * n);
+      if (cost < best) {
+        best = cost;
+        *lps = l;
+        *rows = K;
+      }
+    }
+  }
+}
+
 }  // namespace tridi
