@@ -68,3 +68,15 @@ def test_nan_system_is_reported_and_apart(cuda):
     keep = np.arange(m) != 5
     assert np.isnan(rel)
     assert np.array_equal(x[:, keep], y[:, keep])
+
+
+@pytest.mark.parametrize("n", [47, 49, 63, 64, 65, 79, 80, 81, 191, 192, 193, 255, 321])
+def test_correction_from_the_back_pass(cuda, n):
+    """The correction's separator system gets its right-hand side from the
+    first sweep's back pass: row counts around its tiles (64 rows) and chunks,
+    on systems whose corrections all matter (one sweep takes the residual of
+    some 1e-7 to 1e-13; a wrong right-hand side in any chunk leaves it)."""
+    m = 64
+    arrs = workloads.weak(m, n, seed=3 * n, layout=1)
+    x, _ = _refine(cuda, arrs, n, m, 1)
+    assert gold.rel_residual(*arrs, x, layout=1).max() <= 1e-10

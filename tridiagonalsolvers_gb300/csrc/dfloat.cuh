@@ -30,20 +30,22 @@ __device__ __forceinline__ double f2d_exact(float f) {
 // so the result's bit pattern is hi's moved by k units, and as hi's double
 // has 29 zero low bits, k's parity is the sum's: the ties go to even.  hi
 // below 2^-75 (where 1/u leaves FP32's range), non-normal hi and a
-// power-of-two hi under a negative lo take one FP64 add.
+// power-of-two hi under a negative lo take one FP64 add, out of line.
+static __device__ __noinline__ uint64_t df_add_bits(float hi, float lo) {
+  return (uint64_t)__double_as_longlong(f2d_exact(hi) + f2d_exact(lo));
+}
 __device__ __forceinline__ double df_to_double(float hi, float lo) {
-  const unsigned uh = __float_as_uint(hi), ul = __float_as_uint(lo);
+  const unsigned uh = __float_as_uint(hi), sign = uh & 0x80000000u;
   const unsigned eh = (uh >> 23) & 0xffu;
-  const bool pow2_down = ((uh ^ ul) >> 31) != 0u && (uh & 0x7fffffu) == 0u && (ul & 0x7fffffffu) != 0u;
-  if (eh >= 52u && eh <= 254u && !pow2_down) {
-    const float inv_u = __uint_as_float((306u - eh) << 23);  // 2^(52 - unbiased exponent of hi)
-    const int k = __float2int_rn(__fmul_rn(lo, inv_u));
-    if (k >= -(1 << 28) && k <= (1 << 28)) {
-      const long long h = __double_as_longlong(f2d_exact(hi));
-      return __longlong_as_double((int)uh < 0 ? h - k : h + k);
-    }
+  // 2^(52 - unbiased exponent of hi), with hi's sign: k > 0 moves away from zero
+  const float sl = __fmul_rn(lo, __uint_as_float(((306u - eh) << 23) | sign));
+  const int k = __float2int_rn(sl);
+  const bool pow2_down = (uh & 0x7fffffu) == 0u && !(sl >= 0.f);
+  if (eh - 52u <= 202u && (unsigned)(k + (1 << 28)) <= (1u << 29) && !pow2_down) {
+    const long long h = (long long)(((unsigned long long)(((uh & 0x7fffffffu) >> 3) + (896u << 20)) << 32) | (uh << 29));
+    return __longlong_as_double((h + k) | (long long)((unsigned long long)sign << 32));
   }
-  return f2d_exact(hi) + f2d_exact(lo);
+  return __longlong_as_double((long long)df_add_bits(hi, lo));
 }
 
 // Knuth's TwoSum: s + e == a + b exactly.

@@ -240,7 +240,10 @@ tridi_status large_solve(const T* a, const T* b, const T* c, const T* d, T* x, l
   // interleaved FP32 with m a multiple of 32: the TMA-tiled passes (large_tma.cu)
   bool tma = false;
   if constexpr (sizeof(T) == 4) tma = large_fusable(a, b, c, d, n, m);
-  if (tma) {
+  if (fused && fused->mode == kBackSecond) {
+    // the separator system is there: the first sweep's matrix, and its right-
+    // hand side from that sweep's back pass
+  } else if (tma) {
     // the separator rows assembled in the pass (the interface area holds the
     // tile-boundary arrays only)
     const tridi_status t = large_tma_reduce(
@@ -257,10 +260,11 @@ tridi_status large_solve(const T* a, const T* b, const T* c, const T* d, T* x, l
   const tridi_status ts = large_solve<T>(r, r + p.PMp, r + 2 * p.PMp, r + 3 * p.PMp, static_cast<T*>(p.sol), p.P, m,
                                          layout, inner, inner_bytes, nullptr, stream);
   if (ts != TRIDI_SUCCESS) return ts;
-  if (tma)
+  if (tma)  // (a first sweep's boundary values: beside the separator solution, P m / 2 elements)
     return large_tma_back(reinterpret_cast<const float*>(a), reinterpret_cast<const float*>(b),
                           reinterpret_cast<const float*>(c), reinterpret_cast<const float*>(d), n, m,
-                          static_cast<const float*>(p.sol), reinterpret_cast<float*>(x), fused, st);
+                          static_cast<const float*>(p.sol), reinterpret_cast<float*>(x), fused,
+                          static_cast<float*>(p.red) + 3 * p.PMp, static_cast<float*>(p.iface) + 2 * p.PMp, st);
   large_back_kernel<T, kChunk><<<(unsigned)((PM + 127) / 128), 128, 0, st>>>(p);
   return cuda_status(cudaGetLastError());
 }

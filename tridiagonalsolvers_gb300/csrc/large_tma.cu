@@ -24,6 +24,7 @@
 
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "dfloat.cuh"
 #include "large_tma.h"
@@ -50,7 +51,8 @@ struct LtParams {
   void* x;          // back: solution (FP32, or FP64 in kBackSecond)
   const float* d;   // kBackSecond: the refined system's right-hand side ...
   const float* e0;  // ... and its first solution
-  float* r;         // kBackFirst: the residual
+  float* r;         // kBackFirst: the residual ...
+  float* red_d;     // ... and the right-hand side of its separator system; bnd: lD, fD of each tile (BS apart)
   double* rr;       // kBackFirst, kBackSecond: per-system sums of r^2 ...
   double* dd;       // ... and, kBackFirst, of d^2
   int row_tiles, col_tiles;
@@ -218,27 +220,31 @@ __global__ void __launch_bounds__(32 * (kLtWarps + 1), 1)
 // below it, by a Thomas sweep.  MODE kBackPlain: x.  kBackFirst: x (FP32,
 // exact) and the residual r = d - T x in double-float, rounded to FP32, with
 // the sums of r^2 and d^2 per system: the first sweep of the refinement without
-// reading the system again.  kBackSecond: the solve was of a correction e1
-// (right-hand side r); x = e0 + e1 in FP64 and the sum of its residuals'
-// squares, d and e0 read beside the tiles.  A tile's last row needs x of the
-// next tile's first: large_tile_edge_kernel adds its share once the pass is
-// done.
+// reading the system again.  The chunk's elimination is at hand, so r goes
+// through it at once, and the correction needs no reduce pass: its separator
+// system has the same matrix, and the right-hand side is written here.
+// kBackSecond: the solve was of a correction e1 (right-hand side r); x = e0 +
+// e1 in FP64 and the sum of its residuals' squares, d and e0 read beside the
+// tiles.  A tile's last row needs x of the next tile's first:
+// large_tile_edge_kernel adds its share once the pass is done.
 //
 // Three groups of four warps an SM, each with tiles of its own (64 rows x 32
 // systems), a private two-stage ring and its own barrier: a tile goes to
 // registers, its stage is refilled at once, and the groups cover one another's
-// dependent chains.  1024 x 65536: plain 188 us, kBackFirst 283 us, kBackSecond
-// 516 us; eight warps in step on 128-row tiles 208, 396 and 668 us; with two
-// rows' residuals in paired FP32 instructions 190, 319 and 530 us (the pairs'
-// registers).  kBackFirst and kBackSecond stand for a back pass and a pass over
-// the system of 330 and 560 us.
+// dependent chains (plain 188 us at 1024 x 65536; eight warps in step on
+// 128-row tiles 208 us).  kBackFirst 270 us and kBackSecond 337 us there (94% of
+// the copy rate); 282 and 514 us before the full-chunk branch and running
+// pointers, when kBackFirst left the correction's elimination to a reduce pass
+// of 172 us; a back pass and a pass over the system each 330 and 560 us.  With
+// two rows' residuals in paired FP32 instructions 319 and 530 us (the pairs'
+// registers).
 constexpr int kBackGroups = 3, kBackWarps = 4;           // groups a CTA, warps a group
 constexpr int kBackRows = kBackWarps * kLtChunk;         // 64
 constexpr int kBackFloats = kBackRows * kTileCols;       // per array of a tile
 constexpr int kBackThreads = 32 * kBackGroups * kBackWarps;
 constexpr size_t kBackSmem = 128 + (size_t)kBackGroups * 2 * 4 * kBackFloats * sizeof(float);
-// per group: x of the warps' first rows (hi, lo) and the norms' partial sums (r^2, d^2), both for two tiles
-constexpr size_t kBackShare = 2 * 2 * kBackWarps * 32;
+// per group, all for two tiles: x of the warps' first rows (hi, lo), the norms' partial sums (r^2, d^2) and fD
+constexpr size_t kBackShare = 2 * 2 * kBackWarps * 32 + 2 * kBackWarps * 32 / 2;
 constexpr size_t kBackResidual = kBackGroups * kBackShare * sizeof(float2);
 
 template <int MODE>
@@ -253,6 +259,7 @@ __global__ void __launch_bounds__(kBackThreads, 1)
   float* ring = reinterpret_cast<float*>(smem + 128) + (size_t)grp * 2 * 4 * kBackFloats;
   float2* exch = reinterpret_cast<float2*>(smem + kBackSmem) + grp * kBackShare;
   float2* norms = exch + 2 * kBackWarps * 32;
+  float* first_d = reinterpret_cast<float*>(norms + 2 * kBackWarps * 32);
   const int row_tiles = (int)((p.n + kBackRows - 1) / kBackRows);
   const int ntiles = row_tiles * p.col_tiles, step = (int)gridDim.x * kBackGroups;
   const int first = (int)blockIdx.x * kBackGroups + grp;
@@ -304,24 +311,43 @@ __global__ void __launch_bounds__(kBackThreads, 1)
     atomicAdd(&p.rr[sys], rs);
     if (MODE == kBackFirst) atomicAdd(&p.dd[sys], ds);
   };
+  // kBackFirst: tile t's right-hand sides of the separator system (the group's
+  // k-th tile), once every warp's fD is there; a tile's last chunk waits for the
+  // tile below (large_tile_edge_kernel)
+  float sep_d = 0.f, sep_c = 0.f;
+  const auto put_rhs = [&](int t, int k) {
+    long sys, r0;
+    column(t, sys, r0);
+    if (r0 >= p.n || (warp == kBackWarps - 1 && r0 + L < p.n)) return;
+    const float nD = warp + 1 < kBackWarps ? first_d[((k & 1) * kBackWarps + warp + 1) * 32 + lane] : 0.f;
+    p.red_d[(r0 / L) * p.m + sys] = sep_d - sep_c * nD;
+  };
+  const long row_bytes = p.m * (long)sizeof(float);
+  const auto down = [&](auto* q, long bytes) {  // q one row on
+    return reinterpret_cast<decltype(q)>(reinterpret_cast<uintptr_t>(q) + bytes);
+  };
   float sl_next, sj_next;
   separators(first, sl_next, sj_next);
   int k = 0;
-  for (int t = first; t < ntiles; t += step, ++k) {
+  bool live = true;
+  // One tile; FULL: all L rows of the warp's chunks exist (their bounds checks
+  // are a tenth of the pass's instructions).
+  const auto tile = [&](auto full_chunk, int t, long sys, long r0, int kr) {
+    constexpr bool FULL = decltype(full_chunk)::value;
     const int s = k & 1;
-    long sys, r0;
-    column(t, sys, r0);
     const float sl = sl_next, sj = sj_next;
     separators(t + step, sl_next, sj_next);
-    const long rem = p.n - r0;
-    const int kr = rem <= 0 ? 0 : (rem < L ? (int)rem : L);
     const long g0 = r0 * p.m + sys;
-    float dv[MODE == kBackSecond ? L : 1], e0[MODE == kBackSecond ? L : 1], e0m = 0.f;
+    [[maybe_unused]] float dv[MODE == kBackSecond ? L : 1], e0[MODE == kBackSecond ? L : 1], e0m = 0.f;
     if constexpr (MODE == kBackSecond) {
+      const float *gd = p.d + g0, *ge = p.e0 + g0;
 #pragma unroll
       for (int q = 0; q < L; ++q) {
-        dv[q] = q < kr ? __ldg(p.d + g0 + (long)q * p.m) : 0.f;
-        e0[q] = q < kr ? __ldg(p.e0 + g0 + (long)q * p.m) : 0.f;
+        const bool in = FULL || q < kr;
+        dv[q] = in ? __ldg(gd) : 0.f;
+        e0[q] = in ? __ldg(ge) : 0.f;
+        gd = down(gd, row_bytes);
+        ge = down(ge, row_bytes);
       }
       if (kr > 0 && r0 > 0) e0m = __ldg(p.e0 + g0 - p.m);
     }
@@ -336,34 +362,38 @@ __global__ void __launch_bounds__(kBackThreads, 1)
       d[q] = st[3 * kBackFloats + q * kTileCols];
     }
     fence_proxy_async_smem();
-    if (!named_sync_and(1 + grp, GT, ok)) return;  // every column is read
+    live = named_sync_and(1 + grp, GT, ok);  // every column is read
+    if (!live) return;
     if (leader && t + 2 * step < ntiles) issue(t + 2 * step, s);
     if (MODE != kBackPlain && k > 0) flush(t - step, k - 1);
+    if (MODE == kBackFirst && k > 0) put_rhs(t - step, k - 1);
     if (r0 == 0) a[0] = 0.f;
-    float cp[L], x[L], cprev = 0.f, dprev = sl;
+    // inv[q] = 1 / pivot (kBackFirst needs it again), or c' = c inv
+    float inv[L], x[L], cprev = 0.f, dprev = sl;
 #pragma unroll
     for (int q = 0; q < L; ++q) {
-      if (q < kr - 1) {
-        tdiv2(c[q], d[q] - a[q] * dprev, q == 0 ? b[q] : b[q] - a[q] * cprev, cp[q], x[q]);
-        cprev = cp[q];
-        dprev = x[q];
+      if (q < L - 1 && (FULL || q < kr - 1)) {
+        inv[q] = tdiv(1.f, q == 0 ? b[q] : b[q] - a[q] * cprev);
+        cprev = c[q] * inv[q];
+        x[q] = dprev = (d[q] - a[q] * dprev) * inv[q];
+        if (MODE != kBackFirst) inv[q] = cprev;
       }
     }
+    const auto cp = [](float ci, float w) { return MODE == kBackFirst ? ci * w : w; };
     float xn = sj;
     if constexpr (MODE == kBackPlain) {
-      float* gx = static_cast<float*>(p.x) + g0;
+      float* gx = static_cast<float*>(p.x) + g0 + (L - 1) * p.m;
 #pragma unroll
       for (int q = L - 1; q >= 0; --q) {
-        if (q <= kr - 1) {
-          if (q <= kr - 2) xn = x[q] - cp[q] * xn;
-          gx[(long)q * p.m] = xn;
-        }
+        if (q < L - 1 && (FULL || q <= kr - 2)) xn = x[q] - cp(c[q], inv[q]) * xn;
+        if (FULL || q <= kr - 1) *gx = xn;
+        gx = down(gx, -row_bytes);
       }
     } else {
 #pragma unroll
       for (int q = L - 1; q >= 0; --q) {
-        if (q <= kr - 2) xn = x[q] - cp[q] * xn;
-        x[q] = q <= kr - 1 ? xn : 0.f;
+        if (q < L - 1 && (FULL || q <= kr - 2)) xn = x[q] - cp(c[q], inv[q]) * xn;
+        x[q] = FULL || q <= kr - 1 ? xn : 0.f;
       }
       // x as pairs: the row above, the lane's rows, the row below
       float lo[MODE == kBackSecond ? L : 1] = {};
@@ -383,46 +413,82 @@ __global__ void __launch_bounds__(kBackThreads, 1)
       const bool end = kr > 0 && r0 + kr == p.n;
       const float2 below = warp + 1 < kBackWarps && !end ? ex[(warp + 1) * 32 + lane] : make_float2(0.f, 0.f);
       float rs = 0.f, ds = 0.f;
+      [[maybe_unused]] float lD = 0.f;
+      float* gx = static_cast<float*>(p.x) + g0;
+      double* gx64 = static_cast<double*>(p.x) + g0;
+      float* gr = p.r + g0;
 #pragma unroll
       for (int q = 0; q < L; ++q) {
-        if (q < kr) {
+        if (FULL || q < kr) {
           const float2 xi = pair(q);
-          const bool lastrow = q == kr - 1;
-          const long o = g0 + (long)q * p.m;
-          if (MODE == kBackFirst) static_cast<float*>(p.x)[o] = xi.x;
-          else static_cast<double*>(p.x)[o] = df_to_double(xi.x, xi.y);
+          const bool lastrow = FULL ? q == L - 1 : q == kr - 1;
+          if (MODE == kBackFirst) *gx = xi.x;
+          else *gx64 = df_to_double(xi.x, xi.y);
           const float2 xp = lastrow ? below : pair(q + 1 < L ? q + 1 : q);
           const float di = MODE == kBackSecond ? dv[MODE == kBackSecond ? q : 0] : d[q];
           const float ci = lastrow && end ? 0.f : c[q];
           const float r = MODE == kBackSecond ? df_residual(a[q], b[q], ci, di, xm, xi, xp)
                                               : f_residual(a[q], b[q], ci, di, xm.x, xi.x, xp.x);
           if (!(lastrow && open)) {
-            if (MODE == kBackFirst) p.r[o] = r;
+            if (MODE == kBackFirst) *gr = r;
             rs = fmaf(r, r, rs);
             ds = fmaf(di, di, ds);
           }
           xm = xi;
+          if constexpr (MODE == kBackFirst) {  // r through the elimination, d' in x's place
+            if (lastrow) {
+              sep_d = r - a[q] * lD;
+              sep_c = ci;
+            } else {
+              lD = (r - a[q] * lD) * inv[q];
+              x[q] = lD;
+            }
+          }
         }
+        gx = down(gx, row_bytes);
+        gx64 = down(gx64, 2 * row_bytes);
+        gr = down(gr, row_bytes);
       }
       norms[((k & 1) * kBackWarps + warp) * 32 + lane] = make_float2(rs, ds);
+      if constexpr (MODE == kBackFirst) {
+        float fD = 0.f;
+#pragma unroll
+        for (int q = L - 2; q >= 0; --q)
+          if (FULL || q <= kr - 2) fD = x[q] - cp(c[q], inv[q]) * fD;
+        first_d[((k & 1) * kBackWarps + warp) * 32 + lane] = fD;
+        const long o = (r0 / kBackRows) * p.m + sys;
+        if (open) p.bnd[o] = lD;
+        if (warp == 0) p.bnd[p.BS + o] = fD;
+      }
     }
+  };
+  for (int t = first; t < ntiles; t += step, ++k) {
+    long sys, r0;
+    column(t, sys, r0);
+    const long rem = p.n - r0;
+    if (rem >= L) tile(std::true_type{}, t, sys, r0, L);
+    else tile(std::false_type{}, t, sys, r0, rem <= 0 ? 0 : (int)rem);
+    if (!live) return;
   }
   if (MODE != kBackPlain && k > 0) {
     named_sync_and(1 + grp, GT, true);
     flush(first + (k - 1) * step, k - 1);
+    if (MODE == kBackFirst) put_rhs(first + (k - 1) * step, k - 1);
   }
 }
 
 // v as hi + lo, hi its significand's upper 24 bits and lo the next 24, on the
 // integer units (three FP64 instructions a value bound the kernel below);
-// values outside FP32's normal range take those.
-__device__ __forceinline__ float2 double_to_pair(double v) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+// values outside FP32's normal range take those, out of line: inline, the
+// compiler issued them for every value and the FP64 pipe was 72% busy).
+__device__ __noinline__ float2 double_to_pair_slow(unsigned long long bits) {
+  const double v = __longlong_as_double((long long)bits);
+  const float hi = __double2float_rn(v);
+  return make_float2(hi, __double2float_rn(v - (double)hi));
+}
+__device__ __forceinline__ float2 double_to_pair(unsigned long long u) {
   const int e = (int)((u >> 52) & 0x7ff) - 1023;  // v = +-1.f * 2^e
-  if (e < -60 || e > 120) {
-    const float hi = __double2float_rn(v);
-    return make_float2(hi, __double2float_rn(v - (double)hi));
-  }
+  if (e < -60 || e > 120) return double_to_pair_slow(u);
   const unsigned sign = (unsigned)(u >> 32) & 0x80000000u;
   const float hi = __uint_as_float(sign | ((unsigned)(e + 127) << 23) | ((unsigned)(u >> 29) & 0x7fffffu));
   const float ulp = __uint_as_float(sign | ((unsigned)(e + 127 - 52) << 23));  // 2^(e - 52)
@@ -430,7 +496,8 @@ __device__ __forceinline__ float2 double_to_pair(double v) {
 }
 
 // The rows that large_back_tile_kernel leaves open (the last of each tile but
-// the system's last row): their residuals and shares of the norms.  A warp
+// the system's last row): their residuals, shares of the norms and separator
+// rows.  A warp
 // takes 32 systems of one tile row, a block eight tile rows.
 template <int MODE>
 __global__ void __launch_bounds__(256) large_tile_edge_kernel(LtParams p, const float* __restrict__ a,
@@ -442,14 +509,18 @@ __global__ void __launch_bounds__(256) large_tile_edge_kernel(LtParams p, const 
   const long i = ((long)(blockIdx.x / p.col_tiles) * 8 + warp + 1) * kBackRows - 1;
   const auto x_at = [&](long o) {
     if constexpr (MODE == kBackFirst) return make_float2(static_cast<const float*>(p.x)[o], 0.f);
-    return double_to_pair(static_cast<const double*>(p.x)[o]);
+    return double_to_pair(static_cast<const unsigned long long*>(p.x)[o]);
   };
   float2 sums = make_float2(0.f, 0.f);
   if (i < p.n - 1) {
     const long o = i * p.m + sys;
     const float di = d[o];
     const float r = df_residual(a[o], b[o], c[o], di, x_at(o - p.m), x_at(o), x_at(o + p.m));
-    if (MODE == kBackFirst) p.r[o] = r;
+    if (MODE == kBackFirst) {  // and the chunk's separator row
+      p.r[o] = r;
+      const long t = (i / kBackRows) * p.m + sys;
+      p.red_d[(i / kLtChunk) * p.m + sys] = r - a[o] * p.bnd[t] - c[o] * p.bnd[p.BS + t + p.m];
+    }
     sums = make_float2(r * r, di * di);
   }
   part[warp][lane] = sums;
@@ -500,7 +571,8 @@ bool large_tma_ok(const float* a, const float* b, const float* c, const float* d
 
 // Bytes of the boundary arrays of a reduce pass (within the 10 * PMp
 // interface floats the register kernels use).
-long large_tma_boundary_stride(long n, long m) { return ((((n + kTileRows - 1) / kTileRows) * m) + 63) & ~63L; }
+long round_up64(long v) { return (v + 63) & ~63L; }
+long large_tma_boundary_stride(long n, long m) { return round_up64((n + kTileRows - 1) / kTileRows * m); }
 
 // One TMA pass.  large_tma_reduce: the separator system (with the assembly of
 // separator rows fused in; bnd: scratch of 10 boundary arrays).
@@ -555,7 +627,8 @@ tridi_status large_tma_reduce(const float* a, const float* b, const float* c, co
 }
 
 tridi_status large_tma_back(const float* a, const float* b, const float* c, const float* d, long n, long m,
-                            const float* sol, float* x, const LargeFused* f, cudaStream_t st) {
+                            const float* sol, float* x, const LargeFused* f, float* red_d, float* bnd,
+                            cudaStream_t st) {
   const DeviceInfo* dev = current_device();
   if (!dev) return TRIDI_ERROR_CUDA;
   const int mode = f ? f->mode : kBackPlain;
@@ -573,6 +646,7 @@ tridi_status large_tma_back(const float* a, const float* b, const float* c, cons
   };
   if (mode == kBackPlain) return cuda_status(run(large_back_tile_kernel<kBackPlain>));
   p.r = f->r; p.rr = f->rr; p.dd = f->dd; p.d = f->d; p.e0 = f->e0;
+  p.red_d = red_d; p.bnd = bnd; p.BS = round_up64((long)row_tiles * m);
   if (mode == kBackSecond) p.x = f->x;
   const cudaError_t e = run(mode == kBackFirst ? large_back_tile_kernel<kBackFirst> : large_back_tile_kernel<kBackSecond>);
   if (e != cudaSuccess) return cuda_status(e);

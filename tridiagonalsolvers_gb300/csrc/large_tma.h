@@ -11,9 +11,11 @@ namespace tridi {
 enum { kBackPlain = 0, kBackFirst = 1, kBackSecond = 2 };
 
 // A solve that is a sweep of the refinement (double-float residual).
-// kBackFirst: x is the first solution (FP32); r, rr and dd are written.
-// kBackSecond: the solve is of the correction to e0; x receives e0 +
-// correction in FP64, rr the squares of d - T x.  rr and dd are added to.
+// kBackFirst: x is the first solution (FP32); r, rr and dd are written, and r's
+// share of the separator system.  kBackSecond: the solve is of the correction
+// to e0, with the separator system that kBackFirst left in the workspace (the
+// next call on it); x receives e0 + correction in FP64, rr the squares of
+// d - T x.  rr and dd are added to.
 struct LargeFused {
   int mode;
   const float* d;   // kBackSecond
@@ -28,7 +30,8 @@ bool large_tma_ok(const float* a, const float* b, const float* c, const float* d
 tridi_status large_tma_reduce(const float* a, const float* b, const float* c, const float* d, long n, long m, long P,
                               long PMp, float* red, float* bnd, cudaStream_t st);
 tridi_status large_tma_back(const float* a, const float* b, const float* c, const float* d, long n, long m,
-                            const float* sol, float* x, const LargeFused* f, cudaStream_t st);
+                            const float* sol, float* x, const LargeFused* f, float* red_d, float* bnd,
+                            cudaStream_t st);
 
 // Whether a solve of this interleaved system takes the TMA passes (and so can
 // be fused with a sweep).
