@@ -192,3 +192,27 @@ def test_double_float_to_fp64_is_correctly_rounded(cuda):
     got = out.cpu().numpy()
     mism = np.flatnonzero(got != want)
     assert mism.size == 0, f"{mism.size} mismatches, first hi={hi[mism[0]]!r} lo={lo[mism[0]]!r}"
+
+
+@pytest.mark.parametrize("residual", ["df", "fp64"])
+@pytest.mark.parametrize("sweeps", [1, 2])
+def test_refined_from_the_factors(cuda, residual, sweeps):
+    """One correction solved with the first solve's factors (two sweeps: the
+    general form), at the limits of the threads a system gets and where chunks
+    and the passes' groups of two and four rows are ragged.  One sweep takes
+    the residual from some 1e-7 to some 1e-13."""
+    from tridiagonalsolvers_gb300.ragged import RaggedRefiner
+
+    rng = np.random.default_rng(7 * sweeps)
+    sizes = np.concatenate([np.arange(1, 70), rng.integers(70, 481, 40), [480, 481, 482, 483, 993, 4799, 4800, 4801],
+                            rng.integers(481, 4801, 20), rng.integers(4801, 6817, 20), [6815, 6816, 6817, 8192, 8961]])
+    rng.shuffle(sizes)
+    a, b, c, d, off = workloads.adi(sizes, seed=sweeps)
+    total = int(off[-1])
+    r = RaggedRefiner(RaggedPlan(off, refine=True), *(_dev(cuda, v, total) for v in (a, b, c, d)), sweeps=sweeps,
+                      residual=residual, graph=False)
+    x, rel = r.run()
+    x = x.cpu().numpy()[:total]
+    res, _ = gold.check_ragged(a, b, c, d, x, off)
+    assert res.max() <= 1e-10
+    assert rel <= 4 * res.max() + 1e-13 and res.max() <= 4 * rel + 1e-13

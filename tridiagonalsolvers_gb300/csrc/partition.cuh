@@ -134,7 +134,6 @@ struct ChunkSummary {
 // right-hand side functor is told the chunk's first row (start) and then
 // called for the chunk's rows in order.
 struct RhsStaged {
-  static constexpr bool kPairs = false;  // true: pair(i, row i, row i + 1) gives two rows' right-hand sides
   __device__ __forceinline__ void start(int) const {}
   template <class T>
   __device__ __forceinline__ T operator()(int, T, T, T, T d) const {
@@ -160,28 +159,10 @@ __device__ __forceinline__ void chunk_eliminate_smem(ChunkSummary<T>& cs, int k,
     sa[i] = an; sc[i] = cn; sd[i] = dn;
     cprev = cn; aprev = an; dprev = dn;
   };
-  if constexpr (Rhs::kPairs) {
-    // the right-hand sides of rows i and i + 1 formed together (they do not
-    // depend on the elimination), the two rows then eliminated in order
-    int i = 0;
-#pragma unroll 2
-    for (; i + 1 < k - 1; i += 2) {
-      const T a0 = sa[i], b0 = sb[i], c0 = sc[i], d0 = sd[i];
-      const T a1 = sa[i + 1], b1 = sb[i + 1], c1 = sc[i + 1], d1 = sd[i + 1];
-      const auto r = rhs.pair(i, a0, b0, c0, d0, a1, b1, c1, d1);
-      step(i, a0, b0, c0, r.x);
-      step(i + 1, a1, b1, c1, r.y);
-    }
-    if (i < k - 1) {
-      const T a0 = sa[i], b0 = sb[i], c0 = sc[i];
-      step(i, a0, b0, c0, rhs(i, a0, b0, c0, sd[i]));
-    }
-  } else {
 #pragma unroll 4
-    for (int i = 0; i < k - 1; ++i) {
-      const T a0 = sa[i], b0 = sb[i], c0 = sc[i];
-      step(i, a0, b0, c0, rhs(i, a0, b0, c0, sd[i]));
-    }
+  for (int i = 0; i < k - 1; ++i) {
+    const T a0 = sa[i], b0 = sb[i], c0 = sc[i];
+    step(i, a0, b0, c0, rhs(i, a0, b0, c0, sd[i]));
   }
   T D = T(0), C = T(-1), A = T(0);
 #pragma unroll 4
@@ -228,17 +209,116 @@ __device__ __forceinline__ void chunk_back_smem(int k, T sj, T sl, const T* __re
   }
 }
 
-// Same, with x_i written over the chunk's d_i (row i's d is read once, by
-// the step that produces x_i).
-template <class T>
-__device__ __forceinline__ void chunk_back_smem_over_d(int k, T sj, T sl, const T* __restrict__ sa,
-                                                       const T* __restrict__ sc, T* __restrict__ sd) {
+// ---- a chunk in shared memory, eliminated once for two right-hand sides ----
+// chunk_factor_smem leaves 1 / p_i over b, with the pivots p_i (the separator
+// row's b becomes 1; a, c and d stay), and the chunk's summary, accumulated on
+// the way (chunk_eliminate_smem reads the rows again for it): with c' = c / p and
+// P the product of the -c' before it, a block of four rows adds P times its own
+// D = d'_0 - c'_0 (d'_1 - c'_1 (d'_2 - c'_2 d'_3)), and A likewise, so that the
+// sums' roundings are those of the few blocks that P leaves large (summed row by
+// row, the error of a refined batch grew by half).  chunk_between_smem then
+// solves between the separators.  For a second right-hand side a / p goes over
+// a, c / p over c and g = r / p anywhere: chunk_rhs_smem gives its D and last
+// d', chunk_between_scaled_smem its unknowns.  (With the scaled rows in the first
+// solve as well, both solves carry the same rounding in the matrix, and the
+// refined error grew by 6%.)
+__device__ __forceinline__ void chunk_factor_smem(ChunkSummary<float>& cs, int k, bool first, bool last,
+                                                  float* __restrict__ sa, float* __restrict__ sb,
+                                                  const float* __restrict__ sc, const float* __restrict__ sd) {
+  float cprev = 0.f, aprev = -1.f, dprev = 0.f, P = 1.f, D = 0.f, A = 0.f;
+  if (first && k >= 1) sa[0] = 0.f;
+  const auto step = [&](int i) {
+    const float a = sa[i];
+    const float inv = tdiv(1.f, sb[i] - a * cprev);
+    cprev = sc[i] * inv;
+    aprev = -a * aprev * inv;
+    dprev = (sd[i] - a * dprev) * inv;
+    sb[i] = inv;
+  };
+  int i = 0;
+  for (; i + 4 < k; i += 4) {
+    float c[4], a[4], d[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      step(i + q);
+      c[q] = cprev; a[q] = aprev; d[q] = dprev;
+    }
+    D += P * (d[0] - c[0] * (d[1] - c[1] * (d[2] - c[2] * d[3])));
+    A += P * (a[0] - c[0] * (a[1] - c[1] * (a[2] - c[2] * a[3])));
+    P *= (c[0] * c[1]) * (c[2] * c[3]);
+  }
+  for (; i < k - 1; ++i) {
+    step(i);
+    D += P * dprev;
+    A += P * aprev;
+    P *= -cprev;
+  }
+  cs.fD = D; cs.fC = -P; cs.fA = A;
+  cs.lD = dprev; cs.lC = cprev; cs.lA = aprev;
+  cs.sep = Row<float>{0.f, 1.f, 0.f, 0.f};
+  if (k >= 1) {
+    cs.sep = Row<float>{sa[k - 1], sb[k - 1], last ? 0.f : sc[k - 1], sd[k - 1]};
+    sb[k - 1] = 1.f;
+  }
+}
+
+// The chunk's unknowns over d, between sl (the row before it) and sj (its last).
+__device__ __forceinline__ void chunk_between_smem(int k, float sj, float sl, const float* __restrict__ sa,
+                                                   const float* __restrict__ inv, const float* __restrict__ sc,
+                                                   float* __restrict__ sd) {
+  float v = sl;
+#pragma unroll 4
+  for (int i = 0; i < k - 1; ++i) {
+    v = (sd[i] - sa[i] * v) * inv[i];
+    sd[i] = v;
+  }
   if (k >= 1) sd[k - 1] = sj;
-  T xn = sj;
+  v = sj;
 #pragma unroll 4
   for (int i = k - 2; i >= 0; --i) {
-    xn = sd[i] - sc[i] * xn - sa[i] * sl;
-    sd[i] = xn;
+    v = sd[i] - sc[i] * v * inv[i];
+    sd[i] = v;
+  }
+}
+
+// The first row's D and the last interior row's d' of a right-hand side g
+// (divided by the pivots, as sa is).
+__device__ __forceinline__ void chunk_rhs_smem(int k, const float* __restrict__ sa, const float* __restrict__ sc,
+                                               const float* __restrict__ g, float& fD, float& lD) {
+  float P = 1.f, D = 0.f, dprev = 0.f;
+  int i = 0;
+  for (; i + 4 < k; i += 4) {
+    float c[4], d[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      d[q] = dprev = g[i + q] - sa[i + q] * dprev;
+      c[q] = sc[i + q];
+    }
+    D += P * (d[0] - c[0] * (d[1] - c[1] * (d[2] - c[2] * d[3])));
+    P *= (c[0] * c[1]) * (c[2] * c[3]);
+  }
+  for (; i < k - 1; ++i) {
+    dprev = g[i] - sa[i] * dprev;
+    D += P * dprev;
+    P *= -sc[i];
+  }
+  fD = D; lD = dprev;
+}
+
+__device__ __forceinline__ void chunk_between_scaled_smem(int k, float sj, float sl, const float* __restrict__ sa,
+                                                          const float* __restrict__ sc, float* __restrict__ g) {
+  float v = sl;
+#pragma unroll 4
+  for (int i = 0; i < k - 1; ++i) {
+    v = g[i] - sa[i] * v;
+    g[i] = v;
+  }
+  if (k >= 1) g[k - 1] = sj;
+  v = sj;
+#pragma unroll 4
+  for (int i = k - 2; i >= 0; --i) {
+    v = g[i] - sc[i] * v;
+    g[i] = v;
   }
 }
 

@@ -49,7 +49,8 @@
 // re-staging, ||d - T x|| / ||d|| per system (its maximum over the batch goes
 // to one device word) and x is written once as FP64.  So HBM sees
 // each coefficient once and each unknown once (16 B in, 8 B out per row).
-// Extended precision is either native FP64 (RES_FP64) or double-float, an
+// One sweep (the usual case) eliminates once and solves the correction from
+// the factors (group_refine1).  Extended precision is either native FP64 (RES_FP64) or double-float, an
 // unevaluated sum of two FP32 values with a 48-bit significand (RES_DF).
 // BIG systems refine the same way with their x and r in a global scratch.
 //
@@ -73,8 +74,15 @@ constexpr int kTeams = 3;              // consumer teams (see the file comment)
 constexpr int kTeamWarps = kRagWarps / kTeams;      // 5
 constexpr int kTeamThreads = 32 * kTeamWarps;       // 160
 constexpr int kSlots = 9;              // items in flight (descriptor slots), 3 per team
+// Default sizes, of the system alone: its solution does not depend on the batch
+// it is in.  A group's separators and barriers cost latency, so a full batch
+// prefers narrow groups (480 to 1000 rows refined, 2000 systems: 33.3 us by
+// teams, 23.1 by warps; 4800 to 6800 rows, 300 systems: 29.0 us by the CTA, 24.8
+// by teams) and a small one wide groups (50 to 900 rows, 300 systems: 14.6 us
+// with warps up to 480 rows, 18.9 up to 992; 4800 to 6800 rows, 150 systems: 18.7
+// by the CTA, 21.1 by teams).  These limits suit the small; tuning knows better.
 constexpr int kWarpMaxRows = 480;      // MULTI systems by default: up to 15 rows per lane
-constexpr int kGroupMaxRows = 4800;    // GROUP systems by default: up to 30 rows per thread
+constexpr int kGroupMaxRows = 4800;    // GROUP systems by default: up to 31 rows per thread
 constexpr int kMaxItemSystems = kTeamWarps;  // 5
 static_assert(kTeamWarps & 1, "odd separator rows per lane in warp_solve_rows");
 static_assert(kTeams * kTeamWarps == kRagWarps && kSlots % kTeams == 0, "team shape");
@@ -88,8 +96,8 @@ constexpr int kBigScratchRows = 2 * kBigSepRows;        // ring rows a BIG item 
 enum ItemKind : int { kMulti = 0, kGroup = 1, kSingle = 2, kBig = 3, kEnd = 4 };
 // Refined modes: kRefineDF / kRefineFP64 keep x in two extra ring arrays
 // (any number of sweeps); the one-correction modes kRefine1DF / kRefine1FP64
-// (sweeps == 1) keep the FP32 solution in the b words and the correction in
-// the d words, so their ring holds as many rows as the plain one.
+// (sweeps == 1) keep the FP32 solution in the d words and the correction in
+// the b words, so their ring holds as many rows as the plain one.
 enum RagMode : int { kPlain = 0, kRefineDF = 1, kRefineFP64 = 2, kRefine1DF = 3, kRefine1FP64 = 4 };
 __host__ __device__ constexpr bool one_correction(int mode) { return mode >= kRefine1DF; }
 // DF or FP64: the residual arithmetic of a refined mode
@@ -271,9 +279,6 @@ __device__ __forceinline__ void group_rel_max(float rr, float dd, int gt, int ba
 // separators solved by PCR in warp shuffles (gt == 32) or by one warp of the
 // group (warp_solve_rows over shared memory R: 4*gt floats, X: gt, F0:
 // 3*(gt/32)), back substitution; emit(i, x_i) for every row.
-// Emit tag: x_i written over the ring's d_i.
-struct EmitOverD {};
-
 // The m = 32 q rows held in R (a, b, c, d at R, R + m, R + 2m, R + 3m; q
 // odd, so the lanes' strided accesses are conflict-free) solved by one warp
 // into X: lane l eliminates rows [l q, l q + q) in place, the 32 lane
@@ -306,21 +311,58 @@ template <class Rhs>
 struct ChunkRhs {
   const Rhs& rhs;
   int r0;
-  static constexpr bool kPairs = Rhs::kPairs;
   __device__ __forceinline__ float operator()(int i, float a, float b, float c, float d) const {
     return rhs(r0 + i, a, b, c, d);
   }
-  __device__ __forceinline__ float2 pair(int i, float a0, float b0, float c0, float d0, float a1, float b1, float c1,
-                                         float d1) const {
-    return rhs.pair(r0 + i, a0, b0, c0, d0, a1, b1, c1, d1);
-  }
 };
+
+// The first lane of each warp gets its first row's value q (of three) to the
+// last lane of the warp before, through F0 (one group barrier); nv: the values
+// of the next lane.
+template <int Q>
+__device__ __forceinline__ void group_next(const float (&v)[Q], float (&nv)[Q], int gt, int bar, int gtid, float* F0) {
+#pragma unroll
+  for (int q = 0; q < Q; ++q) nv[q] = __shfl_down_sync(kFull, v[q], 1);
+  if (gt == 32) return;
+  const int lane = gtid & 31, gw = gtid >> 5;
+  if (lane == 0) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) F0[gw * 3 + q] = v[q];
+  }
+  group_sync(bar, gt);
+  if (lane == 31 && gw + 1 < gt / 32) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) nv[q] = F0[(gw + 1) * 3 + q];
+  }
+}
+
+// The separators of a group, one row sr a thread: x of the thread's (sj) and
+// of the one before (sl).
+__device__ __forceinline__ void group_separators(const Row<float>& sr, int gt, int bar, int gtid, float* R, float* X,
+                                                 float& sj, float& sl) {
+  const int lane = gtid & 31;
+  if (gt == 32) {
+    sj = warp_pcr32<float>(sr);
+    sl = __shfl_up_sync(kFull, sj, 1);
+    if (lane == 0) sl = 0.f;
+    return;
+  }
+  // one warp solves the separators (gt / 32 rows per lane: 5 for a team,
+  // 15 for the CTA), the others wait at the barrier: measured faster than
+  // a PCR over the CTA's 480 rows in shared memory (9 steps, each two
+  // barriers of all 15 warps)
+  R[gtid] = sr.a; R[gt + gtid] = sr.b; R[2 * gt + gtid] = sr.c; R[3 * gt + gtid] = sr.d;
+  group_sync(bar, gt);
+  if (gtid < 32) warp_solve_rows(R, X, gt, lane);
+  group_sync(bar, gt);
+  sj = X[gtid];
+  sl = gtid > 0 ? X[gtid - 1] : 0.f;
+}
 
 template <class Emit, class Rhs = RhsStaged>
 __device__ __forceinline__ void group_solve(int n, int gt, int bar, int gtid, float* sa, const float* sb, float* sc,
                                             float* sd, float* R, float* X, float* F0, Emit& emit,
                                             const Rhs& rhs = Rhs()) {
-  const int lane = gtid & 31, gw = gtid >> 5;
   const int kk = odd_ceil_dev((n + gt - 1) / gt);
   const int r0 = gtid * kk;
   int kr = n - r0;
@@ -329,40 +371,12 @@ __device__ __forceinline__ void group_solve(int n, int gt, int bar, int gtid, fl
   rhs.start(r0);
   chunk_eliminate_smem<float>(cs, kr, gtid == 0, r0 + kr == n && kr > 0, sa + r0, sb + r0, sc + r0, sd + r0,
                               ChunkRhs<Rhs>{rhs, r0});
-  float nD = __shfl_down_sync(kFull, cs.fD, 1);
-  float nC = __shfl_down_sync(kFull, cs.fC, 1);
-  float nA = __shfl_down_sync(kFull, cs.fA, 1);
-  float sj, sl;
-  if (gt == 32) {
-    sj = warp_pcr32<float>(separator_row_s<float>(cs, nD, nC, nA));
-    sl = __shfl_up_sync(kFull, sj, 1);
-    if (lane == 0) sl = 0.f;
-  } else {
-    if (lane == 0) {
-      F0[gw * 3 + 0] = cs.fD; F0[gw * 3 + 1] = cs.fC; F0[gw * 3 + 2] = cs.fA;
-    }
-    group_sync(bar, gt);
-    if (lane == 31 && gw + 1 < gt / 32) {
-      nD = F0[(gw + 1) * 3 + 0]; nC = F0[(gw + 1) * 3 + 1]; nA = F0[(gw + 1) * 3 + 2];
-    }
-    Row<float> sr = separator_row_s<float>(cs, nD, nC, nA);
-    // one warp solves the separators (gt / 32 rows per lane: 5 for a team,
-    // 15 for the CTA), the others wait at the barrier: measured faster than
-    // a PCR over the CTA's 480 rows in shared memory (9 steps, each two
-    // barriers of all 15 warps)
-    R[gtid] = sr.a; R[gt + gtid] = sr.b; R[2 * gt + gtid] = sr.c; R[3 * gt + gtid] = sr.d;
-    group_sync(bar, gt);
-    if (gw == 0) warp_solve_rows(R, X, gt, lane);
-    group_sync(bar, gt);
-    sj = X[gtid];
-    sl = gtid > 0 ? X[gtid - 1] : 0.f;
-  }
-  if constexpr (std::is_same_v<Emit, EmitOverD>) {
-    chunk_back_smem_over_d<float>(kr, sj, sl, sa + r0, sc + r0, sd + r0);
-  } else {
-    auto em = [&](int i, float v) { emit(r0 + i, v); };
-    chunk_back_smem<float>(kr, sj, sl, sa + r0, sc + r0, sd + r0, em);
-  }
+  const float f[3] = {cs.fD, cs.fC, cs.fA};
+  float nf[3], sj, sl;
+  group_next(f, nf, gt, bar, gtid, F0);
+  group_separators(separator_row_s<float>(cs, nf[0], nf[1], nf[2]), gt, bar, gtid, R, X, sj, sl);
+  auto em = [&](int i, float v) { emit(r0 + i, v); };
+  chunk_back_smem<float>(kr, sj, sl, sa + r0, sc + r0, sd + r0, em);
   if (gt != 32) group_sync(bar, gt);  // F0 / R / X reused by the next solve
 }
 
@@ -458,7 +472,6 @@ struct Restage {
   const float* src_c;
   const float* src_d;
   uint32_t bytes;
-  bool with_d;  // false: a and c only
 };
 
 __device__ __forceinline__ void restage(const Restage& rs, uint32_t& par, int gt, int bar, int gtid,
@@ -466,10 +479,10 @@ __device__ __forceinline__ void restage(const Restage& rs, uint32_t& par, int gt
   fence_proxy_async_smem();
   gsync(bar, gt);
   if (gtid == 0) {
-    mbar_arrive_expect_tx(rs.mb, (rs.with_d ? 3u : 2u) * rs.bytes);
+    mbar_arrive_expect_tx(rs.mb, 3u * rs.bytes);
     bulk_g2s(rs.dst_a, rs.src_a, rs.bytes, rs.mb);
     bulk_g2s(rs.dst_c, rs.src_c, rs.bytes, rs.mb);
-    if (rs.with_d) bulk_g2s(rs.dst_d, rs.src_d, rs.bytes, rs.mb);
+    bulk_g2s(rs.dst_d, rs.src_d, rs.bytes, rs.mb);
   }
   mbar_wait(rs.mb, (par >> rs.pbit) & 1u, status);
   par ^= 1u << rs.pbit;
@@ -489,7 +502,7 @@ __device__ __forceinline__ void group_refine(const RagParams& p, const RagSys& s
   const long lo = sy.off & ~3L, hi = (sy.off + n + 3) & ~3L;
   const int pad = (int)(sy.off - lo);
   const Restage rs{mb, pbit, sa - pad, sc - pad, sd - pad, p.a + lo, p.c + lo, p.d + lo,
-                   (uint32_t)(4 * (hi - lo)), true};
+                   (uint32_t)(4 * (hi - lo))};
   EmitX<MODE> first{xs, true};
   group_solve(n, gt, bar, gtid, sa, sb, sc, sd, R, X, F0, first);
   for (int sw = 0; sw < p.sweeps; ++sw) {
@@ -512,170 +525,198 @@ __device__ __forceinline__ void group_refine(const RagParams& p, const RagSys& s
                 reinterpret_cast<unsigned long long*>(red + 2 * kRagWarps));
 }
 
-// Right-hand side of the one-correction modes' correction solve: row i's
-// residual d - (T x0)_i for the FP32 solution x0 (held in the ring's b
-// words), rows of a chunk in order, x0_{i-1} and x0_i carried.
-template <int M>
-struct RhsResidual1 {
-  static constexpr bool kPairs = M == kRefineDF;
-  const float* x0w;
-  int n;
-  mutable float xm, x0;
-  __device__ __forceinline__ float at(int i) const { return i >= 0 && i < n ? x0w[i] : 0.f; }
-  __device__ __forceinline__ void start(int i) const {
-    xm = at(i - 1);
-    x0 = at(i);
-  }
-  __device__ __forceinline__ float operator()(int i, float a, float b, float c, float d) const {
-    const float xp = at(i + 1);
-    a = i > 0 ? a : 0.f;
-    c = i < n - 1 ? c : 0.f;
-    float r;
-    if constexpr (M == kRefineFP64) {
-      double v = fma(-f2d_exact(b), f2d_exact(x0), f2d_exact(d));
-      v = fma(-f2d_exact(a), f2d_exact(xm), v);
-      v = fma(-f2d_exact(c), f2d_exact(xp), v);
-      r = (float)v;
-    } else {
-      r = f_residual(a, b, c, d, xm, x0, xp);
-    }
-    xm = x0;
-    x0 = xp;
-    return r;
-  }
-  // Rows i and i + 1, both interior rows of a chunk (so 0 < i + 1 and
-  // i + 2 < n: only row i's a can lie outside the system), in paired
-  // instructions: residual_parts2 is residual_parts component by component.
-  __device__ __forceinline__ float2 pair(int i, float a0, float b0, float c0, float d0, float a1, float b1, float c1,
-                                         float d1) const {
-    const float x1 = x0w[i + 1], x2 = x0w[i + 2];
-    float2 s, t;
-    residual_parts2(make_float2(i > 0 ? a0 : 0.f, a1), make_float2(b0, b1), make_float2(c0, c1),
-                    make_float2(d0, d1), make_float2(xm, x0), make_float2(x0, x1), make_float2(x1, x2), s, t);
-    xm = x1;
-    x0 = x2;
-    return __fadd2_rn(s, t);
+// A pass of the one-correction modes over a staged system's rows, V
+// consecutive ones a thread and step (rows aligned to V in the arrays, in the
+// ring and in x alike): the original a, b, c, d come from global memory (L2,
+// the first step's before the group's barrier, each further step's a step
+// ahead), x from the ring.  The double-float form takes its rows two at a time
+// in paired FP32 instructions, the same operations as the scalar form component
+// by component; steps away from the system's ends skip the bounds checks.
+//   FINAL = false: r = d - T x0 (x0 in xw), times 1 / pivot in place of it (ew),
+//                  and a and c times 1 / pivot over a and c (aw, cw): what the
+//                  correction's solve from the factors takes.
+//   FINAL = true:  x = x0 + e (e in ew), written as FP64; the group's
+//                  ||d - T x|| / ||d|| folded into the CTA's maximum.
+// With single-word accesses (22 a pair of rows, 11 now, 6 with V = 4) and the
+// sum split and reassembled on the integer units the two passes took 870 us of
+// a 1700 us batch (100000 systems of 32 to 8192 rows); 1588 us so then.  Loading the
+// first step's rows before the separators are solved: 1617 us (registers).
+template <int V>
+struct alignas(4 * V) RowWords {
+  float v[V];
+};
+template <int V>
+struct RowGroup {  // V rows' coefficients
+  RowWords<V> a, b, c, d;
+  __device__ __forceinline__ void load(const RagParams& p, long lo, int g) {
+    using W = RowWords<V>;
+    a = reinterpret_cast<const W*>(p.a + lo)[g];
+    b = reinterpret_cast<const W*>(p.b + lo)[g];
+    c = reinterpret_cast<const W*>(p.c + lo)[g];
+    d = reinterpret_cast<const W*>(p.d + lo)[g];
   }
 };
-
-// The last pass of the one-correction modes: x = x0 + e (x0 in the ring's b
-// words xw, e in its d words ew), its residual d - T x, the group's
-// ||d - T x|| / ||d|| folded into the CTA's maximum, and x written as FP64.
-// Rows i = gtid + q gt; the original a, b, c, d come from global memory (L2,
-// coalesced across the group), each thread keeping the loads of its next
-// kAhead rows in flight.  The double-float form takes its rows two at a time
-// (i and i + gt) in paired FP32 instructions, the same operations as the
-// scalar form component by component.
-template <int M>
-__device__ __forceinline__ void refine1_final(const RagParams& p, const RagSys& sy, int gt, int bar, int gtid,
-                                              const float* xw, const float* ew, double* red) {
+template <int M, bool FINAL, int V>
+__device__ __forceinline__ void refine1_pass(const RagParams& p, const RagSys& sy, int gt, int bar, int gtid,
+                                             const float* xw, float* ew, float* aw, float* cw, double* red) {
+  using W = RowWords<V>;
   const int n = sy.n;
-  const float* ga = p.a + sy.off;
-  const float* gb = p.b + sy.off;
-  const float* gc = p.c + sy.off;
-  const float* gd = p.d + sy.off;
+  const int pad = (int)(sy.off & (V - 1));
   double* xo = p.x64 + sy.off;
-  constexpr int kAhead = 4;  // two pairs
-  float na[kAhead], nb[kAhead], nc[kAhead], nd[kAhead];
-#pragma unroll
-  for (int q = 0; q < kAhead; ++q) {
-    const int j = gtid + q * gt;
-    const bool in = j < n;
-    na[q] = in ? ga[j] : 0.f;
-    nb[q] = in ? gb[j] : 0.f;
-    nc[q] = in ? gc[j] : 0.f;
-    nd[q] = in ? gd[j] : 0.f;
-  }
+  const bool vec = (reinterpret_cast<uintptr_t>(p.x64) & 15) == 0;
+  const int groups = (n + pad + V - 1) / V;
+  RowGroup<V> next{};
+  if (gtid < groups) next.load(p, sy.off - pad, gtid);
+  gsync(bar, gt);  // the group's solution is in the ring
   float2 rr = make_float2(0.f, 0.f), dd = make_float2(0.f, 0.f);
-  const auto out = [&](int i, float h0, float e0) {
-    float l;
-    const float h = two_sum(h0, e0, l);
-    xo[i] = df_to_double(h, l);
-  };
-  for (int i0 = gtid; i0 < n; i0 += kAhead * gt) {
+  // the rows from i0 on; INNER: all of them in 1 .. n - 2
+  const auto rows = [&](auto inner, int i0, W a, W b, W c, W d) {
+    constexpr bool INNER = decltype(inner)::value;
+    // words of rows i0 - 1 .. i0 + V (zero outside the system)
+    const auto words = [&](const float* w, float (&x)[V + 2]) {
+      if (INNER) {
+        x[0] = w[i0 - 1];
+        const W m = *reinterpret_cast<const W*>(w + i0);
 #pragma unroll
-    for (int q = 0; q < kAhead; q += 2) {
-      const int i = i0 + q * gt, j = i + gt;  // j > 0
-      if (i >= n) break;
-      const bool jin = j < n;
-      float2 a = make_float2(na[q], na[q + 1]), b = make_float2(nb[q], nb[q + 1]);
-      float2 c = make_float2(nc[q], nc[q + 1]), d = make_float2(nd[q], nd[q + 1]);
+        for (int q = 0; q < V; ++q) x[q + 1] = m.v[q];
+        x[V + 1] = w[i0 + V];
+      } else {
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int f = i + (u + kAhead) * gt;
-        if (f < n) {
-          na[q + u] = ga[f];
-          nb[q + u] = gb[f];
-          nc[q + u] = gc[f];
-          nd[q + u] = gd[f];
+        for (int q = 0; q < V + 2; ++q) {
+          const int i = i0 - 1 + q;
+          x[q] = i >= 0 && i < n ? w[i] : 0.f;
         }
       }
-      if (i == 0) a.x = 0.f;
-      if (i == n - 1) c.x = 0.f;
-      if (j >= n - 1) c.y = 0.f;
-      // x words of rows i - 1, i, i + 1 and j - 1, j, j + 1 (zero outside the system)
-      const float2 xmh = make_float2(i > 0 ? xw[i - 1] : 0.f, jin ? xw[j - 1] : 0.f);
-      const float2 xml = make_float2(i > 0 ? ew[i - 1] : 0.f, jin ? ew[j - 1] : 0.f);
-      const float2 x0h = make_float2(xw[i], jin ? xw[j] : 0.f);
-      const float2 x0l = make_float2(ew[i], jin ? ew[j] : 0.f);
-      const float2 xph = make_float2(i + 1 < n ? xw[i + 1] : 0.f, j + 1 < n ? xw[j + 1] : 0.f);
-      const float2 xpl = make_float2(i + 1 < n ? ew[i + 1] : 0.f, j + 1 < n ? ew[j + 1] : 0.f);
-      float2 r;
-      if constexpr (M == kRefineFP64) {
-        const auto x64 = [](float h0, float e0) {
-          float l;
-          const float h = two_sum(h0, e0, l);
-          return df_to_double(h, l);
-        };
-        const auto res = [&](float a1, float b1, float c1, float d1, double m1, double z1, double p1) {
-          double v = fma(-f2d_exact(b1), z1, f2d_exact(d1));
-          v = fma(-f2d_exact(a1), m1, v);
-          v = fma(-f2d_exact(c1), p1, v);
-          return (float)v;
-        };
-        r.x = res(a.x, b.x, c.x, d.x, x64(xmh.x, xml.x), x64(x0h.x, x0l.x), x64(xph.x, xpl.x));
-        r.y = jin ? res(a.y, b.y, c.y, d.y, x64(xmh.y, xml.y), x64(x0h.y, x0l.y), x64(xph.y, xpl.y)) : 0.f;
-      } else {
-        r = df_residual2(a, b, c, d, xmh, xml, x0h, x0l, xph, xpl);
+    };
+    if (!INNER) {
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        const int i = i0 + q;
+        const bool in = i >= 0 && i < n;
+        if (!in || i == 0) a.v[q] = 0.f;
+        if (!in || i == n - 1) c.v[q] = 0.f;
+        if (!in) b.v[q] = d.v[q] = 0.f;
       }
-      if (!jin) {  // no row j: its prefetch registers may hold an earlier row
-        r.y = 0.f;
-        d.y = 0.f;
-      }
-      rr = __ffma2_rn(r, r, rr);
-      dd = __ffma2_rn(d, d, dd);
-      out(i, x0h.x, x0l.x);
-      if (jin) out(j, x0h.y, x0l.y);
     }
+    float x[V + 2], e[V + 2] = {}, r[V];
+    words(xw, x);
+    if (FINAL) words(ew, e);
+    if constexpr (M == kRefineFP64) {
+      double xd[V + 2];
+#pragma unroll
+      for (int q = 0; q < V + 2; ++q) xd[q] = FINAL ? f_sum_to_double(x[q], e[q]) : f2d_exact(x[q]);
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        double v = fma(-f2d_exact(b.v[q]), xd[q + 1], f2d_exact(d.v[q]));
+        v = fma(-f2d_exact(a.v[q]), xd[q], v);
+        v = fma(-f2d_exact(c.v[q]), xd[q + 2], v);
+        r[q] = (float)v;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < V; q += 2) {
+        const auto two = [q](const float* w) { return make_float2(w[q], w[q + 1]); };
+        float2 r2;
+        if (FINAL) {
+          r2 = df_residual2(two(a.v), two(b.v), two(c.v), two(d.v), two(x), two(e), two(x + 1), two(e + 1),
+                            two(x + 2), two(e + 2));
+        } else {
+          float2 s, t;
+          residual_parts2(two(a.v), two(b.v), two(c.v), two(d.v), two(x), two(x + 1), two(x + 2), s, t);
+          r2 = __fadd2_rn(s, t);
+        }
+        r[q] = r2.x;
+        r[q + 1] = r2.y;
+      }
+    }
+    if constexpr (FINAL) {
+#pragma unroll
+      for (int q = 0; q < V; q += 2) {
+        const float2 r2 = make_float2(r[q], r[q + 1]), d2 = make_float2(d.v[q], d.v[q + 1]);
+        rr = __ffma2_rn(r2, r2, rr);
+        dd = __ffma2_rn(d2, d2, dd);
+        const double v0 = f_sum_to_double(x[q + 1], e[q + 1]), v1 = f_sum_to_double(x[q + 2], e[q + 2]);
+        const int i = i0 + q;
+        if (INNER && vec) {
+          *reinterpret_cast<double2*>(xo + i) = make_double2(v0, v1);
+        } else {
+          if (INNER || (i >= 0 && i < n)) xo[i] = v0;
+          if (INNER || (i + 1 >= 0 && i + 1 < n)) xo[i + 1] = v1;
+        }
+      }
+    } else {
+      // (words of the ring outside the system, in its first and last group,
+      // belong to it and are not read again)
+      W* w = reinterpret_cast<W*>(ew + i0);
+      W g = *w;
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        a.v[q] *= g.v[q];
+        c.v[q] *= g.v[q];
+        g.v[q] *= r[q];
+      }
+      *w = g;
+      *reinterpret_cast<W*>(aw + i0) = a;
+      *reinterpret_cast<W*>(cw + i0) = c;
+    }
+  };
+  for (int g = gtid; g < groups; g += gt) {
+    const RowGroup<V> at = next;
+    if (g + gt < groups) next.load(p, sy.off - pad, g + gt);
+    // (one branch a warp)
+    const int i0 = g * V - pad, w0 = i0 - (gtid & 31) * V;
+    if (w0 > 0 && w0 + 32 * V < n) rows(std::true_type{}, i0, at.a, at.b, at.c, at.d);
+    else rows(std::false_type{}, i0, at.a, at.b, at.c, at.d);
   }
-  group_rel_max(rr.x + rr.y, dd.x + dd.y, gt, bar, gtid, reinterpret_cast<float*>(red),
-                reinterpret_cast<unsigned long long*>(red + 2 * kRagWarps));
+  if constexpr (FINAL)
+    group_rel_max(rr.x + rr.y, dd.x + dd.y, gt, bar, gtid, reinterpret_cast<float*>(red),
+                  reinterpret_cast<unsigned long long*>(red + 2 * kRagWarps));
 }
 
 // One-correction refinement (sweeps == 1) of one staged system by its solve
-// group, in the ring's four arrays: the FP32 solve leaves x0 in the b words;
-// a, c, d are re-staged; the correction solve (b read from global memory,
-// each row's residual formed as the row is eliminated) leaves its solution e
-// in the d words; a and c are re-staged once more, and the final pass forms
-// d - T (x0 + e) with b and d from global memory, folds its norm into the
-// CTA's maximum and writes x0 + e as FP64.  M: kRefineDF or kRefineFP64.
-template <int M>
+// group, in the ring's four arrays.  The system is eliminated once
+// (chunk_factor_smem): its factors stay in the ring and x0 goes to the d words;
+// the pass over the originals puts the residual, divided by the pivots, over
+// the pivots' reciprocals (the b words), where the correction is solved with
+// the factors and stays; a second pass writes x0 + e as FP64 and the residual's
+// norm.  100000 systems of 32 to 8192 rows:
+// 1793 us with two eliminations and the originals staged again in between,
+// 1630 us so.  M: kRefineDF or kRefineFP64.
+// (Four rows a thread and step in the passes; two for a warp's small systems, and
+// in the kernel with the BIG path, which has no registers left: 400 systems of
+// 9000 to 24000 rows 616 us with four, 605 with two.)
+template <int M, int V>
 __device__ __forceinline__ void group_refine1(const RagParams& p, const RagSys& sy, int gt, int bar, int gtid,
                                               float* sa, float* sb, float* sc, float* sd, float* R, float* X,
-                                              float* F0, double* red, uint64_t* mb, int pbit, uint32_t& par) {
-  const int n = sy.n;
-  const long lo = sy.off & ~3L, hi = (sy.off + n + 3) & ~3L;
-  const int pad = (int)(sy.off - lo);
-  const uint32_t bytes = (uint32_t)(4 * (hi - lo));
-  const float* gb = p.b + sy.off;
-  EmitStore to_b{sb};
-  group_solve(n, gt, bar, gtid, sa, sb, sc, sd, R, X, F0, to_b);
-  restage(Restage{mb, pbit, sa - pad, sc - pad, sd - pad, p.a + lo, p.c + lo, p.d + lo, bytes, true}, par, gt, bar,
-          gtid, p.status);
-  EmitOverD to_d;
-  group_solve(n, gt, bar, gtid, sa, gb, sc, sd, R, X, F0, to_d, RhsResidual1<M>{sb, n});
-  if (gt == 32) __syncwarp();  // the e words are complete (group_solve ends on the barrier otherwise)
-  refine1_final<M>(p, sy, gt, bar, gtid, sb, sd, red);
+                                              float* F0, double* red) {
+  const int kk = odd_ceil_dev((sy.n + gt - 1) / gt);
+  const int r0 = gtid * kk;
+  int kr = sy.n - r0;
+  kr = kr < 0 ? 0 : (kr > kk ? kk : kr);
+  Row<float> sr;   // the thread's separator
+  float ea, ec;    // its row's couplings
+  float sj, sl;
+  {
+    ChunkSummary<float> cs;
+    chunk_factor_smem(cs, kr, gtid == 0, r0 + kr == sy.n && kr > 0, sa + r0, sb + r0, sc + r0, sd + r0);
+    const float f[3] = {cs.fD, cs.fC, cs.fA};
+    float nf[3];
+    group_next(f, nf, gt, bar, gtid, F0);
+    sr = separator_row_s<float>(cs, nf[0], nf[1], nf[2]);
+    ea = cs.sep.a;
+    ec = cs.sep.c;
+  }
+  group_separators(sr, gt, bar, gtid, R, X, sj, sl);
+  chunk_between_smem(kr, sj, sl, sa + r0, sb + r0, sc + r0, sd + r0);
+  refine1_pass<M, false, V>(p, sy, gt, bar, gtid, sd, sb, sa, sc, red);
+  gsync(bar, gt);  // the right-hand side is complete
+  float fD[1], nD[1], lD;
+  chunk_rhs_smem(kr, sa + r0, sc + r0, sb + r0, fD[0], lD);
+  group_next(fD, nD, gt, bar, gtid, F0);
+  sr.d = (kr > 0 ? sb[r0 + kr - 1] : 0.f) - ea * lD - ec * nD[0];
+  group_separators(sr, gt, bar, gtid, R, X, sj, sl);
+  chunk_between_scaled_smem(kr, sj, sl, sa + r0, sc + r0, sb + r0);
+  refine1_pass<M, true, V>(p, sy, gt, bar, gtid, sd, sb, sa, sc, red);
 }
 
 // A BIG system (rows read straight from global memory, right-hand side rhs):
@@ -961,8 +1002,8 @@ __global__ void __launch_bounds__(kRagThreads + 32, 1) ragged_kernel(RagParams p
           group_solve_plain(sy.n, kRagThreads, 1, tid, A + base, B + base, C + base, D + base, Rsh, Xsh, F0,
                             p.x + sy.off);
         } else if constexpr (one_correction(MODE)) {
-          group_refine1<residual_mode(MODE)>(p, sy, kRagThreads, 1, tid, A + base, B + base, C + base, D + base,
-                                             Rsh, Xsh, F0, red, &rbar[kRagWarps + kTeams], kRagWarps + kTeams, rpar);
+          group_refine1<residual_mode(MODE), BIG ? 2 : 4>(p, sy, kRagThreads, 1, tid, A + base, B + base, C + base, D + base,
+                                             Rsh, Xsh, F0, red);
         } else {
           group_refine<MODE>(p, sy, kRagThreads, 1, tid, A + base, B + base, C + base, D + base, XH + base, XL + base,
                              Rsh, Xsh, F0, red, &rbar[kRagWarps + kTeams], kRagWarps + kTeams, rpar);
@@ -1006,8 +1047,8 @@ __global__ void __launch_bounds__(kRagThreads + 32, 1) ragged_kernel(RagParams p
             group_solve_plain(sy.n, 32, 0, lane, A + base, B + base, C + base, D + base, nullptr, nullptr, nullptr,
                               p.x + sy.off);
           } else if constexpr (one_correction(MODE)) {
-            group_refine1<residual_mode(MODE)>(p, sy, 32, 0, lane, A + base, B + base, C + base, D + base, nullptr,
-                                               nullptr, nullptr, red, &rbar[warp], warp, rpar);
+            group_refine1<residual_mode(MODE), 2>(p, sy, 32, 0, lane, A + base, B + base, C + base, D + base, nullptr,
+                                               nullptr, nullptr, red);
           } else {
             group_refine<MODE>(p, sy, 32, 0, lane, A + base, B + base, C + base, D + base, XH + base, XL + base,
                                nullptr, nullptr, nullptr, red, &rbar[warp], warp, rpar);
@@ -1020,8 +1061,8 @@ __global__ void __launch_bounds__(kRagThreads + 32, 1) ragged_kernel(RagParams p
           group_solve_plain(sy.n, kTeamThreads, tbar, ttid, A + base, B + base, C + base, D + base, tR, tX, tF,
                             p.x + sy.off);
         } else if constexpr (one_correction(MODE)) {
-          group_refine1<residual_mode(MODE)>(p, sy, kTeamThreads, tbar, ttid, A + base, B + base, C + base, D + base,
-                                             tR, tX, tF, red, &rbar[kRagWarps + team], kRagWarps + team, rpar);
+          group_refine1<residual_mode(MODE), BIG ? 2 : 4>(p, sy, kTeamThreads, tbar, ttid, A + base, B + base, C + base, D + base,
+                                             tR, tX, tF, red);
         } else {
           group_refine<MODE>(p, sy, kTeamThreads, tbar, ttid, A + base, B + base, C + base, D + base, XH + base,
                              XL + base, tR, tX, tF, red, &rbar[kRagWarps + team], kRagWarps + team, rpar);
@@ -1110,7 +1151,7 @@ tridi_status plan_create(const long* offsets, int num_systems, bool refine, void
   plan->sys.reserve(num_systems);
   for (int s : order) plan->sys.push_back(RagSys{offsets[s], (int)(offsets[s + 1] - offsets[s]), 0});
   // threads per system: the autotuned choice for the system's size bucket,
-  // else 32 up to 480 rows, 160 up to 4800, the whole CTA above
+  // else by the limits above
   auto threads_for = [refine](long n) {
     int t = refine ? tuned(TRIDI_AUTOTUNE_RAGGED_REFINE_THREADS, ilog2(n)) : 0;
     if (t == 0) t = tuned(TRIDI_AUTOTUNE_RAGGED_THREADS, ilog2(n));
