@@ -109,8 +109,10 @@ __global__ void __launch_bounds__(256) large_assemble_kernel(LargeParams p) {
 
 template <class T, int L>
 __global__ void __launch_bounds__(128) large_back_kernel(LargeParams p) {
-  const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= p.P * p.m) return;
+  // last rows first: what the reduce pass read last is still in L2 (FP32 12000 x
+  // 1000 134 -> 129 us, FP64 20000 x 500 367 -> 360 us)
+  const long gid = p.P * p.m - 1 - ((long)blockIdx.x * blockDim.x + threadIdx.x);
+  if (gid < 0) return;
   long s, j;
   large_coords(p, gid, &s, &j);
   const long r0 = j * L;
