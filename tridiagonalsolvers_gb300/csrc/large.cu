@@ -26,6 +26,7 @@
 // once (4 B), plus ~20/L B of interface data.  No reference kernel
 // corresponds; the reference's large-system path is pcrGauss's global-memory
 // PCR steps (pcrGauss_kernel.cu:272-386).  Oracle: the gold Thomas solver.
+#include "columns.cuh"
 #include "large_tma.h"
 #include "partition.cuh"
 #include "runtime.h"
@@ -179,8 +180,56 @@ __global__ void __launch_bounds__(32) thomas_interleaved_kernel(const T* __restr
   }
 }
 
+// Systems that a CTA holds whole (columns.cuh), staged by plain loads: any
+// number of them, FP32 or FP64.
+template <class T>
+__global__ void __launch_bounds__(32 * kColWarps<T>, 1)
+    columns_plain_kernel(const T* __restrict__ a, const T* __restrict__ b, const T* __restrict__ c,
+                         const T* __restrict__ d, T* __restrict__ x, int n, long m) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr int F = kColArray<T>, B = 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long s = (long)blockIdx.x * kColSystems + lane;
+  const bool live = s < m;
+  T* base = reinterpret_cast<T*>(smem + kColHead);
+  T* st = base + (size_t)warp * 4 * F + lane;
+#pragma unroll
+  for (int i0 = 0; i0 < kColChunk; i0 += B) {
+    T r[4][B];
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      const int i = warp * kColChunk + i0 + q;
+      const bool in = live && i < n;
+      const long o = (long)i * m + s;
+      r[0][q] = in ? a[o] : T(0);
+      r[1][q] = in ? b[o] : T(1);
+      r[2][q] = in ? c[o] : T(0);
+      r[3][q] = in ? d[o] : T(0);
+    }
+#pragma unroll
+    for (int q = 0; q < B; ++q)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) st[v * F + (i0 + q) * kColSystems] = r[v][q];
+  }
+  columns_solve<T>(base, n, m, true, live, x + s);
+}
+
 namespace {
 constexpr int kChunk = 16;
+
+template <class T>
+tridi_status large_columns_plain(const T* a, const T* b, const T* c, const T* d, T* x, long n, long m,
+                                 cudaStream_t st) {
+  const DeviceInfo* dev = current_device();
+  if (!dev) return TRIDI_ERROR_CUDA;
+  const int warps = (int)((n + kColChunk - 1) / kColChunk);
+  const size_t smem = columns_smem<T>(warps);
+  int per_sm = 0;
+  const cudaError_t e = resident_blocks(columns_plain_kernel<T>, 32 * warps, smem, *dev, &per_sm);
+  if (e != cudaSuccess) return cuda_status(e);
+  return cuda_status(launch_kernel(columns_plain_kernel<T>, (unsigned)((m + kColSystems - 1) / kColSystems), 32 * warps,
+                                   smem, st, a, b, c, d, x, (int)n, m));
+}
 
 long round64(long v) { return (v + 63) & ~63L; }
 
@@ -227,6 +276,15 @@ tridi_status large_solve(const T* a, const T* b, const T* c, const T* d, T* x, l
     thomas_interleaved_kernel<T><<<(unsigned)((m + 31) / 32), 32, 0, st>>>(a, b, c, d, x, (int)n, m);
     return cuda_status(cudaGetLastError());
   }
+  // interleaved FP32 with m a multiple of 32: the TMA-tiled passes (large_tma.cu),
+  // or one kernel where a CTA holds 32 systems whole
+  bool tma = false;
+  if constexpr (sizeof(T) == 4) tma = large_fusable(a, b, c, d, n, m);
+  if (!fused && n <= kColRows<T>) {
+    if constexpr (sizeof(T) == 4)
+      if (tma) return large_columns(a, b, c, d, n, m, x, st);
+    return large_columns_plain<T>(a, b, c, d, x, n, m, st);
+  }
   LargeParams p{};
   p.a = a; p.b = b; p.c = c; p.d = d; p.x = x;
   p.n = n; p.m = m;
@@ -239,9 +297,6 @@ tridi_status large_solve(const T* a, const T* b, const T* c, const T* d, T* x, l
   void* inner = w + (size_t)14 * p.PMp * sizeof(T) + 256;
   const size_t inner_bytes = ws_bytes - ((size_t)14 * p.PMp * sizeof(T) + 256);
   const unsigned blocks = (unsigned)((PM + 255) / 256);
-  // interleaved FP32 with m a multiple of 32: the TMA-tiled passes (large_tma.cu)
-  bool tma = false;
-  if constexpr (sizeof(T) == 4) tma = large_fusable(a, b, c, d, n, m);
   if (fused && fused->mode == kBackSecond) {
     // the separator system is there: the first sweep's matrix, and its right-
     // hand side from that sweep's back pass

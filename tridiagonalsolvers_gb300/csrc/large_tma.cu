@@ -26,6 +26,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "columns.cuh"
 #include "dfloat.cuh"
 #include "large_tma.h"
 #include "partition.cuh"
@@ -568,6 +569,32 @@ __global__ void __launch_bounds__(256) large_tile_boundary_kernel(LtParams p) {
                 b[(kBndLast + 2) * p.BS], nD, nC, nA);
 }
 
+// Systems that a CTA holds whole (columns.cuh), staged by tensor copies, each
+// warp's rows on a barrier of its own.
+__global__ void __launch_bounds__(32 * kColWarps<float>, 1)
+    large_columns_kernel(LtParams p, const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb,
+                         const __grid_constant__ CUtensorMap mc, const __grid_constant__ CUtensorMap md) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr int F = kColArray<float>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int s0 = (int)blockIdx.x * kColSystems;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem) + warp;
+  float* base = reinterpret_cast<float*>(smem + kColHead);
+  if (lane == 0) {
+    float* st = base + (size_t)warp * 4 * F;
+    mbar_init(bar, 1);
+    mbar_fence_init();
+    mbar_arrive_expect_tx(bar, 4u * F * sizeof(float));
+    tma_load_2d(st + 0 * F, &ma, s0, warp * kColChunk, bar);
+    tma_load_2d(st + 1 * F, &mb, s0, warp * kColChunk, bar);
+    tma_load_2d(st + 2 * F, &mc, s0, warp * kColChunk, bar);
+    tma_load_2d(st + 3 * F, &md, s0, warp * kColChunk, bar);
+  }
+  __syncwarp();
+  const bool ok = mbar_wait(bar, 0, p.status);
+  columns_solve<float>(base, (int)p.n, p.m, ok, true, static_cast<float*>(p.x) + s0 + lane);
+}
+
 bool make_map(CUtensorMap* map, const float* base, long n, long m, int rows) {
   return make_tensor_map_2d(map, base, (uint64_t)m, (uint64_t)n, (uint64_t)m * sizeof(float), kTileCols, rows, false);
 }
@@ -668,6 +695,25 @@ tridi_status large_tma_back(const float* a, const float* b, const float* c, cons
     else large_tile_edge_kernel<kBackSecond><<<grid, 256, 0, st>>>(p, a, b, c, f->d);
   }
   return cuda_status(cudaGetLastError());
+}
+
+tridi_status large_columns(const float* a, const float* b, const float* c, const float* d, long n, long m, float* x,
+                           cudaStream_t st) {
+  const DeviceInfo* dev = current_device();
+  if (!dev) return TRIDI_ERROR_CUDA;
+  const int warps = (int)((n + kColChunk - 1) / kColChunk);
+  const size_t smem = columns_smem<float>(warps);
+  if (n > kColRows<float> || (size_t)dev->max_smem_optin < smem) return TRIDI_ERROR_UNSUPPORTED_SIZE;
+  CUtensorMap tm[4];
+  const tridi_status ts = make_maps(tm, a, b, c, d, n, m, kColChunk);
+  if (ts != TRIDI_SUCCESS) return ts;
+  LtParams p = tile_params(n, m, dev);
+  p.x = x;
+  int per_sm = 0;
+  const cudaError_t e = resident_blocks(large_columns_kernel, 32 * warps, smem, *dev, &per_sm);
+  if (e != cudaSuccess) return cuda_status(e);
+  return cuda_status(launch_kernel(large_columns_kernel, (unsigned)p.col_tiles, 32 * warps, smem, st, p, tm[0], tm[1],
+                                   tm[2], tm[3]));
 }
 
 }  // namespace tridi

@@ -32,6 +32,9 @@ tridi_status large_tma_reduce(const float* a, const float* b, const float* c, co
 tridi_status large_tma_back(const float* a, const float* b, const float* c, const float* d, long n, long m,
                             const float* sol, float* x, const LargeFused* f, float* red_d, float* bnd,
                             cudaStream_t st);
+// Systems of at most kColRows<float> rows (large_tma_ok() holds) in one kernel.
+tridi_status large_columns(const float* a, const float* b, const float* c, const float* d, long n, long m, float* x,
+                           cudaStream_t st);
 
 // Whether a solve of this interleaved system takes the TMA passes (and so can
 // be fused with a sweep).

@@ -146,7 +146,8 @@ struct RhsStaged {
 // back substitution reads them again instead of holding 3k registers.
 // Row i's right-hand side is rhs(i, a_i, b_i, c_i, d_i) of its staged values
 // (a correction solve forms its residual there, as the row is eliminated).
-template <class T, class Rhs = RhsStaged>
+// RS: words from one row to the next.
+template <class T, int RS = 1, class Rhs = RhsStaged>
 __device__ __forceinline__ void chunk_eliminate_smem(ChunkSummary<T>& cs, int k, bool first, bool last,
                                                      T* __restrict__ sa, const T* __restrict__ sb,
                                                      T* __restrict__ sc, T* __restrict__ sd,
@@ -156,21 +157,21 @@ __device__ __forceinline__ void chunk_eliminate_smem(ChunkSummary<T>& cs, int k,
     const T a = (i == 0 && first) ? T(0) : a0;
     T cn, an, dn;
     tdiv3(c0, i == 0 ? a : -a * aprev, r - a * dprev, b0 - a * cprev, cn, an, dn);
-    sa[i] = an; sc[i] = cn; sd[i] = dn;
+    sa[i * RS] = an; sc[i * RS] = cn; sd[i * RS] = dn;
     cprev = cn; aprev = an; dprev = dn;
   };
 #pragma unroll 4
   for (int i = 0; i < k - 1; ++i) {
-    const T a0 = sa[i], b0 = sb[i], c0 = sc[i];
-    step(i, a0, b0, c0, rhs(i, a0, b0, c0, sd[i]));
+    const T a0 = sa[i * RS], b0 = sb[i * RS], c0 = sc[i * RS];
+    step(i, a0, b0, c0, rhs(i, a0, b0, c0, sd[i * RS]));
   }
   T D = T(0), C = T(-1), A = T(0);
 #pragma unroll 4
   for (int i = k - 2; i >= 0; --i) {
-    const T c = sc[i];
-    D = sd[i] - c * D;
+    const T c = sc[i * RS];
+    D = sd[i * RS] - c * D;
     C = -c * C;
-    A = sa[i] - c * A;
+    A = sa[i * RS] - c * A;
   }
   cs.fD = D; cs.fC = C; cs.fA = A;
   if (k >= 2) {
@@ -179,8 +180,8 @@ __device__ __forceinline__ void chunk_eliminate_smem(ChunkSummary<T>& cs, int k,
     cs.lD = T(0); cs.lC = T(0); cs.lA = T(-1);
   }
   if (k >= 1) {
-    const T a0 = sa[k - 1], b0 = sb[k - 1], c0 = sc[k - 1];
-    cs.sep = Row<T>{a0, b0, c0, rhs(k - 1, a0, b0, c0, sd[k - 1])};
+    const T a0 = sa[(k - 1) * RS], b0 = sb[(k - 1) * RS], c0 = sc[(k - 1) * RS];
+    cs.sep = Row<T>{a0, b0, c0, rhs(k - 1, a0, b0, c0, sd[(k - 1) * RS])};
     if (k == 1 && first) cs.sep.a = T(0);
     if (last) cs.sep.c = T(0);
   } else {
@@ -197,14 +198,14 @@ __device__ __forceinline__ Row<T> separator_row_s(const ChunkSummary<T>& cs, T n
 // Back substitution of a chunk eliminated by chunk_eliminate_smem: emit(i, x_i)
 // for every row i < k of the chunk, last row first.
 // (emit writes to arrays other than sa, sc, sd.)
-template <class T, class Emit>
+template <class T, int RS = 1, class Emit>
 __device__ __forceinline__ void chunk_back_smem(int k, T sj, T sl, const T* __restrict__ sa,
                                                 const T* __restrict__ sc, const T* __restrict__ sd, Emit& emit) {
   if (k >= 1) emit(k - 1, sj);
   T xn = sj;
 #pragma unroll 4
   for (int i = k - 2; i >= 0; --i) {
-    xn = sd[i] - sc[i] * xn - sa[i] * sl;
+    xn = sd[i * RS] - sc[i * RS] * xn - sa[i * RS] * sl;
     emit(i, xn);
   }
 }
