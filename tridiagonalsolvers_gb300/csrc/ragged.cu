@@ -601,10 +601,15 @@ __device__ __forceinline__ void refine1_pass(const RagParams& p, const RagSys& s
     float x[V + 2], e[V + 2] = {}, r[V];
     words(xw, x);
     if (FINAL) words(ew, e);
+    [[maybe_unused]] double xd[V + 2];  // x in FP64 (FINAL or FP64 residuals)
     if constexpr (M == kRefineFP64) {
-      double xd[V + 2];
+      // (the FP64 pipe bounds this form: x0 + e on the integer units)
 #pragma unroll
-      for (int q = 0; q < V + 2; ++q) xd[q] = FINAL ? f_sum_to_double(x[q], e[q]) : f2d_exact(x[q]);
+      for (int q = 0; q < V + 2; ++q) {
+        float l;
+        const float h = two_sum(x[q], e[q], l);
+        xd[q] = FINAL ? df_to_double(h, l) : f2d_exact(x[q]);
+      }
 #pragma unroll
       for (int q = 0; q < V; ++q) {
         double v = fma(-f2d_exact(b.v[q]), xd[q + 1], f2d_exact(d.v[q]));
@@ -630,12 +635,16 @@ __device__ __forceinline__ void refine1_pass(const RagParams& p, const RagSys& s
       }
     }
     if constexpr (FINAL) {
+      if constexpr (M != kRefineFP64) {
+#pragma unroll
+        for (int q = 1; q <= V; ++q) xd[q] = f_sum_to_double(x[q], e[q]);
+      }
 #pragma unroll
       for (int q = 0; q < V; q += 2) {
         const float2 r2 = make_float2(r[q], r[q + 1]), d2 = make_float2(d.v[q], d.v[q + 1]);
         rr = __ffma2_rn(r2, r2, rr);
         dd = __ffma2_rn(d2, d2, dd);
-        const double v0 = f_sum_to_double(x[q + 1], e[q + 1]), v1 = f_sum_to_double(x[q + 2], e[q + 2]);
+        const double v0 = xd[q + 1], v1 = xd[q + 2];
         const int i = i0 + q;
         if (INNER && vec) {
           *reinterpret_cast<double2*>(xo + i) = make_double2(v0, v1);
