@@ -477,9 +477,11 @@ tridi_status cr64_solve(const double* a, const double* b, const double* c, const
   if (!dev) return TRIDI_ERROR_CUDA;
   // Rows a thread.  CR: 8 (three levels in registers, 128 registers, 16 warps
   // an SM): 16384 x 1024 371 us, 441 us with 4.  PCR on several rows a thread
-  // (stride below 8): 4 rows, 24 warps: 4096 x 1024 pcr 548 us, 647 us with 8;
-  // crpcr rest 256 152 and 161 us.  2048 rows need 8 for 256 threads.
-  const int K = n <= 8 ? n / 2 : (stride >= 8 || n == 2048) ? 8 : 4;
+  // (stride below 8): 4 rows, 24 warps: crpcr rest 256 of 4096 x 1024 152 and
+  // 161 us.  PCR alone up to 512 unknowns: 2 rows (20000 x 512 1081 us, 1139 with
+  // 4; one system of 128 11 and 21 us; 1024 unknowns would need 512 threads:
+  // 2500 systems 427 us, 332 with 4).  2048 rows need 8 for 256 threads.
+  const int K = n <= 8 ? n / 2 : stride == 1 && n <= 512 ? 2 : (stride >= 8 || n == 2048) ? 8 : 4;
   Cr64Params p{};
   p.a = a; p.b = b; p.c = c; p.d = d; p.x = x;
   p.n = n; p.m = m; p.tps = n / K; p.rest = n / stride;
