@@ -165,9 +165,9 @@ tridi_status tridi_pcr_thomas_f64(const double *a, const double *b, const double
 
 /* ---- GB300 additions (no counterpart kernel in the reference) ----------- */
 /* Generic batched solve, any size 1 <= n <= 8704 (FP64: <= 4608), not only
-   powers of two:
-   partition method (per-lane Thomas-like chunk elimination in registers,
-   PCR on the separator system, back substitution).  Uniform n, contiguous.
+   powers of two: the partition method (per-lane Thomas-like chunk elimination
+   in registers, PCR on the separator system, back substitution); in FP64
+   cyclic reduction on the n rows.  Uniform n, contiguous.
    Checked against the gold Thomas solver of tridiagonal_gold.h:26-44. */
 tridi_status tridi_solve_f32(const float *a, const float *b, const float *c, const float *d, float *x, int n,
                              int num_systems, tridi_stream_t stream);
@@ -175,8 +175,9 @@ tridi_status tridi_solve_f64(const double *a, const double *b, const double *c, 
                              int n, int num_systems, tridi_stream_t stream);
 
 /* Large systems, any n, in either layout: TRIDI_LAYOUT_CONTIGUOUS (s*n + i) or TRIDI_LAYOUT_INTERLEAVED
-   (i*num_systems + s, system-fastest).  Three kernels on `stream`: chunk
-   elimination, separator-system solve, chunk back substitution.  Needs a
+   (i*num_systems + s, system-fastest).  On `stream`: chunk elimination,
+   separator-system solve, chunk back substitution; one kernel where a CTA
+   holds whole systems (8704 rows contiguous, 448 interleaved in FP32).  Needs a
    device workspace of tridi_large_workspace_bytes() bytes (no allocation
    inside the call). */
 #define TRIDI_LAYOUT_CONTIGUOUS 0
@@ -288,14 +289,17 @@ tridi_status tridi_server_destroy(void *server);
 /* Mixed-precision iterative refinement: FP32 a, b, c, d in, FP64 x out.
    Only the residual r = d - T x and the accumulation x += e run in extended
    precision (TRIDI_TUNE_RESIDUAL: double-float by default, native FP64);
-   every solve (the first and each correction) is an FP32 solve: CR-PCR for
-   power-of-two contiguous n <= 4096, the partition solver for other
-   contiguous n <= 8704, the large-system solver otherwise.  Stops when
+   every solve (the first and each correction) is an FP32 solve: the partition
+   method for contiguous n <= 8704 at tolerances up to 1e-8, there with its
+   residuals in one kernel (CR-PCR or the partition solver with separate
+   residual passes at looser tolerances and in native FP64), the large-system
+   solver otherwise.  Stops when
    max over systems of ||d - T x|| / ||d|| <= tol, or after max_sweeps
    corrections (then returns TRIDI_ERROR_NOT_CONVERGED; x is still the best
    iterate).  *sweeps receives the number of corrections applied and
    *rel_residual the final maximum relative residual (either may be NULL).
-   Synchronises `stream` once per sweep to read the residual. */
+   Synchronises `stream` once per residual read back (once a call where the
+   first correction suffices in one kernel). */
 size_t tridi_refine_workspace_bytes(long n, long num_systems, int layout);
 tridi_status tridi_refine_f32(const float *a, const float *b, const float *c, const float *d, double *x, long n,
                               long num_systems, int layout, double tol, int max_sweeps, void *workspace,

@@ -2,14 +2,14 @@
 // two passes over blocks of 128 * K consecutive rows, staged and solved as in
 // strip.cuh, around one small system of block rows.
 //
-//   1. rows_reduce_kernel: a CTA per block; what is left of it is its last
+//   1. rows_kernel<BACK = 0>: a CTA per block; what is left of it is its last
 //      row (coupled to the last row of the block before and to the first row
 //      of the block after) and the form of its first row: seven values.  Each
 //      lane's and each warp's separator is kept as a function of its
 //      neighbours, three values each.
 //   2. rows_sep_kernel: a warp per system assembles and solves the system of
 //      its ceil(n / 128 K) block rows.
-//   3. rows_back_kernel: the separators from what pass 1 kept, then every
+//   3. rows_kernel<BACK = 1>: the separators from what pass 1 kept, then every
 //      lane's chunk again, between two known rows: a plain Thomas sweep.
 // The blocks of pass 3 run in reverse, so that the rows pass 1 read last are
 // still in L2 (129 MB).  What bounds it is HBM in FP32 (two reads of the
