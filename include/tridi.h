@@ -68,7 +68,7 @@ tridi_status tridi_device_status(unsigned *bits, int reset);
    algorithm. */
 #define TRIDI_TUNE_STAGES 1     /* cp.async.bulk pipeline stages per CTA (1..8) */
 #define TRIDI_TUNE_CRPCR_REST 2 /* switch level of the CR-PCR correction solves */
-#define TRIDI_TUNE_CR_ROWS 3    /* rows per thread of the CR/PCR/CR-PCR kernels (2, 4, 8, 16) */
+#define TRIDI_TUNE_CR_ROWS 3    /* rows per thread of the FP32 hybrid CR/PCR/CR-PCR kernels (2, 4, 8, 16) */
 #define TRIDI_TUNE_RESIDUAL 4   /* arithmetic of the refinements' residual and update: */
 #define TRIDI_RESIDUAL_DF 1     /*   double-float (pairs of FP32, 48-bit significand; the default) */
 #define TRIDI_RESIDUAL_FP64 2   /*   native FP64 */
@@ -84,10 +84,11 @@ tridi_status tridi_device_status(unsigned *bits, int reset);
                                      shared-memory kernel always */
 #define TRIDI_TUNE_DROPIN_CHUNK 9 /* host-pointer launchers: KiB of each coefficient array per pipelined chunk
                                      (0 = 8192 from pinned memory, 65536 from pageable memory) */
-#define TRIDI_TUNE_PCR_KERNEL 10  /* FP32 PCR on 64..1024 unknowns: 0/1 = the two-phase kernel (rows transposed
+#define TRIDI_TUNE_PCR_KERNEL 10  /* FP32 PCR on 64..4096 unknowns: 0/1 = the two-phase kernels (rows transposed
                                      once between the register phases) with paired FP32 instructions,
-                                     3 = the same on single rows, 2 = the hybrid warp kernel (the same
-                                     algorithm throughout; results differ in rounding only) */
+                                     3 = the same on single rows (up to 1024), 2 = the hybrid kernels, of CR
+                                     and CR-PCR too (the same algorithm throughout; results differ in
+                                     rounding only) */
 #define TRIDI_TUNE_DROPIN_MAPPED 11 /* host-pointer launchers (cr, pcr, crpcr, crNBC, crNBC32, crpcrNBC):
                                      0/1 = arrays that are pinned and mapped into the device's address
                                      space, or ordinary pageable arrays on a device that reaches them
