@@ -1,0 +1,63 @@
+"""Right-hand sides of any size: the refinements' convergence tests sum squares
+of residuals, which leave FP32's range long before the residuals do (a
+residual of 1e-10 of a right-hand side of 1e-16 squares to zero).  Scaling d
+by a power of two scales every FP32 intermediate without rounding, up to
+subnormal numbers, so the sweeps and the relative residual of the scaled
+system are those of the unscaled one: the residual to 1e-4 (its FP32 sums, and
+the last bits of residuals near 2^-130), x to the 1e-10 of every refinement."""
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+
+import tridiagonalsolvers_gb300 as tg
+from oracle import gold
+from tridiagonalsolvers_gb300 import workloads
+
+pytestmark = pytest.mark.gpu
+
+SCALES = (-66, -53, 60, 100)  # 2^-66 = 1.4e-20, 2^100 = 1.3e30
+
+
+def _refine(cuda, arrs, n, m, layout, tol=1e-10, max_sweeps=10, residual=1):
+    """(status, x, sweeps, rel) of tridi_refine_f32."""
+    import torch
+
+    from tridiagonalsolvers_gb300 import _lib
+
+    L = _lib.lib()
+    t = [torch.from_numpy(np.ascontiguousarray(v).ravel()).to(cuda) for v in arrs]
+    x = torch.full((n * m,), float("nan"), dtype=torch.float64, device=cuda)
+    wsb = L.tridi_refine_workspace_bytes(n, m, layout)
+    ws = torch.empty(wsb, dtype=torch.uint8, device=cuda)
+    sweeps, rel = ctypes.c_int(-1), ctypes.c_double(-1.0)
+    prev = L.tridi_get_tunable(4)  # TRIDI_TUNE_RESIDUAL
+    assert L.tridi_set_tunable(4, residual) == 0
+    try:
+        st = L.tridi_refine_f32(*(v.data_ptr() for v in t), x.data_ptr(), n, m, layout, tol, max_sweeps, ws.data_ptr(),
+                                wsb, torch.cuda.current_stream().cuda_stream, ctypes.byref(sweeps), ctypes.byref(rel))
+    finally:
+        L.tridi_set_tunable(4, prev)
+    return st, x.cpu().numpy().reshape(np.shape(arrs[0])), sweeps.value, rel.value
+
+
+def _check(cuda, k, arrs, n, m, layout, **kw):
+    st1, x1, sweeps1, rel1 = _refine(cuda, arrs, n, m, layout, **kw)
+    assert st1 == 0 and 0 < rel1 <= kw.get("tol", 1e-10)
+    f = np.float64(2.0) ** k
+    scaled = (*arrs[:3], (arrs[3] * f).astype(np.float32))
+    st, x, sweeps, rel = _refine(cuda, scaled, n, m, layout, **kw)
+    assert (st, sweeps) == (0, sweeps1), (st, sweeps, rel, rel1)
+    assert abs(rel - rel1) <= 1e-4 * rel1, (rel, rel1)
+    if sweeps:
+        x64 = gold.solve_f64(*(np.ascontiguousarray(v.T) for v in arrs)).T if layout else gold.solve_f64(*arrs)
+        assert np.abs(x / f - x64).max() <= 1e-10 * np.abs(x64).max()
+
+
+@pytest.mark.parametrize("k", SCALES)
+@pytest.mark.parametrize("n,m", [(5, 40), (64, 333), (500, 7), (1000, 20), (2200, 6), (8704, 3)])
+def test_contiguous_one_kernel(cuda, n, m, k):
+    """csrc/refine_rows.cu, a warp's and a CTA's systems."""
+    _check(cuda, k, workloads.dominant(m, n, seed=n), n, m, 0, max_sweeps=1)

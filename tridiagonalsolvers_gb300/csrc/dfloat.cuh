@@ -63,6 +63,52 @@ __device__ __forceinline__ double f_sum_to_double(float x, float y) {
   return __longlong_as_double((long long)df_add_bits(x, y));
 }
 
+// Sums of squares of FP32 values over the whole of FP32's range (a residual of
+// 1e-26 squares to zero in FP32, a value of 1e20 to infinity): the squares of
+// the values times 2^58, taken while that sum is below 2^114, and those of the
+// values times 2^-58.  Where the second takes over it is 2^-118, so what
+// subnormal squares lose there is below 2^-31 of it.
+constexpr int kSquareScale = 116;
+struct SquareSum {  // one sum
+  float2 s = {0.f, 0.f};
+  __device__ __forceinline__ void add(float v) {
+    const float2 u = __fmul2_rn(make_float2(v, v), make_float2(0x1p58f, 0x1p-58f));
+    s = __ffma2_rn(u, u, s);
+  }
+};
+struct SquareSums {  // two sums at once
+  float2 up = {0.f, 0.f}, dn = {0.f, 0.f};
+  __device__ __forceinline__ void add(float2 v) {
+    const float2 u = __fmul2_rn(v, make_float2(0x1p58f, 0x1p58f)), w = __fmul2_rn(v, make_float2(0x1p-58f, 0x1p-58f));
+    up = __ffma2_rn(u, u, up);
+    dn = __ffma2_rn(w, w, dn);
+  }
+  __device__ __forceinline__ SquareSum first() const { return SquareSum{make_float2(up.x, dn.x)}; }
+  __device__ __forceinline__ SquareSum second() const { return SquareSum{make_float2(up.y, dn.y)}; }
+};
+// The sum in FP64, off the FP64 pipe (infinite or NaN where it is).
+__device__ __forceinline__ double square_value(const SquareSum& q) {
+  const bool small = q.s.x < 0x1p114f;
+  const double v = f2d_exact(small ? q.s.x : q.s.y);
+  const unsigned long long u = div64_bits(v);
+  if (u == 0 || u >= 0x7ff0000000000000ull) return v;
+  return __longlong_as_double((long long)(u + ((unsigned long long)(small ? -kSquareScale : kSquareScale) << 52)));
+}
+// The sum over the `width` lanes of a group, in its first lane.
+__device__ __forceinline__ SquareSum square_total(SquareSum q, int width) {
+  for (int o = width / 2; o > 0; o >>= 1)
+    q.s = __fadd2_rn(q.s, make_float2(__shfl_down_sync(kFull, q.s.x, o, width), __shfl_down_sync(kFull, q.s.y, o, width)));
+  return q;
+}
+
+// ||r||^2 / ||d||^2 from the two sums: ||r||^2 itself for a zero right-hand
+// side, NaN where ||d||^2 is infinite or NaN.
+__device__ __forceinline__ double square_ratio(double rr, double dd) {
+  const unsigned long long u = div64_bits(dd);
+  if (u >= 0x7ff0000000000000ull) return __longlong_as_double(0x7ff8000000000000ll);
+  return u == 0 ? rr : tdiv(rr, dd);
+}
+
 // Knuth's TwoSum: s + e == a + b exactly.
 __device__ __forceinline__ float two_sum(float a, float b, float& e) {
   const float s = __fadd_rn(a, b);

@@ -13,9 +13,13 @@
 // 200000 x 64: 4798 -> 224 us; 16000 x 1000: 829 -> 314 us; 2000 x 8000: 590 ->
 // 368 us (a call, with its two host round trips before and one now).
 //
-// Per-system sums of squares are double-float sums of FP32 squares; their
-// quotient is formed on the integer units (div64.cuh), so the FP64 pipe takes
-// no part.
+// Sums of squares are FP32, in two scales (SquareSum: d and r of any size);
+// their quotient is formed on the integer units (div64.cuh), so the FP64 pipe
+// takes no part.  The first residual's are added over the lanes before the
+// second elimination, which needs the registers.  (One scale and double-float
+// sums over the lanes: 16000 x 1000 283 us, 269 us so; 2000 x 8000 351 and 334;
+// 20000 x 500, whose 17 rows a lane spill, 229 and 240.  Two scales and FP64 sums
+// over the lanes: 299, 367 and 232 us.)
 #include "dfloat.cuh"
 #include "refine_rows.h"
 #include "runtime.h"
@@ -38,27 +42,10 @@ struct RowsRefine {
   unsigned* status;
 };
 
-__device__ __forceinline__ float2 df_sum(float2 a, float2 b) {
-  float e, lo;
-  const float s = two_sum(a.x, b.x, e);
-  const float hi = fast_two_sum(s, __fadd_rn(e, __fadd_rn(a.y, b.y)), lo);
-  return make_float2(hi, lo);
-}
-// Sum over the `width` lanes of a group, in its first lane.
-__device__ __forceinline__ float2 group_sum(float2 v, int width) {
-  for (int o = width / 2; o > 0; o >>= 1) {
-    const float2 w = make_float2(__shfl_down_sync(kFull, v.x, o, width), __shfl_down_sync(kFull, v.y, o, width));
-    v = df_sum(v, w);
-  }
-  return v;
-}
-
 // The larger of `best` and the bits of ||r||^2 / ||d||^2 (a non-negative
 // double: integer order; a NaN's bits lie above every number's).
-__device__ __forceinline__ unsigned long long max_rel2(unsigned long long best, float2 rr, float2 dd) {
-  const double den = dd.x > 0.f ? df_to_double(dd.x, dd.y) : 1.0;
-  const double q = tdiv(df_to_double(rr.x, rr.y), den);
-  const unsigned long long u = div64_bits(q) & 0x7fffffffffffffffull;
+__device__ __forceinline__ unsigned long long max_rel2(unsigned long long best, const SquareSum& rr, double dd) {
+  const unsigned long long u = div64_bits(square_ratio(square_value(rr), dd)) & 0x7fffffffffffffffull;
   return u > best ? u : best;
 }
 // A warp's maxima into the kernel's, once at its end.
@@ -82,8 +69,7 @@ struct Rows {
 // the sums of r^2 and d^2.  above / below: x of the rows around the chunk.
 template <int K>
 __device__ __forceinline__ void first_residual(const Rows& w, const float (&x)[K], float above, float below,
-                                               float (&r)[K], float& rs, float& ds) {
-  rs = ds = 0.f;
+                                               float (&r)[K], SquareSums& rd) {
 #pragma unroll
   for (int i = 0; i < K; ++i) {
     r[i] = 0.f;
@@ -93,17 +79,16 @@ __device__ __forceinline__ void first_residual(const Rows& w, const float (&x)[K
       const float d = w.d[i];
       const float xp = end ? below : x[i + 1 < K ? i + 1 : i];
       r[i] = f_residual(a, w.b[i], c, d, i > 0 ? x[i > 0 ? i - 1 : 0] : above, x[i], xp);
-      rs = fmaf(r[i], r[i], rs);
-      ds = fmaf(d, d, ds);
+      rd.add(make_float2(r[i], d));
     }
   }
 }
 
 // The same for x = hi + lo, the sum of r^2 only.
 template <int K>
-__device__ __forceinline__ float second_residual(const Rows& w, const float (&hi)[K], const float (&lo)[K],
-                                                 float2 above, float2 below) {
-  float rs = 0.f;
+__device__ __forceinline__ SquareSum second_residual(const Rows& w, const float (&hi)[K], const float (&lo)[K],
+                                                     float2 above, float2 below) {
+  SquareSum rs;
   float2 xm = above;
 #pragma unroll
   for (int i = 0; i < K; ++i) {
@@ -113,7 +98,7 @@ __device__ __forceinline__ float second_residual(const Rows& w, const float (&hi
       const float2 xi = make_float2(hi[i], lo[i]);
       const float2 xp = end ? below : make_float2(hi[i + 1 < K ? i + 1 : i], lo[i + 1 < K ? i + 1 : i]);
       const float r = df_residual(a, w.b[i], c, w.d[i], xm, xi, xp);
-      rs = fmaf(r, r, rs);
+      rs.add(r);
       xm = xi;
     }
   }
@@ -174,26 +159,26 @@ __global__ void __launch_bounds__(128, MINB) refine_warp_kernel(RowsRefine p) {
       above = t == 0 ? 0.f : up;
       chunk_back<float, K>(ch, k, sj, above, x);
     };
-    float x[K], r[K], lo[K], above, rs0, ds;
+    float x[K], r[K], lo[K], above;
+    SquareSums rd;
     solve([&](Chunk<float, K>& ch) { chunk_eliminate<float, K>(ch, k, w.first, w.last, w.a, w.b, w.c, w.d); }, x, above);
     const float below = __shfl_down_sync(kFull, x[0], 1, lps);
-    first_residual<K>(w, x, above, w.last ? 0.f : below, r, rs0, ds);
+    first_residual<K>(w, x, above, w.last ? 0.f : below, r, rd);
+    const double dd = square_value(square_total(rd.second(), lps));
+    const SquareSum r0 = square_total(rd.first(), lps);
+    if (t == 0 && in) best0 = max_rel2(best0, r0, dd);
     float e[K], unused;
     solve([&](Chunk<float, K>& ch) { chunk_eliminate_rhs<float, K>(ch, k, w.first, w.last, w.a, w.b, w.c, r); }, e, unused);
     add_correction<K>(x, e, lo);
     const float2 dn = make_float2(__shfl_down_sync(kFull, x[0], 1, lps), __shfl_down_sync(kFull, lo[0], 1, lps));
     const float2 up = make_float2(__shfl_up_sync(kFull, x[K - 1], 1, lps), __shfl_up_sync(kFull, lo[K - 1], 1, lps));
     const float2 zero = make_float2(0.f, 0.f);
-    const float rs1 = second_residual<K>(w, x, lo, t == 0 ? zero : up, w.last ? zero : dn);
+    const SquareSum rs1 = second_residual<K>(w, x, lo, t == 0 ? zero : up, w.last ? zero : dn);
     fence_proxy_async_smem();
     __syncwarp();
     if (bulk && lane == 0 && tile + step < tiles) strip_issue(strip(tile + step), p.in, buf, p.cap, bar);
-    const float2 r0 = group_sum(make_float2(rs0, 0.f), lps), r1 = group_sum(make_float2(rs1, 0.f), lps);
-    const float2 dd = group_sum(make_float2(ds, 0.f), lps);
-    if (t == 0 && in) {
-      best0 = max_rel2(best0, r0, dd);
-      best1 = max_rel2(best1, r1, dd);
-    }
+    const SquareSum r1 = square_total(rs1, lps);
+    if (t == 0 && in) best1 = max_rel2(best1, r1, dd);
     // (x of the tile at the place its first element has in a 16-byte group)
     const long xlo = s.e0 & ~1L;
     const int xoff = (int)(s.e0 - xlo) + g * n + t * K;
@@ -216,7 +201,7 @@ __global__ void __launch_bounds__(MAXT, MINB) refine_cta_kernel(RowsRefine p) {
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
   float* scratch = reinterpret_cast<float*>(smem + 16);         // 7 W
   float2* edge = reinterpret_cast<float2*>(smem + 512);         // per warp: x of its first and of its last row
-  float2* sums = edge + 2 * 16;                                 // per warp: r0, r1, d
+  SquareSum* sums = reinterpret_cast<SquareSum*>(edge + 2 * 16);  // per warp: r0, r1, d
   float* buf = reinterpret_cast<float*>(smem + 1280);
   double* xs = reinterpret_cast<double*>(buf + 4 * p.cap);
   const bool bulk = p.bulk != 0;
@@ -251,7 +236,8 @@ __global__ void __launch_bounds__(MAXT, MINB) refine_cta_kernel(RowsRefine p) {
       if (lane == 31) below = warp + 1 < W ? edge[2 * (warp + 1 < W ? warp + 1 : warp)] : make_float2(0.f, 0.f);
       if (last) below = make_float2(0.f, 0.f);
     };
-    float x[K], r[K], lo[K], e[K], rs0, ds;
+    float x[K], r[K], lo[K], e[K];
+    SquareSums rd;
     float2 above, below;
     {
       Chunk<float, K> ch;
@@ -260,7 +246,14 @@ __global__ void __launch_bounds__(MAXT, MINB) refine_cta_kernel(RowsRefine p) {
       block_back<float, K>(f, ch, k, W, 0.0f, tdiv(f.last.d, f.last.b), x);
     }
     around(make_float2(x[0], 0.f), make_float2(x[K - 1], 0.f), above, below);
-    first_residual<K>(w, x, above.x, below.x, r, rs0, ds);
+    first_residual<K>(w, x, above.x, below.x, r, rd);
+    {
+      const SquareSum r0 = square_total(rd.first(), 32), dd = square_total(rd.second(), 32);
+      if (lane == 0) {
+        sums[3 * warp] = r0;
+        sums[3 * warp + 2] = dd;
+      }
+    }
     {
       Chunk<float, K> ch;
       chunk_eliminate_rhs<float, K>(ch, k, w.first, last, w.a, w.b, w.c, r);
@@ -269,24 +262,20 @@ __global__ void __launch_bounds__(MAXT, MINB) refine_cta_kernel(RowsRefine p) {
     }
     add_correction<K>(x, e, lo);
     around(make_float2(x[0], lo[0]), make_float2(x[K - 1], lo[K - 1]), above, below);
-    const float rs1 = second_residual<K>(w, x, lo, above, below);
-    const float2 r0 = group_sum(make_float2(rs0, 0.f), 32), r1 = group_sum(make_float2(rs1, 0.f), 32);
-    const float2 dd = group_sum(make_float2(ds, 0.f), 32);
-    if (lane == 0) {
-      sums[3 * warp] = r0;
-      sums[3 * warp + 1] = r1;
-      sums[3 * warp + 2] = dd;
-    }
+    const SquareSum rs1 = second_residual<K>(w, x, lo, above, below);
+    const SquareSum r1 = square_total(rs1, 32);
+    if (lane == 0) sums[3 * warp + 1] = r1;
     fence_proxy_async_smem();
     __syncthreads();  // every row is read
     if (bulk && tid == 0 && sys + gridDim.x < p.m) strip_issue(strip(sys + gridDim.x), p.in, buf, p.cap, bar);
-    if (tid == 32) {
-      float2 v[3] = {sums[0], sums[1], sums[2]};
-      for (int q = 1; q < W; ++q)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) v[j] = df_sum(v[j], sums[3 * q + j]);
-      best0 = max_rel2(best0, v[0], v[2]);
-      best1 = max_rel2(best1, v[1], v[2]);
+    if (warp == 1) {
+      const auto total = [&](int q) { return square_total(lane < W ? sums[3 * lane + q] : SquareSum{}, 16); };
+      const SquareSum r0 = total(0), r1 = total(1), dd = total(2);
+      if (lane == 0) {
+        const double d2 = square_value(dd);
+        best0 = max_rel2(best0, r0, d2);
+        best1 = max_rel2(best1, r1, d2);
+      }
     }
     const long xlo = s.e0 & ~1L;
     const int xoff = (int)(s.e0 - xlo) + tid * K;
