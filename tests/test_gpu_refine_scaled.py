@@ -61,3 +61,10 @@ def _check(cuda, k, arrs, n, m, layout, **kw):
 def test_contiguous_one_kernel(cuda, n, m, k):
     """csrc/refine_rows.cu, a warp's and a CTA's systems."""
     _check(cuda, k, workloads.dominant(m, n, seed=n), n, m, 0, max_sweeps=1)
+
+
+@pytest.mark.parametrize("k", SCALES)
+@pytest.mark.parametrize("n,m", [(40, 64), (129, 32), (5000, 32)])
+def test_interleaved_back_pass(cuda, n, m, k):
+    """csrc/large_tma.cu: the residuals of its back pass and of its tiles' last rows."""
+    _check(cuda, k, workloads.dominant(m, n, seed=n, layout=1), n, m, 1, max_sweeps=1)

@@ -238,15 +238,17 @@ __global__ void __launch_bounds__(32 * (kLtWarps + 1), 1)
 // pointers, when kBackFirst left the correction's elimination to a reduce pass
 // of 172 us; a back pass and a pass over the system each 330 and 560 us.  With
 // two rows' residuals in paired FP32 instructions 319 and 530 us (the pairs'
-// registers).
+// registers).  The norms' squares are summed in two scales (SquareSum): 1024 x
+// 65536 refined 963 us with one, 971 us so.
 constexpr int kBackGroups = 3, kBackWarps = 4;           // groups a CTA, warps a group
 constexpr int kBackRows = kBackWarps * kLtChunk;         // 64
 constexpr int kBackFloats = kBackRows * kTileCols;       // per array of a tile
 constexpr int kBackThreads = 32 * kBackGroups * kBackWarps;
 constexpr size_t kBackSmem = 128 + (size_t)kBackGroups * 2 * 4 * kBackFloats * sizeof(float);
-// per group, all for two tiles: x of the warps' first rows (hi, lo), the norms' partial sums (r^2, d^2) and fD
-constexpr size_t kBackShare = 2 * 2 * kBackWarps * 32 + 2 * kBackWarps * 32 / 2;
+// per group, all for two tiles: x of the warps' first rows (hi, lo), the norms' partial sums (r^2, d^2 in FP64) and fD
+constexpr size_t kBackShare = 2 * kBackWarps * 32 * (1 + 2) + 2 * kBackWarps * 32 / 2;
 constexpr size_t kBackResidual = kBackGroups * kBackShare * sizeof(float2);
+static_assert(kBackSmem + kBackResidual <= 232448, "back pass: shared memory");
 
 template <int MODE>
 __global__ void __launch_bounds__(kBackThreads, 1)
@@ -259,7 +261,7 @@ __global__ void __launch_bounds__(kBackThreads, 1)
   uint64_t* full = reinterpret_cast<uint64_t*>(smem) + 2 * grp;
   float* ring = reinterpret_cast<float*>(smem + 128) + (size_t)grp * 2 * 4 * kBackFloats;
   float2* exch = reinterpret_cast<float2*>(smem + kBackSmem) + grp * kBackShare;
-  float2* norms = exch + 2 * kBackWarps * 32;
+  double2* norms = reinterpret_cast<double2*>(exch + 2 * kBackWarps * 32);
   float* first_d = reinterpret_cast<float*>(norms + 2 * kBackWarps * 32);
   const int row_tiles = (int)((p.n + kBackRows - 1) / kBackRows);
   const int ntiles = row_tiles * p.col_tiles, step = (int)gridDim.x * kBackGroups;
@@ -315,7 +317,7 @@ __global__ void __launch_bounds__(kBackThreads, 1)
     if (warp != (k & (kBackWarps - 1))) return;
     double rs = 0.0, ds = 0.0;
     for (int w = 0; w < kBackWarps; ++w) {
-      const float2 v = norms[((k & 1) * kBackWarps + w) * 32 + lane];
+      const double2 v = norms[((k & 1) * kBackWarps + w) * 32 + lane];
       rs += v.x;
       ds += v.y;
     }
@@ -425,7 +427,8 @@ __global__ void __launch_bounds__(kBackThreads, 1)
       const bool open = warp == kBackWarps - 1 && r0 + L < p.n;
       const bool end = kr > 0 && r0 + kr == p.n;
       const float2 below = warp + 1 < kBackWarps && !end ? ex[(warp + 1) * 32 + lane] : make_float2(0.f, 0.f);
-      float rs = 0.f, ds = 0.f;
+      SquareSums rd;  // of r and of d (kBackSecond: rs, of r)
+      SquareSum rs;
       [[maybe_unused]] float lD = 0.f;
       float* gx = static_cast<float*>(p.x) + g0;
       double* gx64 = static_cast<double*>(p.x) + g0;
@@ -444,8 +447,8 @@ __global__ void __launch_bounds__(kBackThreads, 1)
                                               : f_residual(a[q], b[q], ci, di, xm.x, xi.x, xp.x);
           if (!(lastrow && open)) {
             if (MODE == kBackFirst) *gr = r;
-            rs = fmaf(r, r, rs);
-            ds = fmaf(di, di, ds);
+            if (MODE == kBackFirst) rd.add(make_float2(r, di));
+            else rs.add(r);
           }
           xm = xi;
           if constexpr (MODE == kBackFirst) {  // r through the elimination, d' in x's place
@@ -462,7 +465,9 @@ __global__ void __launch_bounds__(kBackThreads, 1)
         gx64 = down(gx64, 2 * row_bytes);
         gr = down(gr, row_bytes);
       }
-      norms[((k & 1) * kBackWarps + warp) * 32 + lane] = make_float2(rs, ds);
+      if (MODE == kBackFirst) rs = rd.first();
+      norms[((k & 1) * kBackWarps + warp) * 32 + lane] =
+          make_double2(square_value(rs), MODE == kBackFirst ? square_value(rd.second()) : 0.0);
       if constexpr (MODE == kBackFirst) {
         float fD = 0.f;
 #pragma unroll
@@ -491,9 +496,10 @@ __global__ void __launch_bounds__(kBackThreads, 1)
 }
 
 // v as hi + lo, hi its significand's upper 24 bits and lo the next 24, on the
-// integer units (three FP64 instructions a value bound the kernel below);
-// values outside FP32's normal range take those, out of line: inline, the
-// compiler issued them for every value and the FP64 pipe was 72% busy).
+// integer units (three FP64 instructions a value bound the kernel below), by
+// one rule over FP32's normal range but its top (lo scaled in two steps: its
+// scale alone would leave that range); values outside take those, out of line:
+// inline, the compiler issued them for every value and the FP64 pipe was 72% busy).
 __device__ __noinline__ float2 double_to_pair_slow(unsigned long long bits) {
   const double v = __longlong_as_double((long long)bits);
   const float hi = __double2float_rn(v);
@@ -501,11 +507,11 @@ __device__ __noinline__ float2 double_to_pair_slow(unsigned long long bits) {
 }
 __device__ __forceinline__ float2 double_to_pair(unsigned long long u) {
   const int e = (int)((u >> 52) & 0x7ff) - 1023;  // v = +-1.f * 2^e
-  if (e < -60 || e > 120) return double_to_pair_slow(u);
+  if (e < -126 || e > 119) return double_to_pair_slow(u);
   const unsigned sign = (unsigned)(u >> 32) & 0x80000000u;
   const float hi = __uint_as_float(sign | ((unsigned)(e + 127) << 23) | ((unsigned)(u >> 29) & 0x7fffffu));
-  const float ulp = __uint_as_float(sign | ((unsigned)(e + 127 - 52) << 23));  // 2^(e - 52)
-  return make_float2(hi, (float)((unsigned)u & 0x1fffffffu) * ulp);
+  const float part = __uint_as_float(sign | ((unsigned)(e + 127 + 8) << 23));  // 2^(e - 52 + 60)
+  return make_float2(hi, (float)((unsigned)u & 0x1fffffffu) * 0x1p-60f * part);
 }
 
 // The rows that large_back_tile_kernel leaves open (the last of each tile but
@@ -516,7 +522,7 @@ template <int MODE>
 __global__ void __launch_bounds__(256) large_tile_edge_kernel(LtParams p, const float* __restrict__ a,
                                                               const float* __restrict__ b, const float* __restrict__ c,
                                                               const float* __restrict__ d) {
-  __shared__ float2 part[8][32];
+  __shared__ double2 part[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long sys = (long)(blockIdx.x % p.col_tiles) * kTileCols + lane;
   const long i = ((long)(blockIdx.x / p.col_tiles) * 8 + warp + 1) * kBackRows - 1;
@@ -524,7 +530,7 @@ __global__ void __launch_bounds__(256) large_tile_edge_kernel(LtParams p, const 
     if constexpr (MODE == kBackFirst) return make_float2(static_cast<const float*>(p.x)[o], 0.f);
     return double_to_pair(static_cast<const unsigned long long*>(p.x)[o]);
   };
-  float2 sums = make_float2(0.f, 0.f);
+  double2 sums = make_double2(0.0, 0.0);
   if (i < p.n - 1) {
     const long o = i * p.m + sys;
     const float di = d[o];
@@ -534,18 +540,19 @@ __global__ void __launch_bounds__(256) large_tile_edge_kernel(LtParams p, const 
       const long t = (i / kBackRows) * p.m + sys;
       p.red_d[(i / kLtChunk) * p.m + sys] = r - a[o] * p.bnd[t] - c[o] * p.bnd[p.BS + t + p.m];
     }
-    sums = make_float2(r * r, di * di);
+    const double r64 = f2d_exact(r), d64 = f2d_exact(di);
+    sums = make_double2(r64 * r64, d64 * d64);
   }
   part[warp][lane] = sums;
   __syncthreads();
   if (warp == 0) {
-    float rs = 0.f, ds = 0.f;
+    double rs = 0.0, ds = 0.0;
     for (int w = 0; w < 8; ++w) {
       rs += part[w][lane].x;
       ds += part[w][lane].y;
     }
-    atomicAdd(&p.rr[sys], (double)rs);
-    if (MODE == kBackFirst) atomicAdd(&p.dd[sys], (double)ds);
+    atomicAdd(&p.rr[sys], rs);
+    if (MODE == kBackFirst) atomicAdd(&p.dd[sys], ds);
   }
 }
 
