@@ -68,3 +68,29 @@ def test_contiguous_one_kernel(cuda, n, m, k):
 def test_interleaved_back_pass(cuda, n, m, k):
     """csrc/large_tma.cu: the residuals of its back pass and of its tiles' last rows."""
     _check(cuda, k, workloads.dominant(m, n, seed=n, layout=1), n, m, 1, max_sweeps=1)
+
+
+@pytest.mark.parametrize("k", SCALES)
+@pytest.mark.parametrize("residual", [1, 2])  # TRIDI_RESIDUAL_DF, TRIDI_RESIDUAL_FP64
+@pytest.mark.parametrize("n,m,layout", [(300, 20, 0), (1024, 9, 0), (9001, 4, 0), (700, 31, 1)])
+def test_separate_passes(cuda, n, m, layout, residual, k):
+    """csrc/refine.cu's residual passes: tolerances that the first solution
+    meets, native FP64 residuals, systems longer than a CTA holds, interleaved
+    batches of no multiple of 32."""
+    arrs = workloads.dominant(m, n, seed=n, layout=layout)
+    _check(cuda, k, arrs, n, m, layout, tol=1e-5, residual=residual)
+    _check(cuda, k, arrs, n, m, layout, max_sweeps=1, residual=residual)
+
+
+@pytest.mark.parametrize("layout", [0, 1])
+def test_no_number_is_no_convergence(cuda, layout):
+    """A system whose ||d||^2 is no number is not converged (its absolute
+    residual is no measure), whatever the others are."""
+    n, m = 300, 9
+    for bad in (np.inf, np.nan):
+        arrs = [v.copy() for v in workloads.dominant(m, n, seed=2, layout=layout)]
+        arrs[3] *= np.float32(2.0**-66)
+        arrs[3][4, 5] = bad
+        for tol in (1e-5, 1e-10):
+            st, _, _, rel = _refine(cuda, arrs, n, m, layout, tol=tol, max_sweeps=1)
+            assert st == 6 and np.isnan(rel)

@@ -70,23 +70,22 @@ struct XNext<false> {
   }
   __device__ __forceinline__ static void put(const RefineParams& p, long k, V v) { p.xout[k] = v; }
   __device__ __forceinline__ static V zero() { return 0.0; }
-  // d - T x at row i, and d^2; r in FP64, returned rounded to FP32
+  // d - T x at row i, and d; r in FP64, returned rounded to FP32
   __device__ __forceinline__ static float residual(const RefineParams& p, long i, long k, long stride, V xi,
-                                                   float* dsq) {
-    const double di = (double)p.d[k];
+                                                   float* dk) {
+    *dk = p.d[k];
+    const double di = (double)*dk;
     double r = di - (double)p.b[k] * xi;
     if (i > 0) r -= (double)p.a[k] * get(p, k - stride);
     if (i < p.n - 1) r -= (double)p.c[k] * get(p, k + stride);
-    *dsq = p.d[k] * p.d[k];
     return (float)r;
   }
   // the same from values already loaded (xm / xp: x of the rows above / below)
   __device__ __forceinline__ static float residual_v(long i, long n, float a, float b, float c, float d, V xm, V xi,
-                                                     V xp, float* dsq) {
+                                                     V xp) {
     double r = (double)d - (double)b * xi;
     if (i > 0) r -= (double)a * xm;
     if (i < n - 1) r -= (double)c * xp;
-    *dsq = d * d;
     return (float)r;
   }
 };
@@ -115,16 +114,15 @@ struct XDF {
   }
   __device__ __forceinline__ static V zero() { return make_float2(0.f, 0.f); }
   __device__ __forceinline__ static float residual(const RefineParams& p, long i, long k, long stride, V xi,
-                                                   float* dsq) {
+                                                   float* dk) {
     const V xm = i > 0 ? get(p, k - stride) : zero();
     const V xp = i < p.n - 1 ? get(p, k + stride) : zero();
-    *dsq = p.d[k] * p.d[k];
-    return df_residual(i > 0 ? p.a[k] : 0.f, p.b[k], i < p.n - 1 ? p.c[k] : 0.f, p.d[k], xm, xi, xp);
+    *dk = p.d[k];
+    return df_residual(i > 0 ? p.a[k] : 0.f, p.b[k], i < p.n - 1 ? p.c[k] : 0.f, *dk, xm, xi, xp);
   }
   // the same from values already loaded (xm / xp zero beyond the system's ends)
   __device__ __forceinline__ static float residual_v(long i, long n, float a, float b, float c, float d, V xm, V xi,
-                                                     V xp, float* dsq) {
-    *dsq = d * d;
+                                                     V xp) {
     return df_residual(i > 0 ? a : 0.f, b, i < n - 1 ? c : 0.f, d, xm, xi, xp);
   }
 };
@@ -155,26 +153,25 @@ __global__ void __launch_bounds__(256) refine_df_to_fp64_kernel(const float2* sr
 }
 
 // Contiguous layout: block (system s, chunk q) covers rows [q*R, q*R + R).
-// Per-thread norm partial sums in FP32 (a few rows each), the block's sums
-// in FP64.
+// Per-thread norm partial sums in FP32 (a few rows each, in two scales: r and
+// d of any size), the block's sums in FP64.
 template <class X>
 __global__ void __launch_bounds__(256) refine_contig_kernel(RefineParams p) {
   const long chunks = (p.n + p.rows_per_block - 1) / p.rows_per_block;
   const long s = blockIdx.x / chunks, q = blockIdx.x % chunks;
-  float rsf = 0.f, dsf = 0.f;
+  SquareSums rd;
   const long i0 = q * p.rows_per_block;
   const long i1 = i0 + p.rows_per_block < p.n ? i0 + p.rows_per_block : p.n;
   for (long i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
     const long k = s * p.n + i;
     const typename X::V xi = X::get(p, k);
-    float dsq;
-    const float r = X::residual(p, i, k, 1, xi, &dsq);
+    float dk;
+    const float r = X::residual(p, i, k, 1, xi, &dk);
     X::put(p, k, xi);
     p.r[k] = r;
-    rsf = fmaf(r, r, rsf);
-    dsf += dsq;
+    rd.add(make_float2(r, dk));
   }
-  double rs = rsf, ds = dsf;
+  double rs = square_value(rd.first()), ds = square_value(rd.second());
   __shared__ double red[2][8];
   for (int o = 16; o > 0; o >>= 1) {
     rs += __shfl_down_sync(kFull, rs, o);
@@ -216,7 +213,7 @@ __global__ void __launch_bounds__(256, X::kMinBlocks) refine_inter_kernel(Refine
   const long s = g * 32 + (threadIdx.x & 31);
   const int lr = threadIdx.x >> 5;
   const long m = p.m;
-  float rsf = 0.f, dsf = 0.f;
+  SquareSums rd;
   const long wrows = p.rows_per_block / 8;
   const long i0 = q * p.rows_per_block + lr * wrows;
   const long i1 = i0 + wrows < p.n ? i0 + wrows : p.n;
@@ -239,19 +236,17 @@ __global__ void __launch_bounds__(256, X::kMinBlocks) refine_inter_kernel(Refine
       for (int u = 0; u < kBatch; ++u) {
         if (ib + u < i1) {
           const long k = kb + u * m;
-          float dsq;
-          const float r = X::residual_v(ib + u, p.n, a[u], b[u], c[u], d[u], xm, xi, xn[u], &dsq);
+          const float r = X::residual_v(ib + u, p.n, a[u], b[u], c[u], d[u], xm, xi, xn[u]);
           X::put(p, k, xi);
           p.r[k] = r;
-          rsf = fmaf(r, r, rsf);
-          dsf += dsq;
+          rd.add(make_float2(r, d[u]));
           xm = xi;
           xi = xn[u];
         }
       }
     }
   }
-  const double rs = rsf, ds = dsf;
+  const double rs = square_value(rd.first()), ds = square_value(rd.second());
   __shared__ double red[2][8][32];
   red[0][lr][threadIdx.x & 31] = rs;
   red[1][lr][threadIdx.x & 31] = ds;
@@ -276,9 +271,7 @@ __global__ void __launch_bounds__(256) refine_maxrel_kernel(const double* __rest
                                                             long m, unsigned long long* out) {
   unsigned long long v = 0;
   for (long s = (long)blockIdx.x * 256 + threadIdx.x; s < m; s += (long)gridDim.x * 256) {
-    const double den = dd[s];
-    const double q = tdiv(rr[s], den > 0 ? den : 1.0);
-    const unsigned long long u = div64_bits(q) & 0x7fffffffffffffffull;
+    const unsigned long long u = div64_bits(square_ratio(rr[s], dd[s])) & 0x7fffffffffffffffull;
     v = u > v ? u : v;
   }
   for (int o = 16; o > 0; o >>= 1) {
