@@ -94,3 +94,53 @@ def test_no_number_is_no_convergence(cuda, layout):
         for tol in (1e-5, 1e-10):
             st, _, _, rel = _refine(cuda, arrs, n, m, layout, tol=tol, max_sweeps=1)
             assert st == 6 and np.isnan(rel)
+
+
+@pytest.mark.parametrize("k", SCALES)
+@pytest.mark.parametrize("residual", ["df", "fp64"])
+@pytest.mark.parametrize("sweeps", [1, 2])
+@pytest.mark.parametrize("big", [False, True])
+def test_ragged(cuda, big, sweeps, residual, k):
+    """csrc/ragged.cu: systems of a warp, a team, the CTA and (big) beyond the
+    staging ring; the residual it returns, and x."""
+    import torch
+
+    from tridiagonalsolvers_gb300.ragged import RaggedPlan, RaggedRefiner, padded
+
+    sizes = [1, 2, 33, 480, 481, 1000, 4800, 4801, 8100, 77] * 3 + ([20000] if big else [])
+    a, b, c, d, off = workloads.adi(np.array(sizes), seed=7)
+    total = int(off[-1])
+
+    def solve(rhs):
+        t = []
+        for v in (a, b, c, rhs):
+            u = torch.zeros(padded(total), dtype=torch.float32, device=cuda)
+            u[:total] = torch.from_numpy(v)
+            t.append(u)
+        r = RaggedRefiner(RaggedPlan(off, refine=True), *t, sweeps=sweeps, graph=False, residual=residual)
+        x, rel = r.run()
+        return x.cpu().numpy()[:total], rel
+
+    f = np.float64(2.0) ** k
+    x1, rel1 = solve(d)
+    x, rel = solve((d * f).astype(np.float32))
+    assert 0 < rel1 <= 1e-10 and abs(rel - rel1) <= 1e-4 * rel1, (rel, rel1)
+    assert np.abs(x / f - x1).max() <= 1e-10 * np.abs(x1).max()
+
+
+def test_ragged_no_number(cuda):
+    """One system's infinite right-hand side: the batch's residual is no number."""
+    import torch
+
+    from tridiagonalsolvers_gb300.ragged import RaggedPlan, RaggedRefiner, padded
+
+    a, b, c, d, off = workloads.adi(np.array([30, 700, 5000, 60]), seed=3)
+    total = int(off[-1])
+    for bad in (np.inf, np.nan):
+        d[35] = bad
+        t = []
+        for v in (a, b, c, d):
+            u = torch.zeros(padded(total), dtype=torch.float32, device=cuda)
+            u[:total] = torch.from_numpy(v)
+            t.append(u)
+        assert np.isnan(RaggedRefiner(RaggedPlan(off, refine=True), *t, sweeps=1, graph=False).run()[1])
