@@ -73,11 +73,12 @@ const DeviceInfo* current_device() {
   return &d;
 }
 
-cudaError_t raise_smem_limit(const void* kern, size_t smem, const DeviceInfo& dev) {
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.max_smem_optin) == cudaSuccess)
-    return cudaSuccess;
-  cudaGetLastError();
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+cudaError_t raise_smem_limit(const void* kern, const DeviceInfo& dev) {
+  cudaFuncAttributes at;
+  const cudaError_t e = cudaFuncGetAttributes(&at, kern);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              dev.max_smem_optin - (int)at.sharedSizeBytes);
 }
 
 cudaError_t resident_blocks(const void* kern, int threads, size_t smem, const DeviceInfo& dev, int* per_sm) {
@@ -93,7 +94,7 @@ cudaError_t resident_blocks(const void* kern, int threads, size_t smem, const De
     *per_sm = t.per_sm;
     return cudaSuccess;
   }
-  cudaError_t e = raise_smem_limit(kern, smem, dev);
+  cudaError_t e = raise_smem_limit(kern, dev);
   if (e != cudaSuccess) return e;
   int n = 0;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem)) != cudaSuccess) return e;

@@ -39,24 +39,36 @@ template <class... P>
 cudaError_t resident_blocks(void (*kern)(P...), int threads, size_t smem, const DeviceInfo& dev, int* per_sm) {
   return resident_blocks(reinterpret_cast<const void*>(kern), threads, smem, dev, per_sm);
 }
-// Raises the kernel's dynamic shared-memory limit to the device's (or to
-// `smem`, where it has static shared memory too).
-cudaError_t raise_smem_limit(const void* kern, size_t smem, const DeviceInfo& dev);
+// Raises the kernel's dynamic shared-memory limit to what the device leaves
+// beside its static shared memory.
+cudaError_t raise_smem_limit(const void* kern, const DeviceInfo& dev);
 
-// Launch of a kernel that resident_blocks() has seen.  A device reset drops
-// the raised limit; the launch then fails and is repeated with the limit set.
-template <class... P, class... A>
-cudaError_t launch_kernel(void (*kern)(P...), unsigned grid, int threads, size_t smem, cudaStream_t stream, A... args) {
-  kern<<<grid, threads, smem, stream>>>(args...);
+// A launch with `smem` bytes of dynamic shared memory, judged by its own error:
+// one that the thread had not read is taken first and returned after the
+// launch, as after every other launch here, and is no reason to launch again.
+// A device reset drops a raised limit; the launch then fails and is repeated
+// with the limit set.
+template <class Launch>
+cudaError_t checked_launch(const Launch& launch, const void* kern, size_t smem) {
+  const cudaError_t unread = cudaGetLastError();
+  launch();
   cudaError_t e = cudaGetLastError();
   if (e == cudaErrorInvalidValue && smem > 48 * 1024) {
     const DeviceInfo* dev = current_device();
-    if (!dev || raise_smem_limit(reinterpret_cast<const void*>(kern), smem, *dev) != cudaSuccess) return e;
-    kern<<<grid, threads, smem, stream>>>(args...);
+    if (!dev || raise_smem_limit(kern, *dev) != cudaSuccess) return e;
+    launch();
     e = cudaGetLastError();
   }
-  return e;
+  return e != cudaSuccess ? e : unread;
 }
+
+#ifdef __CUDACC__
+// Launch of a kernel that resident_blocks() has seen.
+template <class... P, class... A>
+cudaError_t launch_kernel(void (*kern)(P...), unsigned grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+  return checked_launch([&] { kern<<<grid, threads, smem, stream>>>(args...); }, reinterpret_cast<const void*>(kern), smem);
+}
+#endif
 
 // Launch-shape tunables (tridi_set_tunable); 0 means "choose automatically".
 int tunable(int key);
