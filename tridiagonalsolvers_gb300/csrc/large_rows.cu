@@ -7,8 +7,9 @@
 //      of the block after) and the form of its first row: seven values.  Each
 //      lane's and each warp's separator is kept as a function of its
 //      neighbours, three values each.
-//   2. rows_sep_kernel: a warp per system assembles and solves the system of
-//      its ceil(n / 128 K) block rows.
+//   2. The system of its ceil(n / 128 K) block rows: rows_sep_kernel, a warp per
+//      system, or for long systems rows_assemble_kernel and the contiguous
+//      solvers again (the any-size solver, beyond its range these passes).
 //   3. rows_kernel<BACK = 1>: the separators from what pass 1 kept, then every
 //      lane's chunk again, between two known rows: a plain Thomas sweep.
 // The blocks of pass 3 run in reverse, so that the rows pass 1 read last are
@@ -21,6 +22,10 @@
 #include "strip.cuh"
 
 namespace tridi {
+
+template <class T>
+tridi_status partition_solve_device(const T* a, const T* b, const T* c, const T* d, T* x, int n, int m,
+                                    tridi_stream_t stream);
 
 namespace {
 
@@ -142,8 +147,22 @@ __global__ void __launch_bounds__(32 * kWarps, MINB) rows_kernel(RowsParams<T> p
   }
 }
 
-// The block rows of one system by one warp: each row's coupling to the next
-// block's first row replaced by that row's form, then the partition method
+// A block row's coupling to the next block's first row replaced by that row's
+// form (f: the row's a; j < NB - 1).
+template <class T>
+__device__ __forceinline__ void join_blocks(T* f, long FS) {
+  const T c = f[2 * FS];
+  f[FS] -= c * f[4 * FS + 1];
+  f[3 * FS] -= c * f[6 * FS + 1];
+  f[2 * FS] = -c * f[5 * FS + 1];
+}
+template <class T>
+__global__ void __launch_bounds__(256) rows_assemble_kernel(RowsParams<T> p) {
+  const long i = (long)blockIdx.x * 256 + threadIdx.x;
+  if (i < p.NB * p.m && i % p.NB < p.NB - 1) join_blocks(p.form + i, p.FS);
+}
+
+// The block rows of one system by one warp: joined, then the partition method
 // with ceil(NB / 32) rows a lane, in place.
 template <class T>
 __global__ void __launch_bounds__(128) rows_sep_kernel(RowsParams<T> p) {
@@ -155,12 +174,7 @@ __global__ void __launch_bounds__(128) rows_sep_kernel(RowsParams<T> p) {
   T* fb = fa + FS;
   T* fc = fa + 2 * FS;
   T* fd = fa + 3 * FS;
-  for (long j = lane; j + 1 < NB; j += 32) {
-    const T c = fc[j];
-    fb[j] -= c * fa[4 * FS + j + 1];
-    fd[j] -= c * fa[6 * FS + j + 1];
-    fc[j] = -c * fa[5 * FS + j + 1];
-  }
+  for (long j = lane; j + 1 < NB; j += 32) join_blocks(fa + j, FS);
   __syncwarp();
   const long kk = (NB + 31) / 32, r0 = lane * kk;
   long k = NB - r0;
@@ -195,14 +209,26 @@ constexpr int kRows = sizeof(T) == 4 ? 17 : 13;  // rows a lane
 
 }  // namespace
 
+// Block rows a system up to which a warp solves them, a serial chain of NB / 32
+// rows from global memory; the two launches of the other way cost 3 to 5 us.
+// Level at 128 block rows (FP32, one system 23.5 us by the warp and 22.9, 64
+// systems 118 and 115; FP64 42.9 and 40.5, 559 and 557), at 64 20.0 and 24.4, at
+// 1024 69 and 28.  One FP32 system of 1e8 rows: 3330 us by the warp, 569 us.
+constexpr long kWarpBlocks = 128;
+
+// Stride of the form arrays: whole 16-byte groups, for the solvers that read them.
+inline long rows_stride(long blocks) { return (blocks + 3) & ~3L; }
+
 // Bytes of workspace: 8 + 3 * 128 + 3 * 4 values a block, at most a quarter of
-// a value a row and one block more; tridi_large_workspace_bytes() asks for
-// 14 / 16 of a value a row.
+// a value a row and one block more, and the same for the block rows where they
+// take these passes; tridi_large_workspace_bytes() asks for 14 / 16 of a value a
+// row.
 template <class T>
 size_t large_rows_bytes(long n, long m) {
   constexpr long B = RowsShape<T, kRows<T>>::B;
-  const long FS = ((n + B - 1) / B) * m;
-  return (size_t)(8 + 3 * 128 + 3 * 4) * FS * sizeof(T);
+  const long NB = (n + B - 1) / B;
+  return (size_t)(8 + 3 * 128 + 3 * 4) * rows_stride(NB * m) * sizeof(T) +
+         (NB > partition_max_rows<T>() ? large_rows_bytes<T>(NB, m) : 0);
 }
 
 template <class T>
@@ -217,7 +243,7 @@ tridi_status large_rows_solve(const T* a, const T* b, const T* c, const T* d, T*
   p.x = x;
   p.n = n; p.m = m; p.status = dev->status;
   p.NB = (n + B - 1) / B;
-  p.FS = p.NB * m;
+  p.FS = rows_stride(p.NB * m);
   p.form = static_cast<T*>(ws);
   p.sep = p.form + 7 * p.FS;
   p.warps = p.sep + p.FS;
@@ -227,8 +253,20 @@ tridi_status large_rows_solve(const T* a, const T* b, const T* c, const T* d, T*
   constexpr int MR = sizeof(T) == 4 ? 5 : 3, MB = sizeof(T) == 4 ? 5 : 3;  // CTAs an SM
   cudaError_t e = launch_rows<T, K, false, MR>(p, *dev, st);
   if (e != cudaSuccess) return cuda_status(e);
-  rows_sep_kernel<T><<<(unsigned)((m + 3) / 4), 128, 0, st>>>(p);
-  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
+  if (p.NB <= kWarpBlocks) {
+    rows_sep_kernel<T><<<(unsigned)((m + 3) / 4), 128, 0, st>>>(p);
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
+  } else {
+    rows_assemble_kernel<T><<<(unsigned)((p.NB * m + 255) / 256), 256, 0, st>>>(p);
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
+    const T* f = p.form;
+    const tridi_status ts =
+        p.NB <= partition_max_rows<T>()
+            ? partition_solve_device<T>(f, f + p.FS, f + 2 * p.FS, f + 3 * p.FS, p.sep, (int)p.NB, (int)m,
+                                        reinterpret_cast<tridi_stream_t>(st))
+            : large_rows_solve<T>(f, f + p.FS, f + 2 * p.FS, f + 3 * p.FS, p.sep, p.NB, m, p.lanes + 3 * 128 * p.FS, st);
+    if (ts != TRIDI_SUCCESS) return ts;
+  }
   return cuda_status(launch_rows<T, K, true, MB>(p, *dev, st));
 }
 
