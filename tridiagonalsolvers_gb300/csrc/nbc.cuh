@@ -7,8 +7,8 @@
 // only helps some levels.  Here every level is conflict-free for the 32
 // banks of the GB300 by construction: each forward level writes the rows it
 // eliminates into a new, dense array (level l+1 holds the odd rows of level
-// l), so at every level thread j touches rows 2j, 2j+1 (one 8- or 16-byte
-// pair load: conflict-free) and 2j+2 (the next lane's pair, by shuffle).
+// l), so at every level thread j touches rows 2j, 2j+1 (one 8-byte pair
+// load: conflict-free) and 2j+2 (the next lane's pair, by shuffle).
 // Back substitution walks the levels in reverse with the same pattern and
 // writes x pairwise; level 0 writes x straight to global memory, coalesced.
 //
@@ -54,24 +54,14 @@ struct Pair {
   T lo, hi;
 };
 
-template <class T>
-__device__ __forceinline__ Pair<T> load_pair(const T* p, int i, bool vec) {
-  if (vec) {
-    if constexpr (sizeof(T) == 4) {
-      const float2 v = *reinterpret_cast<const float2*>(p + i);
-      return {v.x, v.y};
-    } else {
-      const double2 v = *reinterpret_cast<const double2*>(p + i);
-      return {v.x, v.y};
-    }
-  }
-  return {p[i], p[i + 1]};
+__device__ __forceinline__ Pair<float> load_pair(const float* p, int i, bool vec) {
+  if (!vec) return {p[i], p[i + 1]};
+  const float2 v = *reinterpret_cast<const float2*>(p + i);
+  return {v.x, v.y};
 }
-template <class T>
-__device__ __forceinline__ void store_pair(T* p, int i, T lo, T hi, bool vec) {
+__device__ __forceinline__ void store_pair(float* p, int i, float lo, float hi, bool vec) {
   if (vec) {
-    if constexpr (sizeof(T) == 4) *reinterpret_cast<float2*>(p + i) = make_float2(lo, hi);
-    else *reinterpret_cast<double2*>(p + i) = make_double2(lo, hi);
+    *reinterpret_cast<float2*>(p + i) = make_float2(lo, hi);
   } else {
     p[i] = lo;
     p[i + 1] = hi;

@@ -411,25 +411,4 @@ __device__ __forceinline__ void chunk_back_emit(const Chunk<T, K>& ch, int k, T 
   }
 }
 
-// Whole system in one warp: lane l owns rows [l*kk, min(l*kk+kk, n)) of the
-// arrays (sa, sb, sc, sd).  Returns the lane's row count.
-template <class T, int K>
-__device__ __forceinline__ int warp_partition_solve(int n, int kk, const T* sa, const T* sb, const T* sc,
-                                                    const T* sd, T (&x)[K]) {
-  const int lane = threadIdx.x & 31;
-  const int r0 = lane * kk;
-  int k = n - r0;
-  k = k < 0 ? 0 : (k > kk ? kk : k);
-  Chunk<T, K> ch;
-  chunk_eliminate<T, K>(ch, k, lane == 0, r0 + k == n && k > 0, sa + r0, sb + r0, sc + r0, sd + r0);
-  const T nD = __shfl_down_sync(kFull, ch.fD, 1);
-  const T nC = __shfl_down_sync(kFull, ch.fC, 1);
-  const T nA = __shfl_down_sync(kFull, ch.fA, 1);
-  const T s = warp_pcr32<T>(separator_row<T, K>(ch, nD, nC, nA));
-  T sl = __shfl_up_sync(kFull, s, 1);
-  if (lane == 0) sl = T(0);
-  chunk_back<T, K>(ch, k, s, sl, x);
-  return k;
-}
-
 }  // namespace tridi

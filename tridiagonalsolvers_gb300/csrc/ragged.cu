@@ -417,7 +417,6 @@ template <int MODE>
 struct RhsResidual;
 template <>
 struct RhsResidual<kRefineDF> {
-  static constexpr bool kPairs = false;
   XStore<kRefineDF> xs;
   int n;
   mutable float2 xm, x0;
@@ -438,7 +437,6 @@ struct RhsResidual<kRefineDF> {
 };
 template <>
 struct RhsResidual<kRefineFP64> {
-  static constexpr bool kPairs = false;
   XStore<kRefineFP64> xs;
   int n;
   mutable double xm, x0;
