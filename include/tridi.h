@@ -206,8 +206,12 @@ tridi_status tridi_solve_large_f64(const double *a, const double *b, const doubl
         ragged plans created afterwards give systems of that bucket; ADI
         systems.
      TRIDI_AUTOTUNE_CR_ROWS           key n (power of two, 32..4096): rows per
-        thread (4, 8 or 16; threads per system = n / rows) of the FP32
-        cr / pcr / crpcr kernels; diagonally dominant systems, timed on cr.
+        thread (4, 8 or 16; threads per system = n / rows) of the FP32 hybrid
+        cr / pcr / crpcr kernels, timed on them (cr); diagonally dominant
+        systems.  Those kernels run cr and crpcr up to 256 unknowns and, where
+        arrays are not 16-byte aligned or lie in host memory, above too; aligned
+        device arrays of 512 (4096 systems and more), 1024, 2048 and 4096
+        unknowns run register kernels that have no such choice.
      TRIDI_AUTOTUNE_RAGGED_REFINE_THREADS  as TRIDI_AUTOTUNE_RAGGED_THREADS,
         timed on the fused one-correction refinement instead of the plain
         solve, for plans created afterwards by tridi_ragged_plan_create_refine

@@ -8,8 +8,9 @@ in csrc/autotune.cu).  Tunes, on the GPU in use:
   * ragged        -- threads per system (32, 160, 480) per size bucket
                      [2^k, 2^(k+1)) of the ragged work queue, used by plans
                      created afterwards;
-  * cr_rows       -- rows per thread (4, 8, 16) of the FP32 CR / PCR / CR-PCR
-                     kernels per power-of-two n (threads per system = n / rows);
+  * cr_rows       -- rows per thread (4, 8, 16) of the FP32 hybrid CR / PCR /
+                     CR-PCR kernels per power-of-two n (threads per system = n /
+                     rows), timed on those kernels;
   * ragged_refine -- as `ragged`, timed on the fused one-correction refinement,
                      used by plans created afterwards with RaggedPlan(...,
                      refine=True) and by the solve server.

@@ -8,7 +8,7 @@
 //   TRIDI_AUTOTUNE_PCR_THOMAS_SPLIT  PCR/Thomas split (Thomas chains g) per n
 //   TRIDI_AUTOTUNE_RAGGED_THREADS    threads per system per size bucket of the
 //                                    ragged work queue (32, 160 or 480)
-//   TRIDI_AUTOTUNE_CR_ROWS           rows per thread of the FP32 CR / PCR /
+//   TRIDI_AUTOTUNE_CR_ROWS           rows per thread of the FP32 hybrid CR / PCR /
 //                                    CR-PCR kernels per power-of-two n
 //   TRIDI_AUTOTUNE_RAGGED_REFINE_THREADS  threads per system per size bucket
 //                                    of plans for the fused refinement, timed
@@ -25,6 +25,9 @@
 #include "tridi.h"
 
 namespace tridi {
+tridi_status hybrid_rows_solve(const float* a, const float* b, const float* c, const float* d, float* x, int n, int m,
+                               int stride, int rows, tridi_stream_t stream);
+
 namespace {
 
 __device__ __forceinline__ float unit_hash(unsigned long long i, unsigned salt) {
@@ -153,21 +156,19 @@ extern "C" tridi_status tridi_autotune(int table, long key, long sample, tridi_s
     Sample smp;
     tridi_status ts = smp.alloc(m * n, st, 0);
     if (ts != TRIDI_SUCCESS) return ts;
-    const int saved = tuned(table, ilog2(n));
+    // (the hybrid kernels themselves: at some sizes and batches the entry points
+    // take a register kernel instead where the arrays are aligned)
     for (int rows : {4, 8, 16}) {
-      if (n / rows > 256 || n / rows < 2) continue;
-      tridi_set_tuned(table, key, rows);
       float ms = 0.f;
-      ts = time_ms([&]() { return tridi_cr_f32(smp.a, smp.b, smp.c, smp.d, smp.x, n, (int)m, stream); }, st, &ms);
+      ts = time_ms(
+          [&]() { return hybrid_rows_solve(smp.a, smp.b, smp.c, smp.d, smp.x, n, (int)m, n / 2, rows, stream); }, st, &ms);
       if (ts == TRIDI_ERROR_UNSUPPORTED_SIZE) continue;
-      if (ts != TRIDI_SUCCESS) break;
+      if (ts != TRIDI_SUCCESS) return ts;
       if (ms < best_t) {
         best_t = ms;
         best = rows;
       }
     }
-    tridi_set_tuned(table, key, saved);
-    if (ts != TRIDI_SUCCESS && ts != TRIDI_ERROR_UNSUPPORTED_SIZE) return ts;
   } else if (table == TRIDI_AUTOTUNE_RAGGED_THREADS || table == TRIDI_AUTOTUNE_RAGGED_REFINE_THREADS) {
     const bool refine = table == TRIDI_AUTOTUNE_RAGGED_REFINE_THREADS;
     const int k = ilog2(key);

@@ -18,21 +18,20 @@ struct Shape {
   bool warp;
 };
 
-bool choose_shape(int n, Shape* s) {
-  if (!is_pow2(n) || n < 2 || n > 4096) return false;
-  int K = n <= 16 ? n / 2 : (n == 4096 ? 16 : 8);
-  // rows per thread: the process-wide tunable, else the autotuned choice for
-  // this n, else the rule above
-  int tk = tunable(TRIDI_TUNE_CR_ROWS);
-  if (tk <= 0) tk = tuned(TRIDI_AUTOTUNE_CR_ROWS, ilog2(n));
-  if (tk > 0 && is_pow2(tk) && tk <= n / 2 && n / tk <= 256) {
-    // only shapes with an instantiated kernel (see solve_hybrid)
-    if (n / tk <= 32 ? tk <= 16 : (tk == 8 || tk == 16)) K = tk;
-  }
-  s->K = K;
-  s->tps = n / K;
-  s->warp = s->tps <= 32;
+// The shape with `rows` rows per thread, where its kernel exists (see run_hybrid).
+bool shape_of(int n, int rows, Shape* s) {
+  if (!is_pow2(n) || n < 2 || n > 4096 || rows < 1 || !is_pow2(rows) || rows > n / 2 || n / rows > 256) return false;
+  if (n / rows <= 32 ? rows > 16 : (rows != 8 && rows != 16)) return false;
+  *s = Shape{rows, n / rows, n / rows <= 32};
   return true;
+}
+
+bool choose_shape(int n, Shape* s) {
+  // rows per thread: the process-wide tunable, else the autotuned choice for
+  // this n, else the rule
+  int rows = tunable(TRIDI_TUNE_CR_ROWS);
+  if (rows <= 0) rows = is_pow2(n) ? tuned(TRIDI_AUTOTUNE_CR_ROWS, ilog2(n)) : 0;
+  return shape_of(n, rows, s) || shape_of(n, n <= 16 ? n / 2 : (n == 4096 ? 16 : 8), s);
 }
 
 constexpr int kWarpThreads = 128 + 32;   // 4 consumer warps + producer warp
@@ -140,6 +139,31 @@ tridi_status solve_hybrid(const double* a, const double* b, const double* c, con
   return cr64_solve(a, b, c, d, x, n, m, stride, as_stream(stream));
 }
 
+// The hybrid kernel of a shape.
+tridi_status run_hybrid(const HybridParams& p0, const Shape& sh, const DeviceInfo& dev, cudaStream_t s) {
+  HybridParams p = p0;
+  p.tps = sh.tps;
+  p.ct = sh.warp ? 128 : (sh.tps > 128 ? sh.tps : 128);
+  p.G = p.ct / sh.tps;
+  p.scratch_rows = p.stride < sh.K ? p.n / p.stride : sh.tps;
+  p.ntiles = (int)(((long)p.m + p.G - 1) / p.G);
+  const int ls = p.stride < sh.K ? p.stride : 0;
+  cudaError_t e = cudaErrorInvalidValue;
+#define TRIDI_LAUNCH_LS(KK, WW, LS) \
+  if (sh.K == KK && sh.warp == WW && ls == LS) e = launch_one<float, KK, WW, LS>(p, dev, s);
+#define TRIDI_LAUNCH(KK, WW)                                                             \
+  TRIDI_LAUNCH_LS(KK, WW, 0)                                                              \
+  if constexpr (KK > 1) { TRIDI_LAUNCH_LS(KK, WW, 1) }                                    \
+  if constexpr (KK > 2) { TRIDI_LAUNCH_LS(KK, WW, (KK > 2 ? 2 : 1)) }                     \
+  if constexpr (KK > 4) { TRIDI_LAUNCH_LS(KK, WW, (KK > 4 ? 4 : 1)) }                     \
+  if constexpr (KK > 8) { TRIDI_LAUNCH_LS(KK, WW, (KK > 8 ? 8 : 1)) }
+  TRIDI_LAUNCH(1, true) TRIDI_LAUNCH(2, true) TRIDI_LAUNCH(4, true) TRIDI_LAUNCH(8, true)
+  TRIDI_LAUNCH(16, true) TRIDI_LAUNCH(8, false) TRIDI_LAUNCH(16, false)
+#undef TRIDI_LAUNCH
+#undef TRIDI_LAUNCH_LS
+  return cuda_status(e);
+}
+
 tridi_status solve_hybrid(const float* a, const float* b, const float* c, const float* d, float* x, int n, int m,
                           int stride, tridi_stream_t stream) {
   if (!a || !b || !c || !d || !x || m <= 0) return TRIDI_ERROR_INVALID_VALUE;
@@ -149,14 +173,9 @@ tridi_status solve_hybrid(const float* a, const float* b, const float* c, const 
   if (!dev) return TRIDI_ERROR_CUDA;
   HybridParams p{};
   p.a = a; p.b = b; p.c = c; p.d = d; p.x = x;
-  p.n = n; p.m = m; p.tps = sh.tps; p.stride = stride;
-  p.ct = sh.warp ? 128 : (sh.tps > 128 ? sh.tps : 128);
-  p.G = p.ct / sh.tps;
-  p.scratch_rows = stride < sh.K ? n / stride : sh.tps;
-  p.ntiles = (int)(((long)m + p.G - 1) / p.G);
+  p.n = n; p.m = m; p.stride = stride;
   p.status = dev->status;
   cudaStream_t s = as_stream(stream);
-  cudaError_t e = cudaErrorInvalidValue;
   if (stride == 1 && pcr_wide_applies(a, b, c, d, n, m, n)) return pcr_wide_solve(a, b, c, d, x, n, m, n, s);
   if (crpcr_wide_applies(a, b, c, d, x, n, m, stride)) return crpcr_wide_solve(a, b, c, d, x, n, m, stride, s);
   if (crpcr_regs_applies(a, b, c, d, x, n, m, stride)) return crpcr_regs_solve(a, b, c, d, x, n, m, stride, s);
@@ -175,20 +194,7 @@ tridi_status solve_hybrid(const float* a, const float* b, const float* c, const 
                                          : launch_pcr_twophase<1024, false>(p, *dev, s));
     }
   }
-  const int ls = stride < sh.K ? stride : 0;
-#define TRIDI_LAUNCH_LS(KK, WW, LS) \
-  if (sh.K == KK && sh.warp == WW && ls == LS) e = launch_one<float, KK, WW, LS>(p, *dev, s);
-#define TRIDI_LAUNCH(KK, WW)                                                             \
-  TRIDI_LAUNCH_LS(KK, WW, 0)                                                              \
-  if constexpr (KK > 1) { TRIDI_LAUNCH_LS(KK, WW, 1) }                                    \
-  if constexpr (KK > 2) { TRIDI_LAUNCH_LS(KK, WW, (KK > 2 ? 2 : 1)) }                     \
-  if constexpr (KK > 4) { TRIDI_LAUNCH_LS(KK, WW, (KK > 4 ? 4 : 1)) }                     \
-  if constexpr (KK > 8) { TRIDI_LAUNCH_LS(KK, WW, (KK > 8 ? 8 : 1)) }
-  TRIDI_LAUNCH(1, true) TRIDI_LAUNCH(2, true) TRIDI_LAUNCH(4, true) TRIDI_LAUNCH(8, true)
-  TRIDI_LAUNCH(16, true) TRIDI_LAUNCH(8, false) TRIDI_LAUNCH(16, false)
-#undef TRIDI_LAUNCH
-#undef TRIDI_LAUNCH_LS
-  return cuda_status(e);
+  return run_hybrid(p, sh, *dev, s);
 }
 
 }  // namespace
@@ -198,6 +204,20 @@ template <class T>
 tridi_status hybrid_solve_device(const T* a, const T* b, const T* c, const T* d, T* x, int n, int m, int stride,
                                  tridi_stream_t stream) {
   return solve_hybrid(a, b, c, d, x, n, m, stride, stream);
+}
+// cr and crpcr by the hybrid kernel with `rows` rows per thread, whichever kernel
+// the entry points take.
+tridi_status hybrid_rows_solve(const float* a, const float* b, const float* c, const float* d, float* x, int n, int m,
+                               int stride, int rows, tridi_stream_t stream) {
+  Shape sh;
+  if (!shape_of(n, rows, &sh)) return TRIDI_ERROR_UNSUPPORTED_SIZE;
+  const DeviceInfo* dev = current_device();
+  if (!dev) return TRIDI_ERROR_CUDA;
+  HybridParams p{};
+  p.a = a; p.b = b; p.c = c; p.d = d; p.x = x;
+  p.n = n; p.m = m; p.stride = stride;
+  p.status = dev->status;
+  return run_hybrid(p, sh, *dev, as_stream(stream));
 }
 template tridi_status hybrid_solve_device<float>(const float*, const float*, const float*, const float*, float*,
                                                  int, int, int, tridi_stream_t);
