@@ -98,6 +98,27 @@ __device__ __forceinline__ void load_rows(const double* p, long at, bool in, boo
   }
 }
 
+// Host memory in place, K = 8: a thread's 64 bytes cross the host link in four
+// pieces (1024 x 4096 cr 1190 us a call, pinned arrays), so the tile's rows (all
+// of them consecutive) move by consecutive threads and change hands in shared
+// memory, a word of padding every 8: STAGED us; 762 us by the kernels before this
+// one.  (Four rows a thread would do too, but round differently.)
+__device__ __forceinline__ int host_at(int e) { return e + (e >> 3); }
+template <int K>
+__device__ __forceinline__ void load_rows_host(const double* p, long base, long total, double other, double* s,
+                                               double (&v)[K]) {
+  const int ct = blockDim.x, tid = threadIdx.x;
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    const long e = base + j * ct + tid;
+    s[host_at(j * ct + tid)] = e < total ? __ldg(p + e) : other;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < K; ++i) v[i] = s[host_at(tid * K + i)];
+  __syncthreads();
+}
+
 // Shared memory of a CTA of ct threads, in words a thread: the exported rows
 // of the in-thread levels (3 words each, up to 3 levels; later the two PCR
 // buffers of one row a thread), then the level arrays a, b, c, d of 2 words
@@ -252,9 +273,11 @@ __device__ __forceinline__ void cr_levels_any(const Levels64& v, int G, int per0
 // LS = 0: the intermediate system has at most one row a thread (n / rest >=
 // K); LS > 0: LS = n / rest < K, K / LS rows a thread; LS = -1: any n, cyclic
 // reduction throughout (rows past the system's end are identity rows).
-template <int K, int LS, int MAXT, int MINB>
+// HOST: the arrays are host memory (K = 8).
+template <int K, int LS, int MAXT, int MINB, bool HOST>
 __global__ void __launch_bounds__(MAXT, MINB) cr64_kernel(Cr64Params p) {
   constexpr bool ANY = LS < 0;
+  static_assert(!HOST || (K == 8 && !ANY && K + 1 <= kExportWords), "cr64: host arrays");
   constexpr int SMAX = LS <= 0 ? K : LS;  // last in-thread CR level
   extern __shared__ __align__(16) double sm[];
   const int ct = blockDim.x, tid = threadIdx.x, tps = p.tps;
@@ -271,17 +294,22 @@ __global__ void __launch_bounds__(MAXT, MINB) cr64_kernel(Cr64Params p) {
     Row<double> r[K];
     const bool whole = in && (!ANY || (t + 1) * K <= p.n);
     {
+      const long base = (long)tile * G * p.n, total = (long)p.m * p.n;
+      const auto load = [&](const double* src, double other, double (&v)[K]) {
+        if constexpr (HOST) load_rows_host<K>(src, base, total, other, ex, v);
+        else load_rows<K>(src, at, whole, p.vec, other, v);
+      };
       double v[K];
-      load_rows<K>(p.a, at, whole, p.vec, 0.0, v);
+      load(p.a, 0.0, v);
 #pragma unroll
       for (int i = 0; i < K; ++i) r[i].a = v[i];
-      load_rows<K>(p.b, at, whole, p.vec, 1.0, v);
+      load(p.b, 1.0, v);
 #pragma unroll
       for (int i = 0; i < K; ++i) r[i].b = v[i];
-      load_rows<K>(p.c, at, whole, p.vec, 0.0, v);
+      load(p.c, 0.0, v);
 #pragma unroll
       for (int i = 0; i < K; ++i) r[i].c = v[i];
-      load_rows<K>(p.d, at, whole, p.vec, 0.0, v);
+      load(p.d, 0.0, v);
 #pragma unroll
       for (int i = 0; i < K; ++i) r[i].d = v[i];
     }
@@ -463,7 +491,17 @@ __global__ void __launch_bounds__(MAXT, MINB) cr64_kernel(Cr64Params p) {
         else xr[i] = fma(-r[i].c, xr[(i + h) % K], fma(-r[i].a, xl, r[i].d));
       }
     }
-    if (ANY && in && !whole) {
+    if constexpr (HOST) {
+#pragma unroll
+      for (int i = 0; i < K; ++i) ex[host_at(tid * K + i)] = xr[i];
+      __syncthreads();
+      const long base = (long)tile * G * p.n, total = (long)p.m * p.n;
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        const int e = j * ct + tid;
+        if (base + e < total) p.x[base + e] = ex[host_at(e)];
+      }
+    } else if (ANY && in && !whole) {
 #pragma unroll
       for (int i = 0; i < K; ++i)
         if (t * K + i < p.n) p.x[at + i] = xr[i];
@@ -483,7 +521,11 @@ __global__ void __launch_bounds__(MAXT, MINB) cr64_kernel(Cr64Params p) {
 
 template <int K, int LS, int MAXT = 256>
 cudaError_t launch_cr64(Cr64Params p, const DeviceInfo& dev, cudaStream_t stream) {
-  auto kern = cr64_kernel<K, LS, MAXT, (MAXT > 256 ? 1 : K == 4 ? 3 : 2)>;
+  constexpr int MINB = MAXT > 256 ? 1 : K == 4 ? 3 : 2;
+  auto kern = cr64_kernel<K, LS, MAXT, MINB, false>;
+  if constexpr (K == 8 && LS >= 0) {
+    if (g_host_mapped_io) kern = cr64_kernel<K, LS, MAXT, MINB, true>;
+  }
   // 128 threads a CTA (a system of 2048 rows takes 256; 256 threads throughout
   // measured 410 us against 371 us at 16384 x 1024, 64 threads no gain), fewer
   // where that would leave SMs without one
