@@ -21,13 +21,17 @@ cudaError_t cudaGetLastError(void) {
 namespace tridi {
 static DeviceInfo g_dev;
 const DeviceInfo* current_device() { return &g_dev; }
+static bool g_allowed = true;  // the kernel's limit is raised
+bool smem_allowed(const void*, size_t) { return g_allowed; }
 cudaError_t raise_smem_limit(const void*, const DeviceInfo&) {
   ++g_raised;
+  g_allowed = true;
   return cudaSuccess;
 }
 }  // namespace tridi
 
-static void scenario(cudaError_t unread, std::vector<cudaError_t> answers, size_t smem) {
+static void scenario(bool allowed, cudaError_t unread, std::vector<cudaError_t> answers, size_t smem) {
+  tridi::g_allowed = allowed;
   g_launches = g_raised = 0;
   g_last = unread;
   g_answers = answers;
@@ -43,12 +47,13 @@ static void scenario(cudaError_t unread, std::vector<cudaError_t> answers, size_
 
 int main() {
   const cudaError_t bad = cudaErrorInvalidValue, other = cudaErrorMemoryAllocation;
-  scenario(cudaSuccess, {}, 100000);
-  scenario(bad, {}, 100000);         // the caller's unread error
-  scenario(other, {}, 100000);
-  scenario(cudaSuccess, {bad}, 100000);       // the limit was dropped
-  scenario(other, {bad}, 100000);
-  scenario(cudaSuccess, {bad, bad}, 100000);  // and cannot be had
-  scenario(cudaSuccess, {bad}, 1000);         // not the limit
-  scenario(cudaSuccess, {other}, 100000);
+  scenario(true, cudaSuccess, {}, 100000);
+  scenario(true, bad, {}, 100000);  // the caller's unread error
+  scenario(true, other, {}, 100000);
+  scenario(false, cudaSuccess, {bad}, 100000);       // the limit was dropped
+  scenario(false, other, {bad}, 100000);
+  scenario(false, cudaSuccess, {bad, bad}, 100000);  // and does not help
+  scenario(true, cudaSuccess, {bad}, 100000);        // not the limit
+  scenario(true, cudaSuccess, {bad}, 1000);
+  scenario(true, cudaSuccess, {other}, 100000);
 }

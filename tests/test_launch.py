@@ -1,7 +1,7 @@
-"""A launch is judged by its own answer (csrc/runtime.h, checked_launch): an
-error that the calling thread had not read does not make it run twice, and is
-returned after it; a launch that fails for want of the shared-memory limit is
-repeated once with the limit set.  On the CPU, against fakes of the runtime."""
+"""Launches run once (csrc/runtime.h, checked_launch): an error that the calling
+thread had not read does not make one run twice, and is returned after it; a
+launch that fails for want of the shared-memory limit is repeated once with the
+limit set.  On the CPU, against fakes of the runtime."""
 from __future__ import annotations
 
 import shutil
@@ -14,7 +14,7 @@ ROOT = Path(__file__).resolve().parents[1]
 BAD, OTHER = 1, 2  # cudaErrorInvalidValue, cudaErrorMemoryAllocation
 
 
-def test_launch_is_judged_by_its_own_answer(tmp_path):
+def test_launches_run_once(tmp_path):
     cxx = shutil.which("g++")
     inc = Path("/usr/local/cuda/include")
     if not cxx or not inc.exists():
@@ -31,8 +31,9 @@ def test_launch_is_judged_by_its_own_answer(tmp_path):
         (1, 0, BAD, 0),
         (1, 0, OTHER, 0),
         (2, 1, 0, 0),
-        (2, 1, OTHER, 0),
+        (2, 1, 0, 0),
         (2, 1, BAD, 0),
+        (1, 0, BAD, 0),
         (1, 0, BAD, 0),
         (1, 0, OTHER, 0),
     ]

@@ -81,6 +81,11 @@ cudaError_t raise_smem_limit(const void* kern, const DeviceInfo& dev) {
                               dev.max_smem_optin - (int)at.sharedSizeBytes);
 }
 
+bool smem_allowed(const void* kern, size_t smem) {
+  cudaFuncAttributes at;
+  return cudaFuncGetAttributes(&at, kern) == cudaSuccess && (size_t)at.maxDynamicSharedSizeBytes >= smem;
+}
+
 cudaError_t resident_blocks(const void* kern, int threads, size_t smem, const DeviceInfo& dev, int* per_sm) {
   struct Entry {
     const void* kern;

@@ -43,23 +43,24 @@ cudaError_t resident_blocks(void (*kern)(P...), int threads, size_t smem, const 
 // beside its static shared memory.
 cudaError_t raise_smem_limit(const void* kern, const DeviceInfo& dev);
 
-// A launch with `smem` bytes of dynamic shared memory, judged by its own error:
-// one that the thread had not read is taken first and returned after the
-// launch, as after every other launch here, and is no reason to launch again.
-// A device reset drops a raised limit; the launch then fails and is repeated
-// with the limit set.
+// Whether the kernel may be launched with `smem` bytes of dynamic shared memory.
+bool smem_allowed(const void* kern, size_t smem);
+
+// A launch with `smem` bytes of dynamic shared memory.  A device reset drops a
+// raised limit; the launch then fails and is repeated with the limit set.  Only
+// then: the same error may be one that the thread had not read, which is
+// returned, as after every other launch here, and is no reason to launch again.
 template <class Launch>
 cudaError_t checked_launch(const Launch& launch, const void* kern, size_t smem) {
-  const cudaError_t unread = cudaGetLastError();
   launch();
   cudaError_t e = cudaGetLastError();
-  if (e == cudaErrorInvalidValue && smem > 48 * 1024) {
+  if (e == cudaErrorInvalidValue && smem > 48 * 1024 && !smem_allowed(kern, smem)) {
     const DeviceInfo* dev = current_device();
     if (!dev || raise_smem_limit(kern, *dev) != cudaSuccess) return e;
     launch();
     e = cudaGetLastError();
   }
-  return e != cudaSuccess ? e : unread;
+  return e;
 }
 
 #ifdef __CUDACC__
