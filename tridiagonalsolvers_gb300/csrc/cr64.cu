@@ -273,11 +273,11 @@ __device__ __forceinline__ void cr_levels_any(const Levels64& v, int G, int per0
 // LS = 0: the intermediate system has at most one row a thread (n / rest >=
 // K); LS > 0: LS = n / rest < K, K / LS rows a thread; LS = -1: any n, cyclic
 // reduction throughout (rows past the system's end are identity rows).
-// HOST: the arrays are host memory (K = 8).
+// HOST: the arrays are host memory, moved in whole lines.
 template <int K, int LS, int MAXT, int MINB, bool HOST>
 __global__ void __launch_bounds__(MAXT, MINB) cr64_kernel(Cr64Params p) {
   constexpr bool ANY = LS < 0;
-  static_assert(!HOST || (K == 8 && !ANY && K + 1 <= kExportWords), "cr64: host arrays");
+  static_assert(!HOST || (!ANY && K + 1 <= kExportWords), "cr64: host arrays");
   constexpr int SMAX = LS <= 0 ? K : LS;  // last in-thread CR level
   extern __shared__ __align__(16) double sm[];
   const int ct = blockDim.x, tid = threadIdx.x, tps = p.tps;
@@ -523,7 +523,7 @@ template <int K, int LS, int MAXT = 256>
 cudaError_t launch_cr64(Cr64Params p, const DeviceInfo& dev, cudaStream_t stream) {
   constexpr int MINB = MAXT > 256 ? 1 : K == 4 ? 3 : 2;
   auto kern = cr64_kernel<K, LS, MAXT, MINB, false>;
-  if constexpr (K == 8 && LS >= 0) {
+  if constexpr (K == 8 && LS == 0) {
     if (g_host_mapped_io) kern = cr64_kernel<K, LS, MAXT, MINB, true>;
   }
   // 128 threads a CTA (a system of 2048 rows takes 256; 256 threads throughout
