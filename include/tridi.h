@@ -66,8 +66,9 @@ tridi_status tridi_device_status(unsigned *bits, int reset);
    autotuner and by experiments; they change speed, and at most the rounding
    of results (TRIDI_TUNE_PCR_KERNEL, TRIDI_TUNE_RESIDUAL), never the
    algorithm. */
-#define TRIDI_TUNE_STAGES 1     /* cp.async.bulk pipeline stages per CTA (1..8) */
-#define TRIDI_TUNE_CRPCR_REST 2 /* switch level of the CR-PCR correction solves */
+#define TRIDI_TUNE_STAGES 1     /* cp.async.bulk pipeline stages per CTA (1..8) of the hybrid, shared-memory CR and
+                                   shared-memory PCR-then-Thomas kernels */
+#define TRIDI_TUNE_CRPCR_REST 2 /* switch level of the refinement's CR-PCR solves (see TRIDI_AUTOTUNE_CRPCR_REST) */
 #define TRIDI_TUNE_CR_ROWS 3    /* rows per thread of the FP32 hybrid CR/PCR/CR-PCR kernels (2, 4, 8, 16) */
 #define TRIDI_TUNE_RESIDUAL 4   /* arithmetic of the refinements' residual and update: */
 #define TRIDI_RESIDUAL_DF 1     /*   double-float (pairs of FP32, 48-bit significand; the default) */
@@ -103,14 +104,14 @@ int tridi_get_tunable(int key);
 
 /* ---- the reference's solvers, device pointers ---------------------------- */
 /* Cyclic reduction.  Replaces cr() of cr_app.cu:4 / crKernel (cr_kernel.cu:1).
-   n a power of two, 2 <= n <= 8192. */
+   n a power of two, 2 <= n <= 4096 (FP64: 2048). */
 tridi_status tridi_cr_f32(const float *a, const float *b, const float *c, const float *d, float *x, int n,
                           int num_systems, tridi_stream_t stream);
 tridi_status tridi_cr_f64(const double *a, const double *b, const double *c, const double *d, double *x,
                           int n, int num_systems, tridi_stream_t stream);
 
 /* Parallel cyclic reduction.  Replaces pcr() of pcr_app.cu:5 / pcrKernel
-   (pcr_kernel.cu:1).  n a power of two, 2 <= n <= 4096. */
+   (pcr_kernel.cu:1).  n a power of two, 2 <= n <= 4096 (FP64: 2048). */
 tridi_status tridi_pcr_f32(const float *a, const float *b, const float *c, const float *d, float *x, int n,
                            int num_systems, tridi_stream_t stream);
 tridi_status tridi_pcr_f64(const double *a, const double *b, const double *c, const double *d, double *x,
@@ -155,7 +156,11 @@ tridi_status tridi_crpcr_nbc_f64(const double *a, const double *b, const double 
    pcrGauss_kernel.cu:1-126).  `gaussian` = g, the number of interleaved
    subsystems (a power of two, 1 <= g <= n) solved by Thomas after log2(g) PCR
    steps.  Exact for every g (the reference's step table is exact only when
-   g = 2^it).  gaussian = 0: the autotuned g for n (TRIDI_AUTOTUNE_PCR_THOMAS_SPLIT),
+   g = 2^it).  The register kernels (FP32, aligned device arrays: powers of two
+   64 to 1024, and 32, 2048 and 4096 from g = 4 on) run a smaller g as the least
+   split whose chains stay in one lane: 2 chains at 32, 4 at 64, 8 at 128, 16 at
+   256, 32 at 512 and 1024, 64 at 2048, 128 at 4096; the solution is the same up
+   to rounding.  gaussian = 0: the autotuned g for n (TRIDI_AUTOTUNE_PCR_THOMAS_SPLIT),
    else n/2 for power-of-two n (else one chain per thread of the system).
    g >= n/2 on power-of-two n runs the register PCR kernels (log2(n/2) PCR
    steps leave exactly the 2-row chains PCR closes with).  Any 1 <= n <= 4096. */
@@ -197,7 +202,10 @@ tridi_status tridi_solve_large_f64(const double *a, const double *b, const doubl
    *chosen (and its time per launch in *best_ms; either may be NULL):
      TRIDI_AUTOTUNE_CRPCR_REST    key n (power of two, 4..4096): the CR-to-PCR
         switch level (rest system size, 2..n/2) that the refinement's FP32
-        correction solves use; diagonally dominant systems.
+        solves use where they run CR-PCR: contiguous powers of two at tolerances
+        above 1e-8, in native FP64 and in sweeps after the first correction (at
+        2048 and 4096 every level above n/32 is one kernel); diagonally dominant
+        systems.
      TRIDI_AUTOTUNE_PCR_THOMAS_SPLIT  key n (power of two, 2..4096): the number
         of Thomas chains g (PCR steps = log2 g) that tridi_pcr_thomas_* use
         when called with gaussian = 0; diagonally dominant systems.

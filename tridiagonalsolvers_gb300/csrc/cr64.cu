@@ -16,7 +16,7 @@
 //     computing all levels and four rows a thread, the same CR issued 98 FP64
 //     instructions an unknown: 2939 us at 16384 x 1024, 1456 us with the
 //     divisions replaced.)
-// Measured at 16384 x 1024: 369 us, 8.8 FP64 instructions an unknown, FP64
+// Measured at 16384 x 1024: 370 us, 8.9 FP64 instructions an unknown, FP64
 // pipe 64 % busy; the rest is the latency of the last levels, in which one
 // warp of a CTA works.
 // Rows are read from global memory as they are (K consecutive rows a thread:
@@ -583,7 +583,7 @@ tridi_status cr64_solve(const double* a, const double* b, const double* c, const
 // per lane and PCR on the 32 to 512 separators, issued 90 FP64 instructions a
 // row at 1000 rows, 15 of them with the integer division: 4096 x 1000 684 and
 // 257 us, cyclic reduction 106 us; 100000 x 20 1571 us, 48 us; 800 x 4608
-// 394 us, 147 us.)
+// 394 us, 152 us.)
 tridi_status cr64_solve_any(const double* a, const double* b, const double* c, const double* d, double* x, int n, int m,
                             cudaStream_t stream) {
   const DeviceInfo* dev = current_device();

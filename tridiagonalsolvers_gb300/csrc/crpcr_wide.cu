@@ -24,7 +24,8 @@
 // warp's solve, which the SM's other CTAs cover.  16.8 M unknowns: cr 57 us at
 // 2048 and 58 us at 4096 (86 and 84 % of the copy rate; the hybrid kernel, CR
 // levels between warps through shared memory, 80 and 151 us), crpcr the same at
-// every rest (79 to 161 and 147 to 327 us).
+// every rest (79 to 161 and 147 to 327 us; above n / 32 the hybrid kernel's times
+// are with PCR steps that are CR levels here).
 #include "crpcr2.cuh"
 #include "hybrid.cuh"
 #include "runtime.h"

@@ -1,23 +1,26 @@
 // TMA-tiled passes of the large-system solver for the interleaved FP32
 // layout (element i of system s at i*m + s, m a multiple of 32).
 //
-// The two passes of large.cu that read the coefficients -- large_reduce
-// (chunk elimination, interface out) and large_back (elimination again, back
-// substitution, x out) -- as persistent kernels: one CTA per SM, a producer
-// warp that streams tiles of kTileRows rows x 32 systems of a, b, c, d into a
-// kStages-deep shared-memory ring with cp.async.bulk.tensor.2d (one tensor
-// map per array), and 8 consumer warps.  Warp w of a tile owns rows
-// [w*16, w*16 + 16) of it, lane l system s0 + l: exactly the chunks (16 rows
-// of one system) of the register kernels, so the interface arrays, the
-// separator assembly and the recursion are shared with them.  A lane reads
-// its column of the tile (row stride 32 words: lane l always on bank l, no
-// conflicts), eliminates it in place, and writes its interface (reduce) or
-// its 16 unknowns (back) straight to global memory: consecutive lanes,
-// consecutive systems, one 128-byte line per row.
+// The passes of large.cu that read the coefficients as persistent kernels, one
+// CTA per SM, on the chunks of its register kernels (16 rows of one system), so
+// that the separator system and the recursion are shared with them:
+//   * large_reduce_tile_kernel eliminates the chunks and writes the separator
+//     system.  A producer warp streams tiles of kTileRows rows x 32 systems of a,
+//     b, c, d into a kStages-deep shared-memory ring with
+//     cp.async.bulk.tensor.2d (one tensor map per array); 8 consumer warps,
+//     warp w rows [w*16, w*16 + 16) of a tile, lane l system s0 + l, eliminate
+//     in registers and give the stage back.
+//   * large_back_tile_kernel solves each chunk between its separators by a
+//     Thomas sweep and writes the unknowns.  Three groups of four warps, each
+//     with tiles of its own (64 rows x 32 systems) and a two-stage ring that
+//     the group's first thread refills; no producer.
+// A lane reads its column of a tile at a row stride of 32 words (lane l always
+// on bank l, no conflicts); what it writes goes straight to global memory:
+// consecutive lanes, consecutive systems, one 128-byte line per row.
 //
 // Against the register kernels (one thread per chunk, 64 prefetched values
-// and the chunk's eliminated rows in registers, two blocks per SM) the ring
-// keeps 128 KB of loads in flight per SM whatever the compute is doing.
+// and the chunk's eliminated rows in registers, two blocks per SM) the rings
+// keep 128 KB and more of loads in flight per SM whatever the compute is doing.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>

@@ -13,8 +13,9 @@
 // chains of the whole system).  x goes out through shared memory, consecutive
 // unknowns by consecutive lanes.
 //
-// What bounds it: latency, at 8 warps of 255 registers an SM, and the nine
-// barriers of a system (the other CTAs of the SM run in their shadow).  16.8 M
+// What bounds it: latency, at 8 warps of 255 registers an SM, and the barriers of
+// a system, six at 2048 rows and seven at 4096 (the other CTAs of the SM run in
+// their shadow).  16.8 M
 // unknowns: pcr 99 us at 2048 and 106 us at 4096 (the hybrid kernel, PCR steps
 // through shared memory with two barriers each: 352 and 630 us), pcrGauss g = 8
 // 84 and 91 us (pcr_thomas.cu: 1085 and 1097 us).

@@ -690,7 +690,8 @@ __device__ __forceinline__ void refine1_pass(const RagParams& p, const RagSys& s
 // the factors and stays; a second pass writes x0 + e as FP64 and the residual's
 // norm.  100000 systems of 32 to 8192 rows:
 // 1793 us with two eliminations and the originals staged again in between,
-// 1630 us so.  M: kRefineDF or kRefineFP64.
+// 1630 us so (before the norms in two scales, see group_rel_max).  M: kRefineDF or
+// kRefineFP64.
 // (Four rows a thread and step in the passes; two for a warp's small systems, and
 // in the kernel with the BIG path, which has no registers left: 400 systems of
 // 9000 to 24000 rows 616 us with four, 605 with two.)

@@ -10,8 +10,8 @@
 // the separate solves and residual passes of refine.cu move 96 B, and a block
 // of 256 threads formed the residual of each system, whatever its size.
 // What bounds it: issue and dependency latency (about 200 instructions a row).
-// 200000 x 64: 4798 -> 224 us; 16000 x 1000: 829 -> 314 us; 2000 x 8000: 590 ->
-// 368 us (a call, with its two host round trips before and one now).
+// 200000 x 64: 4798 -> 210 us; 16000 x 1000: 829 -> 270 us; 2000 x 8000: 590 ->
+// 335 us (a call, with its two host round trips before and one now).
 //
 // Sums of squares are FP32, in two scales (SquareSum: d and r of any size);
 // their quotient is formed on the integer units (div64.cuh), so the FP64 pipe
