@@ -239,37 +239,61 @@ struct XStore {
   }
 };
 
-// Adds the sums of squares rd (of r, of d) over a solve group, and its leader
-// folds ||r|| / ||d|| into the CTA's maximum `rel` (shared memory; the kernel
-// folds it into the batch maximum once at the end): ||r|| itself for a zero
-// right-hand side, NaN where ||d|| is infinite or NaN.  The sums stay in FP32,
-// like the per-lane partials (GB300's FP64 adds, square roots and divisions are
-// slow), in two scales (r and d of any size; in one, which took residuals below
-// 1e-22 for zero, 100000 systems of 32 to 8192 rows took 1625 us, 1683 us so).
-// red: 4 floats per warp.
-__device__ __forceinline__ float square_root(const SquareSum& q) {
-  return q.s.x < 0x1p114f ? sqrtf(q.s.x) * 0x1p-58f : sqrtf(q.s.y) * 0x1p58f;
+// Norms.  r and d are squared times a power of two s, one a system, that brings
+// its largest |d| to 1 .. 2: the squares of any right-hand side stay in FP32's
+// range, and those of residuals down to 1e-19 of it.  (Unscaled, residuals below
+// 1e-22 counted as zero; 100000 systems of 32 to 8192 rows took 1630 us, 1660 us
+// so, and 1683 us with sums in two fixed scales.)
+// red: 4 floats per warp, the third for the scale.
+//
+// A thread's largest |d|, over its warp, left for the group's other warps (a
+// group barrier must follow before group_scale); returns the warp's.
+__device__ __forceinline__ unsigned put_largest(float m, int gt, float* red) {
+  const unsigned u = __reduce_max_sync(kFull, __float_as_uint(m));
+  if (gt > 32 && (threadIdx.x & 31) == 0) red[4 * (threadIdx.x >> 5) + 2] = __uint_as_float(u);
+  return u;
 }
-__device__ __forceinline__ void group_rel_max(const SquareSums& rd, int gt, int bar, int gtid, SquareSum* red,
+// The system's scale s (u: put_largest's answer).
+__device__ __forceinline__ float group_scale(unsigned u, int gt, int gtid, const float* red) {
+  if (gt > 32) {
+    const float* q = red + 4 * (((int)threadIdx.x - gtid) >> 5) + 2;
+    for (int w = 0; w < gt / 32; ++w) {
+      const unsigned v = __float_as_uint(q[4 * w]);
+      u = v > u ? v : u;
+    }
+  }
+  const unsigned e = u >> 23;  // (zero right-hand side: any scale; infinite: the smallest)
+  return __uint_as_float((e < 253u ? 254u - e : 1u) << 23);
+}
+
+// Adds the sums of squares (rr, dd) over a solve group, and its leader folds
+// sqrt(rr) / sqrt(dd) into the CTA's maximum `rel` (shared memory; the kernel
+// folds it into the batch maximum once at the end): 0 over 0 is 0, and NaN where
+// dd is infinite or NaN.  The sums stay in FP32, like the per-lane partials
+// (GB300's FP64 adds, square roots and divisions are slow).
+__device__ __forceinline__ void group_rel_max(float rr, float dd, int gt, int bar, int gtid, float* red,
                                               unsigned long long* rel) {
-  SquareSum rr = square_total(rd.first(), 32), dd = square_total(rd.second(), 32);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    rr += __shfl_down_sync(kFull, rr, o);
+    dd += __shfl_down_sync(kFull, dd, o);
+  }
   if (gt > 32) {
     const int w = threadIdx.x >> 5;
     if ((threadIdx.x & 31) == 0) {
-      red[2 * w] = rr;
-      red[2 * w + 1] = dd;
+      red[4 * w] = rr;
+      red[4 * w + 1] = dd;
     }
     group_sync(bar, gt);
     if (gtid == 0) {
       for (int q = 1; q < gt / 32; ++q) {
-        rr.s = __fadd2_rn(rr.s, red[2 * (w + q)].s);
-        dd.s = __fadd2_rn(dd.s, red[2 * (w + q) + 1].s);
+        rr += red[4 * (w + q)];
+        dd += red[4 * (w + q) + 1];
       }
     }
   }
   if (gtid == 0) {
-    const float r = square_root(rr), d = square_root(dd), inf = __int_as_float(0x7f800000);
-    const float v = d == 0.f ? r : d < inf ? r / d : __int_as_float(0x7fffffff);
+    const float v = dd == 0.f ? sqrtf(rr) : dd < INFINITY ? sqrtf(rr) / sqrtf(dd) : __int_as_float(0x7fffffff);
     atomicMax(rel, (unsigned long long)__double_as_longlong((double)v));  // the CTA's maximum, in shared memory
   }
 }
@@ -512,15 +536,21 @@ __device__ __forceinline__ void group_refine(const RagParams& p, const RagSys& s
     group_solve(n, gt, bar, gtid, sa, sb, sc, sd, R, X, F0, add, RhsResidual<MODE>{xs, n});
   }
   restage(rs, par, gt, bar, gtid, p.status);
-  SquareSums rd;
+  float* redf = reinterpret_cast<float*>(red);
+  float m = 0.f, rr = 0.f, dd = 0.f;
+  for (int i = gtid; i < n; i += gt) m = fmaxf(m, fabsf(sd[i]));
+  const unsigned largest = put_largest(m, gt, redf);
+  if (gt > 32) group_sync(bar, gt);
+  const float scale = group_scale(largest, gt, gtid, redf);
   double* xo = p.x64 + sy.off;
   for (int i = gtid; i < n; i += gt) {
     const float d = sd[i];
     const float r = xs.residual(i, n, sa[i], sb[i], sc[i], d);
-    rd.add(make_float2(r, d));
+    rr = fmaf(r * scale, r * scale, rr);
+    dd = fmaf(d * scale, d * scale, dd);
     xo[i] = xs.get64(i);
   }
-  group_rel_max(rd, gt, bar, gtid, reinterpret_cast<SquareSum*>(red),
+  group_rel_max(rr, dd, gt, bar, gtid, redf,
                 reinterpret_cast<unsigned long long*>(red + 2 * kRagWarps));
 }
 
@@ -533,7 +563,8 @@ __device__ __forceinline__ void group_refine(const RagParams& p, const RagSys& s
 // by component; steps away from the system's ends skip the bounds checks.
 //   FINAL = false: r = d - T x0 (x0 in xw), times 1 / pivot in place of it (ew),
 //                  and a and c times 1 / pivot over a and c (aw, cw): what the
-//                  correction's solve from the factors takes.
+//                  correction's solve from the factors takes.  Returns the
+//                  thread's largest |d|.
 //   FINAL = true:  x = x0 + e (e in ew), written as FP64; the group's
 //                  ||d - T x|| / ||d|| folded into the CTA's maximum.
 // With single-word accesses (22 a pair of rows, 11 now, 6 with V = 4) and the
@@ -556,8 +587,9 @@ struct RowGroup {  // V rows' coefficients
   }
 };
 template <int M, bool FINAL, int V>
-__device__ __forceinline__ void refine1_pass(const RagParams& p, const RagSys& sy, int gt, int bar, int gtid,
-                                             const float* xw, float* ew, float* aw, float* cw, double* red) {
+__device__ __forceinline__ float refine1_pass(const RagParams& p, const RagSys& sy, int gt, int bar, int gtid,
+                                              const float* xw, float* ew, float* aw, float* cw, float scale,
+                                              double* red) {
   using W = RowWords<V>;
   const int n = sy.n;
   const int pad = (int)(sy.off & (V - 1));
@@ -567,7 +599,9 @@ __device__ __forceinline__ void refine1_pass(const RagParams& p, const RagSys& s
   RowGroup<V> next{};
   if (gtid < groups) next.load(p, sy.off - pad, gtid);
   gsync(bar, gt);  // the group's solution is in the ring
-  SquareSums rr, dd;  // over the even and over the odd rows
+  [[maybe_unused]] float2 rr = make_float2(0.f, 0.f), dd = make_float2(0.f, 0.f);
+  [[maybe_unused]] const float2 scale2 = make_float2(scale, scale);
+  float largest = 0.f;
   // the rows from i0 on; INNER: all of them in 1 .. n - 2
   const auto rows = [&](auto inner, int i0, W a, W b, W c, W d) {
     constexpr bool INNER = decltype(inner)::value;
@@ -640,9 +674,10 @@ __device__ __forceinline__ void refine1_pass(const RagParams& p, const RagSys& s
       }
 #pragma unroll
       for (int q = 0; q < V; q += 2) {
-        const float2 r2 = make_float2(r[q], r[q + 1]), d2 = make_float2(d.v[q], d.v[q + 1]);
-        rr.add(r2);
-        dd.add(d2);
+        const float2 r2 = __fmul2_rn(make_float2(r[q], r[q + 1]), scale2);
+        const float2 d2 = __fmul2_rn(make_float2(d.v[q], d.v[q + 1]), scale2);
+        rr = __ffma2_rn(r2, r2, rr);
+        dd = __ffma2_rn(d2, d2, dd);
         const double v0 = xd[q + 1], v1 = xd[q + 2];
         const int i = i0 + q;
         if (INNER && vec) {
@@ -659,6 +694,7 @@ __device__ __forceinline__ void refine1_pass(const RagParams& p, const RagSys& s
       W g = *w;
 #pragma unroll
       for (int q = 0; q < V; ++q) {
+        largest = fmaxf(largest, fabsf(d.v[q]));
         a.v[q] *= g.v[q];
         c.v[q] *= g.v[q];
         g.v[q] *= r[q];
@@ -677,9 +713,9 @@ __device__ __forceinline__ void refine1_pass(const RagParams& p, const RagSys& s
     else rows(std::false_type{}, i0, at.a, at.b, at.c, at.d);
   }
   if constexpr (FINAL)
-    group_rel_max({make_float2(rr.up.x + rr.up.y, dd.up.x + dd.up.y), make_float2(rr.dn.x + rr.dn.y, dd.dn.x + dd.dn.y)},
-                  gt, bar, gtid, reinterpret_cast<SquareSum*>(red),
+    group_rel_max(rr.x + rr.y, dd.x + dd.y, gt, bar, gtid, reinterpret_cast<float*>(red),
                   reinterpret_cast<unsigned long long*>(red + 2 * kRagWarps));
+  return largest;
 }
 
 // One-correction refinement (sweeps == 1) of one staged system by its solve
@@ -718,15 +754,16 @@ __device__ __forceinline__ void group_refine1(const RagParams& p, const RagSys& 
   }
   group_separators(sr, gt, bar, gtid, R, X, sj, sl);
   chunk_between_smem(kr, sj, sl, sa + r0, sb + r0, sc + r0, sd + r0);
-  refine1_pass<M, false, V>(p, sy, gt, bar, gtid, sd, sb, sa, sc, red);
-  gsync(bar, gt);  // the right-hand side is complete
+  float* redf = reinterpret_cast<float*>(red);
+  const unsigned largest = put_largest(refine1_pass<M, false, V>(p, sy, gt, bar, gtid, sd, sb, sa, sc, 1.f, red), gt, redf);
+  gsync(bar, gt);  // the right-hand side is complete, and every warp's largest |d|
   float fD[1], nD[1], lD;
   chunk_rhs_smem(kr, sa + r0, sc + r0, sb + r0, fD[0], lD);
   group_next(fD, nD, gt, bar, gtid, F0);
   sr.d = (kr > 0 ? sb[r0 + kr - 1] : 0.f) - ea * lD - ec * nD[0];
   group_separators(sr, gt, bar, gtid, R, X, sj, sl);
   chunk_between_scaled_smem(kr, sj, sl, sa + r0, sc + r0, sb + r0);
-  refine1_pass<M, true, V>(p, sy, gt, bar, gtid, sd, sb, sa, sc, red);
+  refine1_pass<M, true, V>(p, sy, gt, bar, gtid, sd, sb, sa, sc, group_scale(largest, gt, gtid, redf), red);
 }
 
 // A BIG system (rows read straight from global memory, right-hand side rhs):
@@ -826,15 +863,21 @@ __device__ __forceinline__ void big_refine(const RagParams& p, const RagSys& sy,
     EmitX<MODE> em{xs, sw < 0};
     solve_big(sy, ga, gb, gc, sw < 0 ? gd : wr, tid, Ra, Rb, Rc, Rd, Xs, FD, FC, FA, em);
   }
-  SquareSums rd;
+  float* redf = reinterpret_cast<float*>(red);
+  float m = 0.f, rr = 0.f, dd = 0.f;
+  for (int i = tid; i < n; i += kRagThreads) m = fmaxf(m, fabsf(gd[i]));
+  const unsigned largest = put_largest(m, kRagThreads, redf);
+  consumer_sync(kRagThreads);
+  const float scale = group_scale(largest, kRagThreads, tid, redf);
   double* xo = p.x64 + sy.off;
   for (int i = tid; i < n; i += kRagThreads) {
     const float d = gd[i];
     const float r = xs.residual(i, n, ga[i], gb[i], gc[i], d);
-    rd.add(make_float2(r, d));
+    rr = fmaf(r * scale, r * scale, rr);
+    dd = fmaf(d * scale, d * scale, dd);
     xo[i] = xs.get64(i);
   }
-  group_rel_max(rd, kRagThreads, 1, tid, reinterpret_cast<SquareSum*>(red),
+  group_rel_max(rr, dd, kRagThreads, 1, tid, redf,
                 reinterpret_cast<unsigned long long*>(red + 2 * kRagWarps));
   consumer_sync(kRagThreads);
 }
